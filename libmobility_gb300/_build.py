@@ -24,6 +24,8 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 UNITS = [
     ("mdot_launch.cu", ["-DLMG_REAL=float"], "mdot_f.o"),
     ("mdot_launch.cu", ["-DLMG_REAL=double"], "mdot_d.o"),
+    ("mdot_pairs.cu", ["-DLMG_REAL=float"], "mdot_pairs_f.o"),
+    ("mdot_pairs.cu", ["-DLMG_REAL=double"], "mdot_pairs_d.o"),
     ("solver.cu", [], "solver.o"),
     ("mdot_sym.cu", [], "mdot_sym.o"),
     ("probes.cu", [], "probes.o"),

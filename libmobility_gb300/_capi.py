@@ -107,7 +107,10 @@ def load():
     lib.lmg_internal_sym_plan.restype = _I
     lib.lmg_internal_sym_plan.argtypes = [_I, _I, ctypes.c_longlong, _I, _VP, _VP, _VP, _VP, _VP]
     _F = ctypes.c_float
+    _L = ctypes.c_longlong
     internal = {
+        "lmg_internal_pairs_max_part": [_L],
+        "lmg_internal_pairs_plan": [_I, _I, _I, _I, _L, _I, _L, _VP, _VP, _VP],
         "lmg_internal_gemm": [_I, _I, _I, _I, _I, _VP, _I, _VP, _I, _VP, _I, _VP, _I, _F, _VP],
         "lmg_internal_tanh_backward": [_SZ, _VP, _VP, _VP],
         "lmg_internal_tc_gemm": [_I, _I, _I, _VP, _I, _VP, _I, _VP, _I, _VP, _I, _VP],

@@ -42,6 +42,8 @@ static inline unsigned long long bounds_status_here(bool) { return 0; }
 // status words of the checked kernels' translation units
 unsigned long long bounds_status_mdot_float(bool reset);
 unsigned long long bounds_status_mdot_double(bool reset);
+unsigned long long bounds_status_pairs_float(bool reset);
+unsigned long long bounds_status_pairs_double(bool reset);
 unsigned long long bounds_status_sym(bool reset);
 
 }  // namespace lmg

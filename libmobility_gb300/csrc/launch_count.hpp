@@ -3,6 +3,7 @@
 // (both defined in probes.cu).
 #pragma once
 #include <atomic>
+#include <cstddef>
 
 namespace lmg {
 extern std::atomic<unsigned long long> g_launches;
@@ -13,6 +14,9 @@ extern std::atomic<int> g_force_tpt, g_force_split;
 // g_sym_warps > 0 caps the warps its steps are spread over; g_sym_variant is
 // its register budget, 2, 3 or 4 resident blocks per SM (0 = default, 2)
 extern std::atomic<int> g_sym_mode, g_sym_warps, g_sym_variant;
+// largest scratch of a pass of the unordered-pair product (0 = default);
+// g_sym_mode and g_sym_warps apply to that product too
+extern std::atomic<size_t> g_pairs_max_part;
 // T^{1/2} e1 of the single-system Lanczos checks: 0 the exact host QL; 1 on
 // the device by quadrature; 2 (default) on the host by quadrature; the host
 // QL wherever a quadrature falls back

@@ -25,7 +25,9 @@ __device__ __forceinline__ F2 operator-(F2 a, F2 b) {
   return {__ffma2_rn(b.v, make_float2(-1.f, -1.f), a.v)};
 }
 __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { return {__ffma2_rn(a.v, b.v, c.v)}; }
-__device__ __forceinline__ F2 neg2(F2 a) { return {__fmul2_rn(a.v, make_float2(-1.f, -1.f))}; }
+// -a: the compiler folds it into the operand of the instruction that uses it (no
+// instruction of its own; a multiplication by -1 cost a slot of the FMA pipe)
+__device__ __forceinline__ F2 neg2(F2 a) { return {make_float2(-a.v.x, -a.v.y)}; }
 // c - a b  (fma with -a: exact negation, one rounding)
 __device__ __forceinline__ F2 fms2(F2 a, F2 b, F2 c) { return {__ffma2_rn(neg2(a).v, b.v, c.v)}; }
 __device__ __forceinline__ F2 rsq2(F2 a) { return mk2(rsqrtf(a.v.x), rsqrtf(a.v.y)); }

@@ -16,12 +16,14 @@
 #include "bounds.cuh"
 #include "common.hpp"
 #include "launch_count.hpp"
+#include "mdot_pairs.cuh"
 #include "mdot_sym.cuh"
 
 namespace lmg {
 std::atomic<unsigned long long> g_launches{0};
 std::atomic<int> g_force_tpt{0}, g_force_split{0};
 std::atomic<int> g_sym_mode{0}, g_sym_warps{0}, g_sym_variant{0};
+std::atomic<size_t> g_pairs_max_part{0};
 std::atomic<unsigned long long *> g_sym_trace{nullptr};
 std::atomic<int> g_lanczos_device_sqrt{2};
 std::atomic<int> g_lanczos_lookahead{0};
@@ -167,6 +169,45 @@ int lmg_internal_sym_plan(int N, int nper, long long resident, int force_warps, 
   return 0;
 }
 
+// Largest scratch (elements) of a pass of the unordered-pair product planned
+// after the call; 0 restores the default.  Applies to new handles.
+int lmg_internal_pairs_max_part(long long elems) {
+  if (elems < 0) return 1;
+  lmg::g_pairs_max_part.store((size_t)elems);
+  return 0;
+}
+
+// Host plan of the unordered-pair product for `resident` resident blocks (no
+// device needed).  info[0..4] receives passes, ints of the cut tables, scratch
+// elements, elements carried between passes and tiles per batch; passes: 7
+// values each (first and end row, steps, steps per warp, warps, blocks, offset
+// of its cut table).  Returns 0, or 2 when the shape does not suit the kernel.
+int lmg_internal_pairs_plan(int N, int nper, int ang, int precision, long long resident,
+                            int force_warps, long long max_part, long long *info,
+                            long long *passes, int *cuts) {
+  lmg::PairsPlan p;
+  if (precision)
+    lmg::mdot_pairs_plan_tables<double>(N, nper, ang != 0, resident, force_warps,
+                                        (size_t)max_part, p);
+  else
+    lmg::mdot_pairs_plan_tables<float>(N, nper, ang != 0, resident, force_warps,
+                                       (size_t)max_part, p);
+  if (!p.ok) return 2;
+  info[0] = (long long)p.passes.size();
+  info[1] = (long long)p.cuts.size();
+  info[2] = (long long)p.part_elems;
+  info[3] = (long long)p.acc_elems;
+  info[4] = p.tpb;
+  for (size_t q = 0; passes && q < p.passes.size(); q++) {
+    const lmg::PairsPass &s = p.passes[q];
+    const long long v[7] = {s.row0, s.row1, s.steps, s.per_warp, s.warps, s.grid,
+                            (long long)s.cut_off};
+    std::memcpy(passes + 7 * q, v, sizeof(v));
+  }
+  if (cuts) std::memcpy(cuts, p.cuts.data(), p.cuts.size() * sizeof(int));
+  return 0;
+}
+
 // Where the single-system Lanczos takes T^{1/2} e1 at its checks: 0 the
 // exact QL on the host; 1 on the device by quadrature; 2 (the default) on
 // the host by quadrature; the host QL wherever a quadrature does not apply.
@@ -213,8 +254,16 @@ int lmg_internal_classify_pointer(int type, int ptr_device, int current_device) 
 // reset clears them.
 unsigned long long lmg_internal_bounds_status(int which, int reset) {
   switch (which) {
-    case 0: return lmg::bounds_status_mdot_float(reset != 0);
-    case 1: return lmg::bounds_status_mdot_double(reset != 0);
+    case 0: {
+      const unsigned long long p = lmg::bounds_status_pairs_float(reset != 0);
+      const unsigned long long m = lmg::bounds_status_mdot_float(reset != 0);
+      return m ? m : p;
+    }
+    case 1: {
+      const unsigned long long p = lmg::bounds_status_pairs_double(reset != 0);
+      const unsigned long long m = lmg::bounds_status_mdot_double(reset != 0);
+      return m ? m : p;
+    }
     case 2: return lmg::bounds_status_sym(reset != 0);
     default: return lmg::bounds_status_here(reset != 0);
   }

@@ -20,6 +20,7 @@
 #include "krylov.cuh"
 #include "launch_count.hpp"
 #include "mdot_launch.cuh"
+#include "mdot_pairs.cuh"
 #include "mdot_sym.cuh"
 #include "precond.cuh"
 #include "solver.hpp"
@@ -187,6 +188,17 @@ template <class R> class Solver final : public SolverBase {
   std::map<std::tuple<int, int, int, int>, std::unique_ptr<SymState>> sym_plans_;
   MappedBuffer<int> sym_err_;
   bool mdot_sym(const R *pos, const R *F, R *U);
+  // unordered-pair product (mdot_pairs.cuh): plans, each with one device
+  // buffer of its barrier counts (one per pass) and then its tables; scratch
+  // of their own (a captured product names it: a solve must not move it)
+  struct PairsState {
+    PairsPlan plan;
+    DeviceBuffer<unsigned long long> bars_and_cuts;
+  };
+  std::map<std::tuple<int, int, int, int>, std::unique_ptr<PairsState>> pairs_plans_;
+  DeviceBuffer<R> pairs_part_, pairs_acc_;
+  bool mdot_pairs(const R *pos, const R *F, const R *T, R *U, R *W);
+  void check_barriers();
 
   void release_all();
   int sms();
@@ -199,10 +211,11 @@ template <class R> class Solver final : public SolverBase {
   size_t red_half() const { return red_part_.count / 2; }
   void ensure_side();
   const R *device_input(const void *p, size_t n, R *stage);
-  // M . [F;T] on device buffers: the Lanczos matvec and the RFD probes; with
-  // row_end > 0 only targets [row_begin, row_end), written from row 0 of U, W
-  void mdot_device(const R *pos, const R *F, const R *T, R *U, R *W, int row_begin = 0,
-                   int row_end = 0);
+  // M . [F;T] on device buffers: the products of a Lanczos solve (solve) and
+  // all others, with two roundings: after a few tens of iterations a solve's
+  // iterate, and with it the step it stops at, depends on the last bit of its
+  // products, and a solve with given noise keeps giving the same numbers
+  void mdot_device(const R *pos, const R *F, const R *T, R *U, R *W, bool solve = false);
   void mdot_rows_device(const R *pos, const R *F, const R *T, R *U, R *W, int row_begin,
                         int row_end);
   std::map<std::tuple<int, int, int, int, int>, MdotPlan> row_plans_;
@@ -232,6 +245,9 @@ template <class R> void Solver<R>::release_all() {
   row_plans_.clear();
   sym_plans_.clear();
   sym_err_.release();
+  pairs_plans_.clear();
+  pairs_part_.release();
+  pairs_acc_.release();
   tickets_zeroed_ = false;
 }
 
@@ -322,13 +338,7 @@ template <class R> const R *Solver<R>::device_input(const void *p, size_t n, R *
 }
 
 template <class R>
-void Solver<R>::mdot_device(const R *pos, const R *F, const R *T, R *U, R *W, int row_begin,
-                            int row_end) {
-  const bool rows = row_end > 0 && !(row_begin == 0 && row_end == (int)N_);
-  if (rows) {
-    mdot_rows_device(pos, F, T, U, W, row_begin, row_end);
-    return;
-  }
+void Solver<R>::mdot_device(const R *pos, const R *F, const R *T, R *U, R *W, bool solve) {
   MdotShape s;
   s.geom = wall_ ? kWall : kOpen;
   s.ang = ang_;
@@ -341,7 +351,16 @@ void Solver<R>::mdot_device(const R *pos, const R *F, const R *T, R *U, R *W, in
     if (W) LMG_CUDA(cudaMemsetAsync(W, 0, 3 * (size_t)N * sizeof(R), stream()));
     return;
   }
-  if (s.geom == kOpen && s.has_f && !s.has_t && !s.ang && mdot_sym(pos, F, U)) return;
+  // Outside a solve the unordered-pair product takes every shape: against
+  // mdot_kernel 12 to 62 us at N = 500 (wall, torques, FP32), 680 to 1399 at
+  // 16384, 69 to 3004 at 500 and 1265 to 4974 at 3000 in FP64, and 6.6 to 5.6
+  // only at N = 50 (open, forces).  The symmetric open-space kernel keeps FP32
+  // forces from batches of 384 on (7.3 to 8.6 us at 200, 8.0 to 8.6 at 333,
+  // 8.4 to 8.3 at 500, 23.7 to 20.2 at 4096): four particles a slot and no
+  // staging of torques, but tiles of 128.
+  const bool few = !solve && nper < 384;
+  if (!few && s.geom == kOpen && s.has_f && !s.has_t && !s.ang && mdot_sym(pos, F, U)) return;
+  if (!solve && mdot_pairs(pos, F, s.has_t ? T : nullptr, U, ang_ ? W : nullptr)) return;
   const int ftpt = g_force_tpt.load(), fsplit = g_force_split.load();
   const long key = ((long)N << 30) | ((long)fsplit << 10) | (ftpt << 8) | (s.geom << 3) |
                    (s.has_f << 2) | (s.has_t << 1) | s.ang;
@@ -475,6 +494,26 @@ void Solver<R>::mdot_rows(int64_t row_begin, int64_t row_end, const void *F, siz
   }
 }
 
+// The flag the grid barriers of the symmetric and unordered-pair kernels raise
+// when a wait ran out in an earlier launch: the arrival counts are then
+// inconsistent, so they start afresh and the caller gets an error.
+template <class R> void Solver<R>::check_barriers() {
+  if (!sym_err_.ptr) sym_err_.ensure(1);
+  if (!*(volatile int *)sym_err_.ptr) return;
+  LMG_CUDA(cudaStreamSynchronize(stream()));
+  for (auto &kv : sym_plans_)
+    if (kv.second->count.ptr)
+      LMG_CUDA(cudaMemsetAsync(kv.second->count.ptr, 0, sizeof(unsigned long long), stream()));
+  for (auto &kv : pairs_plans_)
+    if (kv.second->bars_and_cuts.ptr)
+      LMG_CUDA(cudaMemsetAsync(kv.second->bars_and_cuts.ptr, 0,
+                               kv.second->plan.passes.size() * sizeof(unsigned long long),
+                               stream()));
+  *(volatile int *)sym_err_.ptr = 0;
+  throw Error(LMG_ERR_TIMEOUT,
+              "[libmobility_gb300] Mdot: grid barrier of the symmetric kernel timed out");
+}
+
 // U = M F with the symmetric open-space kernel (FP32, forces only, no
 // angular part): returns false where that kernel does not apply.
 template <class R> bool Solver<R>::mdot_sym(const R *pos, const R *F, R *U) {
@@ -515,19 +554,7 @@ template <class R> bool Solver<R>::mdot_sym(const R *pos, const R *F, R *U) {
     const SymState &st = *it->second;
     const SymPlan &p = st.plan;
     if (p.grid <= 0) return false;
-    if (!sym_err_.ptr) sym_err_.ensure(1);
-    if (*(volatile int *)sym_err_.ptr) {
-      // a barrier wait ran out in an earlier launch: arrival counts are
-      // inconsistent, start them afresh
-      LMG_CUDA(cudaStreamSynchronize(stream()));
-      for (auto &kv : sym_plans_)
-        if (kv.second->count.ptr)
-          LMG_CUDA(cudaMemsetAsync(kv.second->count.ptr, 0, sizeof(unsigned long long),
-                                   stream()));
-      *(volatile int *)sym_err_.ptr = 0;
-      throw Error(LMG_ERR_TIMEOUT,
-                  "[libmobility_gb300] Mdot: grid barrier of the symmetric kernel timed out");
-    }
+    check_barriers();
     const PairConst<float> k = make_pair_const<float>(t0_, r0_, rt0_);
     SymTables tab;
     tab.pairs = st.pairs.ptr;
@@ -537,6 +564,43 @@ template <class R> bool Solver<R>::mdot_sym(const R *pos, const R *F, R *U) {
                              sym_err_.device_ptr(), stream()));
     return true;
   }
+}
+
+// U, W = M [F;T] over unordered pairs: returns false where mdot_kernel is the
+// better one.
+template <class R>
+bool Solver<R>::mdot_pairs(const R *pos, const R *F, const R *T, R *U, R *W) {
+  if (g_sym_mode.load() != 0 || g_force_tpt.load() != 0 || g_force_split.load() != 0)
+    return false;
+  const int N = (int)N_;
+  const int warps = g_sym_warps.load();
+  const auto key = std::make_tuple(N, batch_size(), (int)ang_, warps);
+  auto it = pairs_plans_.find(key);
+  if (it == pairs_plans_.end()) {
+    auto st = std::make_unique<PairsState>();
+    LMG_CUDA(mdot_pairs_plan<R>(N, batch_size(), wall_, ang_, sms(), warps,
+                                g_pairs_max_part.load(), st->plan));
+    const PairsPlan &p = st->plan;
+    if (p.ok) {
+      std::vector<unsigned long long> up(p.passes.size() + (p.cuts.size() + 1) / 2, 0ull);
+      std::memcpy(up.data() + p.passes.size(), p.cuts.data(), p.cuts.size() * sizeof(int));
+      LMG_CUDA(cudaMemcpyAsync(st->bars_and_cuts.ensure(up.size()), up.data(),
+                               up.size() * sizeof(up[0]), cudaMemcpyHostToDevice, stream()));
+    }
+    it = pairs_plans_.insert_or_assign(key, std::move(st)).first;
+  }
+  const PairsState &st = *it->second;
+  if (!st.plan.ok) return false;
+  check_barriers();
+  pairs_part_.ensure(st.plan.part_elems);
+  if (st.plan.acc_elems) pairs_acc_.ensure(st.plan.acc_elems);
+  unsigned long long *bars = st.bars_and_cuts.ptr;
+  LMG_CUDA(mdot_pairs_launch<R>(st.plan,
+                                reinterpret_cast<const int *>(bars + st.plan.passes.size()), pos,
+                                F, T, U, W, (R)(1.0 / a_), make_pair_scale<R>(t0_, rt0_),
+                                pairs_part_.ptr, pairs_acc_.ptr, bars, sym_err_.device_ptr(),
+                                stream()));
+  return true;
 }
 
 template <class R>
@@ -1135,6 +1199,7 @@ template <class R> void Solver<R>::clean() {
   V_.release(); w_.release(); y_.release(); ybuf_.release(); z_.release();
   rot_cs_ = {}; rot_idx_ = {};
   part_.release(); tickets_.release(); tickets_zeroed_ = false; plans_.clear();
+  pairs_plans_.clear(); pairs_part_.release(); pairs_acc_.release();
   rfd_noise_.release(); rfd_pos_.release(); rfd_mp_.release(); rfd_mm_.release();
 }
 
@@ -1194,7 +1259,7 @@ template <class R> void Solver<R>::prec_build() {
 template <class R> void Solver<R>::apply_operator(const R *v, R *out) {
   const size_t n3 = 3 * (size_t)N_;
   if (!prec_active()) {
-    mdot_device(pos_.ptr, v, ang_ ? v + n3 : nullptr, out, ang_ ? out + n3 : nullptr);
+    mdot_device(pos_.ptr, v, ang_ ? v + n3 : nullptr, out, ang_ ? out + n3 : nullptr, true);
     return;
   }
   if constexpr (std::is_same<R, float>::value) {
@@ -1210,7 +1275,7 @@ template <class R> void Solver<R>::apply_operator(const R *v, R *out) {
       scale_kernel<R><<<vec_blocks(n3), kRedThreads, 0, stream()>>>(t + n3, v + n3, n3, s);
       count_launch();
     }
-    mdot_device(pos_.ptr, t, ang_ ? t + n3 : nullptr, u, ang_ ? u + n3 : nullptr);
+    mdot_device(pos_.ptr, t, ang_ ? t + n3 : nullptr, u, ang_ ? u + n3 : nullptr, true);
     LMG_CUDA(precond_apply_launch(prec_k_, prec_blocks_.ptr, true, prec_scale(), prec_nb_.ptr, N, u, out, stream()));
     if (ang_) {
       scale_kernel<R><<<vec_blocks(n3), kRedThreads, 0, stream()>>>(out + n3, u + n3, n3, s);

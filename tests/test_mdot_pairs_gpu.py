@@ -1,0 +1,57 @@
+"""The unordered-pair product (csrc/mdot_pairs.cu) on the GPU, against the FP64
+oracle at the sizes where its tiles, ranges and passes change, with the
+tolerances of every Mdot test: 1e-5 (FP32) and 1e-12 (FP64) relative.
+"""
+import numpy as np
+import pytest
+
+from test_mdot_gpu import make_solver, rel_err
+
+pytestmark = pytest.mark.gpu
+TOL = {"float": 1e-5, "double": 1e-12}
+
+
+@pytest.fixture()
+def lib(cuda):
+    from libmobility_gb300 import _capi
+    lib = _capi.load()
+    yield lib
+    lib.lmg_internal_sym_override(0, 0)
+    lib.lmg_internal_pairs_max_part(0)
+
+
+# (N, nper, warps, scratch elements): ragged tiles and slots, batches, ranges cut
+# at many steps, several passes of whole batches and of bands of rows
+SHAPES = [(1, 1, 0, 0), (2, 1, 0, 0), (33, 11, 0, 0), (63, 63, 0, 0), (65, 65, 1, 0),
+          (129, 43, 3, 0), (640, 128, 0, 0), (1537, 1537, 0, 0), (1537, 1537, 37, 0),
+          (1537, 1537, 40, 100000), (1998, 333, 16, 60000)]
+
+
+@pytest.mark.parametrize("precision", ["float", "double"])
+@pytest.mark.parametrize("wall", [0, 1])
+@pytest.mark.parametrize("N,nper,warps,part", SHAPES)
+def test_matches_oracle(lib, oracle, precision, wall, N, nper, warps, part):
+    """Overlapping, coincident and (above a wall) damped particles included."""
+    rng = np.random.default_rng(77 + N + wall)
+    p = rng.uniform(0, (N * 4 * np.pi / 3 / 0.15) ** (1 / 3), (N, 3))
+    if wall:
+        p[:, 2] = rng.uniform(0.3, 9, N)
+    if nper > 10:
+        p[3] = p[7]
+        p[nper - 1] = p[0]
+    F, T = rng.normal(size=(2, N, 3))
+    assert lib.lmg_internal_sym_override(0, warps) == 0
+    assert lib.lmg_internal_pairs_max_part(part) == 0
+    p, F, T = (x.astype(np.float32 if precision == "float" else np.float64) for x in (p, F, T))
+    for ang, f, t in ((0, F, None), (1, F, T), (1, None, T), (1, F, None)):
+        s = make_solver(wall, ang, 1.1, 0.9, precision, N, nper)
+        s.setPositions(p)
+        U, W = s.Mdot(f, t)
+        U2, W2 = s.Mdot(f, t)
+        Uo, Wo = oracle.mdot(p, f, t, a=1.1, viscosity=0.9, wall=wall, include_angular=ang,
+                             nper_batch=nper)
+        assert rel_err(U, Uo) <= TOL[precision], (ang, f is None, t is None)
+        assert np.array_equal(U, U2)  # the order of every sum is fixed
+        if ang:
+            assert rel_err(W, Wo) <= TOL[precision], (f is None, t is None)
+            assert np.array_equal(W, W2)
