@@ -211,6 +211,7 @@ template <class R> class Solver final : public SolverBase {
   size_t red_half() const { return red_part_.count / 2; }
   void ensure_side();
   const R *device_input(const void *p, size_t n, R *stage);
+  const R *staged_input(const void *p, size_t n, R *stage);  // host memory
   // M . [F;T] on device buffers: the products of a Lanczos solve (solve) and
   // all others, with two roundings: after a few tens of iterations a solve's
   // iterate, and with it the step it stops at, depends on the last bit of its
@@ -328,7 +329,10 @@ template <class R> void Solver<R>::set_positions(const void *pos, size_t n) {
 // otherwise copied through the pinned bounce buffer into `stage`.
 template <class R> const R *Solver<R>::device_input(const void *p, size_t n, R *stage) {
   if (!p || n == 0) return nullptr;
-  if (is_device_ptr(p)) return static_cast<const R *>(p);
+  return is_device_ptr(p) ? static_cast<const R *>(p) : staged_input(p, n, stage);
+}
+
+template <class R> const R *Solver<R>::staged_input(const void *p, size_t n, R *stage) {
   R *h = pin_.ensure(n);
   std::memcpy(h, p, n * sizeof(R));
   LMG_CUDA(cudaMemcpyAsync(stage, h, n * sizeof(R), cudaMemcpyHostToDevice, stream()));
@@ -613,15 +617,17 @@ void Solver<R>::mdot(const void *F, size_t nF, const void *T, size_t nT, void *U
   if (!W) nW = 0;
   check_mdot_args(nF, nT, nU, nW);
   const size_t n3 = 3 * (size_t)N_;
-  R *stage = in_stage_.ensure(2 * n3);
-  out_stage_.ensure(2 * n3);
-  pin_.ensure(2 * n3);
-  const R *Fd = device_input(F, nF, stage);
-  const R *Td = device_input(T, nT, stage + n3);
+  // staging only for the arrays that live on the host
+  const bool f_host = nF && !is_device_ptr(F), t_host = nT && !is_device_ptr(T);
   const bool u_dev = nU && is_device_ptr(U);
   const bool w_dev = nW && is_device_ptr(W);
-  R *Ud = nU ? (u_dev ? static_cast<R *>(U) : out_stage_.ensure(2 * n3)) : nullptr;
-  R *Wd = nW ? (w_dev ? static_cast<R *>(W) : out_stage_.ensure(2 * n3) + n3) : nullptr;
+  R *stage = f_host || t_host ? in_stage_.ensure(2 * n3) : nullptr;
+  R *out = (nU && !u_dev) || (nW && !w_dev) ? out_stage_.ensure(2 * n3) : nullptr;
+  if (stage || out) pin_.ensure(2 * n3);
+  const R *Fd = f_host ? staged_input(F, nF, stage) : nF ? static_cast<const R *>(F) : nullptr;
+  const R *Td = t_host ? staged_input(T, nT, stage + n3) : nT ? static_cast<const R *>(T) : nullptr;
+  R *Ud = nU ? (u_dev ? static_cast<R *>(U) : out) : nullptr;
+  R *Wd = nW ? (w_dev ? static_cast<R *>(W) : out + n3) : nullptr;
   mdot_device(pos_.ptr, Fd, Td, Ud, Wd);
   LMG_CUDA(cudaGetLastError());
   if ((nU && !u_dev) || (nW && !w_dev)) {
@@ -1030,13 +1036,11 @@ void Solver<R>::sqrt_mdot_w(void *U, size_t nU, void *W, size_t nW, double prefa
                 "[libmobility_gb300] dW must hold 3N values (6N with includeAngular)");
   ensure_lanczos();
   R *z = z_.ensure(n);
-  pin_.ensure(2 * n3);
-  out_stage_.ensure(2 * n3);
   if (dW) {
     if (is_device_ptr(dW)) {
       LMG_CUDA(cudaMemcpyAsync(z, dW, n * sizeof(R), cudaMemcpyDeviceToDevice, stream()));
     } else {
-      R *h = pin_.ensure(n);
+      R *h = pin_.ensure(2 * n3);
       std::memcpy(h, dW, n * sizeof(R));
       LMG_CUDA(cudaMemcpyAsync(z, h, n * sizeof(R), cudaMemcpyHostToDevice, stream()));
     }
@@ -1143,8 +1147,6 @@ void Solver<R>::div_m(void *U, size_t nU, void *W, size_t nW, double prefactor) 
   R *pd = rfd_pos_.ensure(n3);
   R *mp = rfd_mp_.ensure(2 * n3);
   R *mm = rfd_mm_.ensure(2 * n3);
-  pin_.ensure(2 * n3);
-  out_stage_.ensure(2 * n3);
   cudaStream_t st = stream();
   const int vb = vec_blocks(n3);
   gauss_fill_kernel<R><<<vec_blocks(n3 / 4 + 1), kRedThreads, 0, st>>>(noise, n3, seed,
