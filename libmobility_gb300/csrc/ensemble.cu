@@ -443,6 +443,9 @@ template <class R> class Ensemble final : public EnsembleBase {
     int s0 = 0, s1 = 0;  // internal systems [s0, s1)
     int p0 = 0, p1 = 0;  // internal (padded) particles [p0, p1)
     int span = 0;        // largest padded system
+    // tiles of two targets a thread (2 kPad) never cover two systems; where
+    // they would, a tile's sources are those of both, more than `span`
+    bool wide_tiles = true;
     DeviceBuffer<int> sys_begin;
     MdotPlan plan;
     bool tuned = false;
@@ -696,6 +699,7 @@ void Ensemble<R>::set_systems(int nsys, const int *sizes, const int *geometry,
     for (int k = g->s0; k <= g->s1; k++) sb[k - g->s0] = ioff_[k] - g->p0;
     for (int k = g->s0; k < g->s1; k++) {
       g->span = std::max(g->span, pad_[k]);
+      g->wide_tiles = g->wide_tiles && (pad_[k] % (2 * kPad) == 0 || k == g->s1 - 1);
       g->work += (double)pad_[k] * pad_[k] * (g->geom ? 160.0 : 36.0);
     }
     int *d = g->sys_begin.ensure(sb.size());
@@ -831,6 +835,7 @@ template <class R> void Ensemble<R>::ensure_plans() {
       // targets per thread (1 or 2) x source splits
       std::vector<MdotPlan> plans;
       for (int tpt : {1, 2}) {
+        if (tpt == 2 && !g.wide_tiles) continue;
         for (int c : cand) {
           MdotPlan p;
           if (mdot_plan<R>(shape(g), N, g.span, sms(), tpt, c, p) != cudaSuccess) {

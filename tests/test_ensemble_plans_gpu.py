@@ -1,0 +1,37 @@
+"""Launch plans of the ensemble's autotuner: every plan it may pick gives every
+system the whole sum over its sources.
+
+Systems whose padded size is an odd multiple of 128 lie side by side in a
+group, so a tile of 256 targets (two per thread) would cover two of them and
+need the sources of both; the splits are made for one.  Products against the
+FP64 oracle, 1e-5 relative as every FP32 Mdot, on fresh handles, since the
+choice is made by timing.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("repeat", range(4))
+@pytest.mark.parametrize("sizes", [[300, 310, 290, 380, 330, 350], [100, 90, 120, 70],
+                                   [600, 700, 620, 760], [200, 256, 250, 130, 140]])
+def test_tuned_plans_sum_every_source(cuda, oracle, sizes, repeat):
+    from libmobility_gb300.ensemble import Ensemble
+    rng = np.random.default_rng(repeat + sum(sizes))
+    sizes = sizes * 4
+    geometry = ["open" if k % 2 else "single_wall" for k in range(len(sizes))]
+    pos = [np.column_stack([rng.uniform(0, n ** 0.5, (n, 2)), rng.uniform(1.5, 20, n)])
+           for n in sizes]
+    F = [rng.normal(size=(n, 3)) for n in sizes]
+    e = Ensemble(precision="float")
+    e.setSystems(sizes, geometry, [0.0] * len(sizes))
+    e.initialize(1.0, 1.0, tolerance=1e-4, seed=1)
+    e.setPositions(np.concatenate(pos).astype(np.float32))
+    U = e.Mdot(np.concatenate(F).astype(np.float32))
+    b = 0
+    for p, f, g in zip(pos, F, geometry):
+        Uo, _ = oracle.mdot(p.astype(np.float32), f.astype(np.float32), None, a=1.0,
+                            viscosity=1.0, wall=g != "open", include_angular=0)
+        assert np.abs(U[b:b + len(p)] - Uo).max() <= 1e-5 * np.abs(Uo).max(), (len(p), g)
+        b += len(p)
