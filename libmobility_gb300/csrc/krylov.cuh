@@ -165,6 +165,7 @@ struct KrylovScalars {
   int pad;
   double alpha[256];  // diagonal of T
   double beta[256];   // off-diagonal of T (beta[i] couples i and i+1)
+  float beta_f[256];  // the same rounded to FP32
 };
 
 // |z|^2 -> normz, and v0 = z/|z| (two kernels: the norm is a grid reduction)
@@ -311,6 +312,11 @@ __device__ __forceinline__ float2 ld_dsmem(const float2 *local, unsigned rank) {
 template <class R> struct DotAcc {
   double v = 0.0;
   __device__ __forceinline__ void add_prod(R x, R y) { v += (double)x * (double)y; }
+  __device__ __forceinline__ void add_diff2(R x, R y) {  // (x - y)^2
+    const double d = (double)x - (double)y;
+    v += d * d;
+  }
+  __device__ __forceinline__ void merge(const DotAcc &o) { v += o.v; }
   __device__ __forceinline__ void warp_merge() { v = warp_sum(v); }
   __device__ __forceinline__ double value() const { return v; }
 };
@@ -328,6 +334,16 @@ template <> struct DotAcc<float> {
     const float p = __fmul_rn(x, y);
     add(p, __fmaf_rn(x, y, -p));
   }
+  // (x - y)^2: the difference as d + e exactly (two-sum), squared to first order
+  // in e
+  __device__ __forceinline__ void add_diff2(float x, float y) {
+    const float d = __fsub_rn(x, y);
+    const float bp = __fsub_rn(d, x);
+    const float e = __fsub_rn(__fsub_rn(x, __fsub_rn(d, bp)), __fadd_rn(y, bp));
+    const float p = __fmul_rn(d, d);
+    add(p, __fmaf_rn(__fadd_rn(d, d), e, __fmaf_rn(d, d, -p)));
+  }
+  __device__ __forceinline__ void merge(const DotAcc &o) { merge(o.s, o.c); }
   // (s, c) += (s2, c2); the same result for either order of the operands
   __device__ __forceinline__ void merge(float s2, float c2) {
     const float t = __fadd_rn(s, s2);
@@ -349,7 +365,8 @@ template <> struct DotAcc<float> {
 template <class R> struct ClusterRed {
   double warp[32];
   double part[2];
-  double tot[2];
+  double alpha, tol, beta;
+  R alpha_r, inv_beta;
   __device__ __forceinline__ void put_warp(int w, const DotAcc<R> &a) { warp[w] = a.v; }
   __device__ __forceinline__ DotAcc<R> get_warp(int w) const { DotAcc<R> a; a.v = warp[w]; return a; }
   __device__ __forceinline__ void put_part(int q, const DotAcc<R> &a) { part[q] = a.v; }
@@ -362,7 +379,8 @@ template <class R> struct ClusterRed {
 template <> struct ClusterRed<float> {
   float2 warp[32];
   float2 part[2];
-  double tot[2];
+  double alpha, tol, beta;
+  float alpha_r, inv_beta;
   __device__ __forceinline__ void put_warp(int w, const DotAcc<float> &a) {
     warp[w] = make_float2(a.s, a.c);
   }
@@ -384,16 +402,16 @@ template <> struct ClusterRed<float> {
   }
 };
 
-// The sum over the cluster of every thread's accumulator, the same value in
-// every thread of every CTA: xor trees within the warps, over the block's
-// warps (warp 0) and over the cluster's CTAs (warp 0, reading the other CTAs'
-// partials in distributed shared memory after a cluster barrier), then
-// broadcast through shared memory.  Each reduction of a launch uses its own
-// partial slot `q`, so no CTA overwrites a partial that another may still
-// be reading.
+// The sum over the cluster of every thread's accumulator: xor trees within the
+// warps, over the block's warps (warp 0) and over the cluster's CTAs (the warps
+// whose index is below `readers`, reading the other CTAs' partials in
+// distributed shared memory after a cluster barrier).  Every lane of those
+// warps returns with the total; the others return with nothing of use.  Each
+// reduction of a launch uses its own partial slot `q`, so no CTA overwrites a
+// partial that another may still be reading.
 template <class R>
-__device__ __forceinline__ double cluster_reduce(DotAcc<R> a, ClusterRed<R> &sh, int q,
-                                                 unsigned nct) {
+__device__ __forceinline__ DotAcc<R> cluster_reduce(DotAcc<R> a, ClusterRed<R> &sh, int q,
+                                                    unsigned nct, int readers) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   a.warp_merge();
   if (lane == 0) sh.put_warp(wid, a);
@@ -406,14 +424,12 @@ __device__ __forceinline__ double cluster_reduce(DotAcc<R> a, ClusterRed<R> &sh,
   }
   cluster_arrive();
   cluster_wait();
-  if (wid == 0) {
-    DotAcc<R> b;
+  DotAcc<R> b;
+  if (wid < readers) {
     if (lane < (int)nct) b = sh.get_part(q, lane);
     b.warp_merge();
-    if (lane == 0) sh.tot[q] = b.value();
   }
-  __syncthreads();
-  return sh.tot[q];
+  return b;
 }
 
 // ---------------------------------------------------------------------------
@@ -428,6 +444,13 @@ __device__ __forceinline__ double cluster_reduce(DotAcc<R> a, ClusterRed<R> &sh,
 // across the phases (n <= EPT x the cluster's threads); EPT = 0 streams them
 // through memory (any n).  Launched as one cluster of up to 16 CTAs of up
 // to kClusterThreads threads (a multiple of 32).
+//
+// FP64 scalars are worked out by one thread each and passed on in the vectors'
+// precision: an SM issues an FP64 instruction of a warp every 19 cycles, so a
+// square root and two divisions in all 8 (32) warps of a CTA took 4.5 (18) us
+// of the step.  Two warps share them after the second reduction: |w| with the
+// breakdown test, and 1/|w| (for FP32 vectors from the reciprocal square root,
+// rounded to FP32).
 // ---------------------------------------------------------------------------
 template <class R, int EPT>
 __global__ void __launch_bounds__(kClusterThreads, 1)
@@ -440,7 +463,9 @@ krylov_step_cluster_kernel(R *w, const R *vi, const R *vprev, R *vnext, size_t n
   const size_t e0 = (size_t)rank * blockDim.x + threadIdx.x;
   R wr[E], vr[E];
   // w -= beta_{i-1} v_{i-1};  alpha_i = w . v_i
-  const R bprev = i > 0 ? (R)sc->beta[i - 1] : R(0);
+  const R bprev = i > 0 ? (sizeof(R) == 4 ? (R)sc->beta_f[i - 1] : (R)sc->beta[i - 1]) : R(0);
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int second = blockDim.x > 32 ? 1 : 0;  // the other warp with FP64 work
   DotAcc<R> acc;
   if (EPT > 0) {
 #pragma unroll
@@ -463,9 +488,18 @@ krylov_step_cluster_kernel(R *w, const R *vi, const R *vprev, R *vnext, size_t n
       acc.add_prod(x, vi[e]);
     }
   }
-  const double alpha = cluster_reduce<R>(acc, red, 0, nct);
+  {
+    const DotAcc<R> t = cluster_reduce<R>(acc, red, 0, nct, 1);
+    if (threadIdx.x == 0) {
+      red.alpha = t.value();
+      red.alpha_r = (R)red.alpha;
+    }
+  }
+  __syncthreads();
+  // the breakdown limit (LanczosAlgorithm.cu:141-143), while the others go on
+  if (wid == second && lane == 0) red.tol = 1e-3 * red.alpha / sc->normz;
   // w -= alpha_i v_i;  beta_i = |w| with the breakdown rule
-  const R al = (R)alpha;
+  const R al = red.alpha_r;
   DotAcc<R> acc2;
   if (EPT > 0) {
 #pragma unroll
@@ -483,29 +517,38 @@ krylov_step_cluster_kernel(R *w, const R *vi, const R *vprev, R *vnext, size_t n
       acc2.add_prod(x, x);
     }
   }
-  double b = sqrt(cluster_reduce<R>(acc2, red, 1, nct));
-  // no CTA reads another's partials after this point; the matching wait
-  // before the exit keeps every CTA's shared memory alive until then
-  cluster_arrive();
-  const double tol = 1e-3 * alpha / sc->normz;  // LanczosAlgorithm.cu:141-143
-  if (b < tol) b = 0.0;
+  {
+    const DotAcc<R> t = cluster_reduce<R>(acc2, red, 1, nct, 2);
+    // no CTA reads another's partials after this point; the matching wait
+    // before the exit keeps every CTA's shared memory alive until then
+    cluster_arrive();
+    if (lane == 0 && wid == 0) {
+      const double b = sqrt(t.value());
+      red.beta = b < red.tol ? 0.0 : b;
+    }
+    if (lane == 0 && wid == second)
+      red.inv_beta = sizeof(R) == 4 ? (R)rsqrt(t.value()) : (R)(1.0 / sqrt(t.value()));
+  }
+  __syncthreads();
+  const bool broke = !(red.beta > 0.0);
   if (rank == 0 && threadIdx.x == 0) {
-    sc->alpha[i] = alpha;
-    sc->beta[i] = b;
-    host_ab[2 * i] = alpha;
-    host_ab[2 * i + 1] = b;
+    sc->alpha[i] = red.alpha;
+    sc->beta[i] = red.beta;
+    sc->beta_f[i] = (float)red.beta;
+    host_ab[2 * i] = red.alpha;
+    host_ab[2 * i + 1] = red.beta;
   }
   // v_{i+1} = w / beta_i, or e1 after a breakdown
-  const R inv = b > 0.0 ? (R)(1.0 / b) : R(0);
+  const R inv = broke ? R(0) : red.inv_beta;
   if (EPT > 0) {
 #pragma unroll
     for (int k = 0; k < E; k++) {
       const size_t e = e0 + (size_t)k * stride;
-      if (e < n) vnext[e] = b > 0.0 ? wr[k] * inv : (e == 0 ? R(1) : R(0));
+      if (e < n) vnext[e] = !broke ? wr[k] * inv : (e == 0 ? R(1) : R(0));
     }
   } else {
     for (size_t e = e0; e < n; e += stride)
-      vnext[e] = b > 0.0 ? w[e] * inv : (e == 0 ? R(1) : R(0));
+      vnext[e] = !broke ? w[e] * inv : (e == 0 ? R(1) : R(0));
   }
   cluster_wait();
 }
@@ -879,6 +922,62 @@ tridiag_sqrt_quad_kernel(const KrylovScalars *sc, int m, double *out, double *G,
   if (t == 0) *flag = 0.0;
 }
 
+// Grid totals of two accumulators, as grid_sum (same trees): FP32 vectors keep
+// them as pairs of floats throughout (two floats in the place of a double), so
+// that the whole grid does no FP64 arithmetic.  True in thread 0 of the last
+// block.
+template <class R>
+__device__ __forceinline__ bool grid_sum_dot(DotAcc<R> (&v)[2], double *partials,
+                                             unsigned *ticket, double (&tot)[2]) {
+  static_assert(sizeof(DotAcc<R>) == sizeof(double), "one partial each");
+  __shared__ DotAcc<R> red[2][kRedThreads / 32];
+  __shared__ bool s_last;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  auto block_merge = [&](DotAcc<R> (&x)[2]) {
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      x[q].warp_merge();
+      if (lane == 0) red[q][wid] = x[q];
+    }
+    __syncthreads();
+    if (wid == 0) {
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        x[q] = lane < kRedThreads / 32 ? red[q][lane] : DotAcc<R>();
+        x[q].warp_merge();
+      }
+    }
+  };
+  DotAcc<R> *part = reinterpret_cast<DotAcc<R> *>(partials);
+  block_merge(v);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int q = 0; q < 2; q++) part[(size_t)q * gridDim.x + blockIdx.x] = v[q];
+    __threadfence();
+    s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return false;
+  __threadfence();
+  DotAcc<R> acc[2];
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const double raw = __ldcg(partials + (size_t)q * gridDim.x + b);
+      DotAcc<R> p;
+      memcpy(&p, &raw, sizeof(p));
+      acc[q].merge(p);
+    }
+  }
+  block_merge(acc);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int q = 0; q < 2; q++) tot[q] = acc[q].value();
+    *ticket = 0u;
+  }
+  return threadIdx.x == 0;
+}
+
 // y = |z| V c over m basis vectors and, when yprev is given, err = |y -
 // yprev| / |yprev| (FP64) -> sc->err and the mapped host copy: the estimate
 // and the error of one convergence check in one launch (each thread's
@@ -901,7 +1000,7 @@ __global__ void krylov_check_kernel(const R *V, size_t ldv, int m, const double 
   const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const int part = (int)(tid % TPE);
   const size_t per_pass = (size_t)gridDim.x * blockDim.x / TPE;
-  double v[2] = {0.0, 0.0};
+  DotAcc<R> v[2];  // |yprev|^2, |y - yprev|^2
   for (size_t e0 = 0; e0 < n; e0 += per_pass) {
     const size_t e = e0 + tid / TPE;
     const bool ok = e < n;
@@ -925,15 +1024,15 @@ __global__ void krylov_check_kernel(const R *V, size_t ldv, int m, const double 
     if (ok && part == 0) {
       y[e] = acc;
       if (yprev) {
-        const double a = (double)yprev[e], dlt = (double)acc - a;
-        v[0] += a * a;
-        v[1] += dlt * dlt;
+        const R a = yprev[e];
+        v[0].add_prod(a, a);
+        v[1].add_diff2(acc, a);
       }
     }
   }
   if (!yprev) return;
   double tot[2];
-  if (grid_sum<2>(v, partials, ticket, tot)) {
+  if (grid_sum_dot<R>(v, partials, ticket, tot)) {
     const double err = fabs(sqrt(tot[1]) / sqrt(tot[0]));
     sc->err = err;
     *host_err = err;
