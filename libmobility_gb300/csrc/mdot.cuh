@@ -6,10 +6,11 @@
 // batch contributes, the self pair included, and the outputs are overwritten.
 //
 // Layout and schedule:
-//   * a CTA owns BT = THREADS*TPT consecutive targets (TPT per thread,
-//     strided by THREADS so loads and stores coalesce) and one contiguous
-//     chunk of their batch's sources (blockIdx.y selects the chunk);
-//   * sources are staged through shared memory in tiles of THREADS, already
+//   * a CTA owns BT = TILE*TPT consecutive targets (TPT per thread,
+//     strided by TILE so loads and stores coalesce) and one contiguous
+//     chunk of their batch's sources (blockIdx.y selects the chunk); in FP64 a
+//     tile is shared by SUB = 4 CTAs of one warp (below);
+//   * sources are staged through shared memory in tiles of TILE, already
 //     divided by the radius a and, for the wall, clamped (h = max(z, a)/a)
 //     and damped (F, T pre-multiplied by b_j); every thread then reads the
 //     tile by broadcast;
@@ -49,7 +50,7 @@ template <class R> struct MdotArgs {
   // row i - tgt_begin of U and W (every source of a target's batch counts)
   int tgt_begin, tgt_end;
   int nper;              // equal batch size when sys_begin == nullptr
-  int chunk;             // sources per split (multiple of THREADS)
+  int chunk;             // sources per split (multiple of TILE)
   R inv_a;               // 1/a
   PairConst<R> k;
   WallConst kw;          // fused all-blocks wall constants (FP32 path)
@@ -122,7 +123,7 @@ template <class R, int GEOM, bool HAS_F, bool HAS_T, bool ANG> struct PairKernel
     if constexpr (EXACT) {
       rpy_coefficients<R, UF, WT, UT || WF, true>(k, r2, dev_rsqrt<R>(r2), f, G, fw, Gw, c);
     } else {
-      const R r2c = r2 > R(4) ? r2 : R(4);
+      const R r2c = below4(r2) ? R(4) : r2;
       rpy_coefficients<R, UF, WT, UT || WF, false>(k, r2c, rsqrt_normal<R>(r2c), f, G, fw, Gw,
                                                    c);
     }
@@ -178,6 +179,21 @@ template <class R, int GEOM, bool HAS_F, bool HAS_T, bool ANG> struct PairKernel
     return r2;
   }
 
+  // Whether a pair is closer than 2a (r^2 as correct() takes it).  A target's
+  // close sources are found first and then corrected one by one in their order,
+  // so a warp takes as many rounds as its busiest target has close sources
+  // (testing inside one loop over the sources took a round for each source
+  // close to any target: all 32 where the targets meet themselves).
+  static __device__ __forceinline__ bool below4(R r2) {
+    // FP64 by the upper word's bits: a comparison takes a slot of the FP64 pipe
+    if constexpr (sizeof(R) == 8) return __double2hiint(r2) < 0x40100000;
+    else return r2 < R(4);
+  }
+  static __device__ __forceinline__ bool near_pair(R xi, R yi, R zi, R xj, R yj, R zj) {
+    const R dx = xi - xj, dy = yi - yj, dz = zi - zj;
+    return below4(fmaR(dx, dx, fmaR(dy, dy, dz * dz)));
+  }
+
   // For a pair with r^2 < 4 already added in the fast form: adds
   // (exact - fast).  Both are O(1) there, so the difference is accurate.
   static __device__ __forceinline__ void correct(const PairConst<R> &k, const WallConst &kw,
@@ -195,11 +211,13 @@ template <class R, int GEOM, bool HAS_F, bool HAS_T, bool ANG> struct PairKernel
   }
 };
 
-template <class R, int GEOM, bool HAS_F, bool HAS_T, bool ANG, int TPT, int THREADS>
-__global__ void __launch_bounds__(THREADS)
+template <class R, int GEOM, bool HAS_F, bool HAS_T, bool ANG, int TPT, int TILE, int SUB>
+__global__ void __launch_bounds__(TILE / SUB)
 mdot_kernel(const MdotArgs<R> a) {
   using PK = PairKernel<R, GEOM, HAS_F, HAS_T, ANG>;
-  constexpr int BT = THREADS * TPT;
+  static_assert(SUB == 1 || TPT == 1, "a tile is shared by CTAs of one target a thread");
+  constexpr int THREADS = TILE / SUB;
+  constexpr int BT = TILE * TPT;
   constexpr bool USE_T = HAS_T && ANG;
   constexpr int NC = ANG ? 6 : 3;  // accumulated components per target
   constexpr bool COMP = sizeof(R) == 4;  // compensated accumulation in FP32
@@ -210,18 +228,19 @@ mdot_kernel(const MdotArgs<R> a) {
   // (x, y, z, F, and T for all blocks) so that one float4 read yields a
   // component of four sources.
   constexpr bool PACK = PK::FUSED_WALL;
-  constexpr bool PACK_UF = sizeof(R) == 4 && HAS_F && !ANG && THREADS % 32 == 0;
+  constexpr bool PACK_UF = sizeof(R) == 4 && HAS_F && !ANG;
   constexpr int NSV = PACK ? 9 : (PACK_UF ? 6 : 1);
   constexpr bool SOA = PACK || PACK_UF;
-  __shared__ Q4<R> sp[SOA ? 1 : THREADS];
-  __shared__ Q4<R> sf[HAS_F && !SOA ? THREADS : 1];
-  __shared__ Q4<R> st[USE_T && !SOA ? THREADS : 1];
-  __shared__ __align__(16) float sv[NSV][SOA ? THREADS : 4];
+  __shared__ Q4<R> sp[SOA ? 1 : TILE];
+  __shared__ Q4<R> sf[HAS_F && !SOA ? TILE : 1];
+  __shared__ Q4<R> st[USE_T && !SOA ? TILE : 1];
+  __shared__ __align__(16) float sv[NSV][SOA ? TILE : 4];
   __shared__ int s_last;
 
   const int N = a.N;
   const int t_lo = a.tgt_begin, t_hi = a.tgt_end > 0 ? a.tgt_end : N;
-  const int tile = blockIdx.x;
+  const int tile = blockIdx.x / SUB;
+  const int me = (blockIdx.x % SUB) * THREADS + threadIdx.x;  // first target in the tile
   const int split = blockIdx.y;
   const int nsplit = gridDim.y;
   const int tgt0 = t_lo + tile * BT;
@@ -232,7 +251,7 @@ mdot_kernel(const MdotArgs<R> a) {
   int lo[TPT], hi[TPT];
 #pragma unroll
   for (int t = 0; t < TPT; t++) {
-    int i = tgt0 + threadIdx.x + t * THREADS;
+    int i = tgt0 + me + t * TILE;
     int ic = i < t_hi ? i : t_hi - 1;
     R x = a.pos[3 * ic], y = a.pos[3 * ic + 1], z = a.pos[3 * ic + 2];
     xi[t] = mul_rn(x, ia);
@@ -274,9 +293,10 @@ mdot_kernel(const MdotArgs<R> a) {
     for (int c = 0; c < NC; c++) { S[t][c] = 0; C[t][c] = 0; }
   }
 
-  for (int ts = c_begin; ts < c_end; ts += THREADS) {
-    {  // stage one tile of sources
-      const int j = ts + threadIdx.x;
+  for (int ts = c_begin; ts < c_end; ts += TILE) {
+#pragma unroll
+    for (int s0 = 0; s0 < TILE; s0 += THREADS) {  // stage one tile of sources
+      const int sj = s0 + threadIdx.x, j = ts + sj;
       Q4<R> p = {0, 0, 0, 0}, fv = {0, 0, 0, 0}, tv = {0, 0, 0, 0};
       if (j < c_end && LMG_IN_BOUNDS(j < N, 1, j)) {
         R x = a.pos[3 * j], y = a.pos[3 * j + 1], z = a.pos[3 * j + 2];
@@ -296,17 +316,17 @@ mdot_kernel(const MdotArgs<R> a) {
       if constexpr (SOA) {
         const float c9[9] = {p.x, p.y, p.z, fv.x, fv.y, fv.z, tv.x, tv.y, tv.z};
 #pragma unroll
-        for (int c = 0; c < NSV; c++) sv[c][threadIdx.x] = c9[c];
+        for (int c = 0; c < NSV; c++) sv[c][sj] = c9[c];
       } else {
-        sp[threadIdx.x] = p;
-        if (HAS_F) sf[threadIdx.x] = fv;
-        if (USE_T) st[threadIdx.x] = tv;
+        sp[sj] = p;
+        if (HAS_F) sf[sj] = fv;
+        if (USE_T) st[sj] = tv;
       }
     }
     __syncthreads();
-    const int n_here = min(THREADS, c_end - ts);
+    const int n_here = min(TILE, c_end - ts);
     if constexpr (PACK) {
-      if (uniform && n_here == THREADS) {
+      if (uniform && n_here == TILE) {
         V3p u2[TPT], w2[TPT];
 #pragma unroll
         for (int t = 0; t < TPT; t++) {
@@ -314,7 +334,7 @@ mdot_kernel(const MdotArgs<R> a) {
           w2[t] = {bc(0.f), bc(0.f), bc(0.f)};
         }
 #pragma unroll 1
-        for (int jj = 0; jj < THREADS; jj += 4) {
+        for (int jj = 0; jj < TILE; jj += 4) {
           float4 q[9];
 #pragma unroll
           for (int c = 0; c < 9; c++) q[c] = *reinterpret_cast<const float4 *>(&sv[c][jj]);
@@ -350,13 +370,13 @@ mdot_kernel(const MdotArgs<R> a) {
         }
       }
     } else if constexpr (PACK_UF && GEOM == kWall) {
-      if (uniform && n_here == THREADS) {
+      if (uniform && n_here == TILE) {
         // two sources per instruction; close pairs fall back lane by lane
         V3p u2[TPT];
 #pragma unroll
         for (int t = 0; t < TPT; t++) u2[t] = {bc(0.f), bc(0.f), bc(0.f)};
 #pragma unroll 1
-        for (int jj = 0; jj < THREADS; jj += 4) {
+        for (int jj = 0; jj < TILE; jj += 4) {
           float4 q[6];
 #pragma unroll
           for (int c = 0; c < 6; c++) q[c] = *reinterpret_cast<const float4 *>(&sv[c][jj]);
@@ -388,10 +408,10 @@ mdot_kernel(const MdotArgs<R> a) {
         }
       }
     } else if constexpr (PACK_UF) {
-      if (uniform && n_here == THREADS) {
+      if (uniform && n_here == TILE) {
         // as the scalar full-tile path below, two sources per instruction
 #pragma unroll 1
-        for (int j0 = 0; j0 < THREADS; j0 += 32) {
+        for (int j0 = 0; j0 < TILE; j0 += 32) {
           V3p u2[TPT];
           float2 mr2[TPT];
 #pragma unroll
@@ -426,12 +446,16 @@ mdot_kernel(const MdotArgs<R> a) {
           if (__any_sync(0xffffffffu, near)) {
 #pragma unroll
             for (int t = 0; t < TPT; t++) {
-              if (fminf(mr2[t].x, mr2[t].y) < 4.f) {
-                for (int jj = j0; jj < j0 + 32; jj++) {
-                  const Q4<R> p = {sv[0][jj], sv[1][jj], sv[2][jj], 0};
-                  const Q4<R> fv = {sv[3][jj], sv[4][jj], sv[5][jj], 0};
-                  PK::correct(a.k, a.kw, xi[t], yi[t], zi[t], p, fv, fv, u[t], w[t]);
-                }
+              unsigned close = 0u;
+#pragma unroll 8
+              for (int jj = 0; jj < 32; jj++)
+                close |= (unsigned)PK::near_pair(xi[t], yi[t], zi[t], sv[0][j0 + jj],
+                                                 sv[1][j0 + jj], sv[2][j0 + jj]) << jj;
+              for (; close != 0u; close &= close - 1u) {
+                const int jj = j0 + __ffs(close) - 1;
+                const Q4<R> p = {sv[0][jj], sv[1][jj], sv[2][jj], 0};
+                const Q4<R> fv = {sv[3][jj], sv[4][jj], sv[5][jj], 0};
+                PK::correct(a.k, a.kw, xi[t], yi[t], zi[t], p, fv, fv, u[t], w[t]);
               }
             }
           }
@@ -446,17 +470,17 @@ mdot_kernel(const MdotArgs<R> a) {
             if (j >= lo[t] && j < hi[t]) PK::eval(a.k, a.kw, xi[t], yi[t], zi[t], p, fv, fv, u[t], w[t]);
         }
       }
-    } else if (uniform && n_here == THREADS) {
+    } else if (uniform && n_here == TILE) {
       // Fast form for every pair, 32 sources at a time; then, in a warp where
       // some target met a pair closer than 2a among those 32 (its self pair,
       // or an overlap), those targets swap the fast value of such pairs for
       // the exact one.  Targets are tile-aligned, so a warp's self pairs all
       // fall in the same 32 sources.
 #pragma unroll 1
-      for (int j0 = 0; j0 < THREADS; j0 += 32) {
-        R mr2[TPT];
+      for (int j0 = 0; j0 < TILE; j0 += 32) {
+        bool near[TPT];
 #pragma unroll
-        for (int t = 0; t < TPT; t++) mr2[t] = R(4);
+        for (int t = 0; t < TPT; t++) near[t] = false;
 #pragma unroll 4
         for (int jj = j0; jj < j0 + 32; jj++) {
           const Q4<R> p = sp[jj];
@@ -466,22 +490,26 @@ mdot_kernel(const MdotArgs<R> a) {
           for (int t = 0; t < TPT; t++) {
             const R r2 = PK::template eval<false>(a.k, a.kw, xi[t], yi[t], zi[t], p, fv, tv,
                                                   u[t], w[t]);
-            mr2[t] = r2 < mr2[t] ? r2 : mr2[t];  // a min in R (no promotion)
+            near[t] |= PK::below4(r2);
           }
         }
-        bool near = false;
+        bool any = false;
 #pragma unroll
-        for (int t = 0; t < TPT; t++) near = near || mr2[t] < R(4);
-        if (__any_sync(0xffffffffu, near)) {
+        for (int t = 0; t < TPT; t++) any = any || near[t];
+        if (__any_sync(0xffffffffu, any)) {
 #pragma unroll
           for (int t = 0; t < TPT; t++) {
-            if (mr2[t] < R(4)) {
-              for (int jj = j0; jj < j0 + 32; jj++) {
-                const Q4<R> p = sp[jj];
-                const Q4<R> fv = HAS_F ? sf[jj] : Q4<R>{0, 0, 0, 0};
-                const Q4<R> tv = USE_T ? st[jj] : Q4<R>{0, 0, 0, 0};
-                PK::correct(a.k, a.kw, xi[t], yi[t], zi[t], p, fv, tv, u[t], w[t]);
-              }
+            unsigned close = 0u;
+#pragma unroll 8
+            for (int jj = 0; jj < 32; jj++)
+              close |= (unsigned)PK::near_pair(xi[t], yi[t], zi[t], sp[j0 + jj].x, sp[j0 + jj].y,
+                                               sp[j0 + jj].z) << jj;
+            for (; close != 0u; close &= close - 1u) {
+              const int jj = j0 + __ffs(close) - 1;
+              const Q4<R> p = sp[jj];
+              const Q4<R> fv = HAS_F ? sf[jj] : Q4<R>{0, 0, 0, 0};
+              const Q4<R> tv = USE_T ? st[jj] : Q4<R>{0, 0, 0, 0};
+              PK::correct(a.k, a.kw, xi[t], yi[t], zi[t], p, fv, tv, u[t], w[t]);
             }
           }
         }
@@ -514,7 +542,7 @@ mdot_kernel(const MdotArgs<R> a) {
   if (nsplit == 1) {
 #pragma unroll
     for (int t = 0; t < TPT; t++) {
-      const int i = tgt0 + threadIdx.x + t * THREADS;
+      const int i = tgt0 + me + t * TILE;
       if (i >= t_hi) continue;
       const int o = i - t_lo;  // output row
       if (a.U && LMG_IN_BOUNDS(i < N, 5, i)) {
@@ -536,7 +564,7 @@ mdot_kernel(const MdotArgs<R> a) {
   R *mine = a.part + mine_off;
 #pragma unroll
   for (int t = 0; t < TPT; t++) {
-    const int l = threadIdx.x + t * THREADS;
+    const int l = me + t * TILE;
 #pragma unroll
     for (int c = 0; c < NC; c++) {
       if (LMG_IN_BOUNDS(mine_off + (size_t)(NC + c) * BT + l < a.part_cap, 2,
@@ -549,8 +577,8 @@ mdot_kernel(const MdotArgs<R> a) {
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
-    const unsigned prev = LMG_IN_BOUNDS((size_t)tile < a.ticket_cap, 4, tile)
-                              ? atomicAdd(a.ticket + tile, 1u) : 0u;
+    const unsigned prev = LMG_IN_BOUNDS((size_t)blockIdx.x < a.ticket_cap, 4, blockIdx.x)
+                              ? atomicAdd(a.ticket + blockIdx.x, 1u) : 0u;
     s_last = (prev == (unsigned)(nsplit - 1));
   }
   __syncthreads();
@@ -559,7 +587,7 @@ mdot_kernel(const MdotArgs<R> a) {
   const R *base = a.part + ((size_t)tile * nsplit * (2 * NC)) * BT;
 #pragma unroll
   for (int t = 0; t < TPT; t++) {
-    const int l = threadIdx.x + t * THREADS;
+    const int l = me + t * TILE;
     const int i = tgt0 + l;
     R Ss[NC], Cs[NC];
 #pragma unroll
@@ -607,12 +635,13 @@ mdot_kernel(const MdotArgs<R> a) {
       }
     }
   }
-  if (threadIdx.x == 0) a.ticket[tile] = 0u;  // ready for the next launch
+  if (threadIdx.x == 0) a.ticket[blockIdx.x] = 0u;  // ready for the next launch
 }
 
 // Host-side launch description chosen by the planner.
 struct MdotPlan {
-  int threads = 128;
+  int threads = 128;  // targets of a tile per targets-per-thread; sources of one
+  int sub = 1;        // CTAs that share a tile (threads / sub threads each)
   int tpt = 1;
   int nsplit = 1;
   int chunk = 0;

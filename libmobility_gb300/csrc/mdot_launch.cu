@@ -13,9 +13,15 @@ namespace lmg {
 namespace {
 constexpr int kThreads = 128;
 
+// CTAs that share a target tile.  An SM runs FP64 at the rate of two lanes, so
+// a tile's 128 x 128 pairs keep one SM for hundreds of microseconds while a
+// small system has fewer tiles than the GPU has SMs: in FP64 each warp of a
+// tile is a CTA of its own (the sums of a target are the same, bit for bit).
+template <class R> constexpr int kSub = sizeof(R) == 8 ? 4 : 1;
+
 template <class R, int GEOM, bool HF, bool HT, bool ANG, int TPT>
 void *kernel_ptr() {
-  return (void *)mdot_kernel<R, GEOM, HF, HT, ANG, TPT, kThreads>;
+  return (void *)mdot_kernel<R, GEOM, HF, HT, ANG, TPT, kThreads, TPT == 1 ? kSub<R> : 1>;
 }
 
 // kernel pointer for a shape; TPT in {1, 2}
@@ -48,14 +54,16 @@ cudaError_t mdot_plan(const MdotShape &s, int N, int max_src_span, int num_sms, 
   if (sizeof(R) == 4 && N >= 2 * kThreads * num_sms) tpt = 2;
   if (force_tpt == 1 || force_tpt == 2) tpt = force_tpt;
   plan.tpt = tpt;
+  plan.sub = tpt == 1 ? kSub<R> : 1;
   const int bt = kThreads * tpt;
   plan.tiles = (N + bt - 1) / bt;
   void *k = select_kernel<R>(s, tpt);
   if (!k) return cudaErrorInvalidValue;
   int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, 0);
+  cudaError_t e =
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads / plan.sub, 0);
   if (e != cudaSuccess) return e;
-  per_sm = std::max(per_sm, 1);
+  per_sm = std::max(per_sm / plan.sub, 1);
   // two waves of CTAs, and at least 32 CTAs per SM: kernels with few
   // resident CTAs (the wall kernel holds 5 per SM) otherwise lose a large
   // share of the last wave; measured on wall N = 16384 / 65536, 32 splits
@@ -76,7 +84,7 @@ cudaError_t mdot_plan(const MdotShape &s, int N, int max_src_span, int num_sms, 
   plan.chunk = chunk;
   const int nc = s.ang ? 6 : 3;
   plan.part_elems = nsplit > 1 ? (size_t)plan.tiles * nsplit * 2 * nc * bt : 0;
-  plan.tickets = nsplit > 1 ? (size_t)plan.tiles : 0;
+  plan.tickets = nsplit > 1 ? (size_t)plan.tiles * plan.sub : 0;
   return cudaSuccess;
 }
 
@@ -89,10 +97,10 @@ cudaError_t mdot_launch(const MdotShape &s, const MdotArgs<R> &args, const MdotP
   a.chunk = plan.chunk;
   a.part_cap = plan.part_elems;
   a.ticket_cap = plan.tickets;
-  dim3 grid(plan.tiles, plan.nsplit);
+  dim3 grid(plan.tiles * plan.sub, plan.nsplit);
   void *params[] = {(void *)&a};
   count_launch();
-  return cudaLaunchKernel(k, grid, dim3(plan.threads), params, 0, stream);
+  return cudaLaunchKernel(k, grid, dim3(plan.threads / plan.sub), params, 0, stream);
 }
 
 // this translation unit's bounds status (the checked build; 0 otherwise)
