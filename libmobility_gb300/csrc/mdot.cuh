@@ -25,6 +25,7 @@
 //     needs no clearing between launches and nothing waits on anything.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 #include "bounds.cuh"
@@ -51,6 +52,7 @@ template <class R> struct MdotArgs {
   int tgt_begin, tgt_end;
   int nper;              // equal batch size when sys_begin == nullptr
   int chunk;             // sources per split (multiple of TILE)
+  int group;             // consecutive splits summed on their own first
   R inv_a;               // 1/a
   PairConst<R> k;
   WallConst kw;          // fused all-blocks wall constants (FP32 path)
@@ -105,8 +107,9 @@ template <class R, int GEOM, bool HAS_F, bool HAS_T, bool ANG> struct PairKernel
   // for an overlapping or self pair, and exact for r >= 2a), and the wall
   // images take the pair formula even for the self pair.  The caller
   // replaces the fast value by the exact one for the pairs with r^2 < 4
-  // (correct() below).
-  template <bool EXACT = true>
+  // (correct() below).  NEAR = false leaves the exact form's branches out, for
+  // pairs known to be at least 2a apart.
+  template <bool EXACT = true, bool NEAR = EXACT>
   static __device__ __forceinline__ R eval(const PairConst<R> &k, const WallConst &kw, R xi,
                                            R yi, R zi, const Q4<R> &p, const Q4<R> &fv,
                                            const Q4<R> &tv, Vec3<R> &u, Vec3<R> &w) {
@@ -121,7 +124,7 @@ template <class R, int GEOM, bool HAS_F, bool HAS_T, bool ANG> struct PairKernel
     const R r2 = fmaR(dx, dx, fmaR(dy, dy, dz * dz));
     R f = 0, G = 0, fw = 0, Gw = 0, c = 0;
     if constexpr (EXACT) {
-      rpy_coefficients<R, UF, WT, UT || WF, true>(k, r2, dev_rsqrt<R>(r2), f, G, fw, Gw, c);
+      rpy_coefficients<R, UF, WT, UT || WF, NEAR>(k, r2, dev_rsqrt<R>(r2), f, G, fw, Gw, c);
     } else {
       const R r2c = below4(r2) ? R(4) : r2;
       rpy_coefficients<R, UF, WT, UT || WF, false>(k, r2c, rsqrt_normal<R>(r2c), f, G, fw, Gw,
@@ -157,7 +160,7 @@ template <class R, int GEOM, bool HAS_F, bool HAS_T, bool ANG> struct PairKernel
       Vec3<R> cu = {0, 0, 0}, cw = {0, 0, 0}, ct = {0, 0, 0}, cf = {0, 0, 0};
       const Vec3<R> F3 = {fv.x, fv.y, fv.z};
       const Vec3<R> T3 = {tv.x, tv.y, tv.z};
-      if (!EXACT || r2 > R(0)) {
+      if (!NEAR || r2 > R(0)) {
         const R iRz = dev_div<R>(R(1), Rz);
         const R hj = p.z * iRz;  // h_j / R_z
         if (UF) wall_uf_pair<R>(ex, ey, ez, iR, hj, F3, cu);
@@ -193,6 +196,11 @@ template <class R, int GEOM, bool HAS_F, bool HAS_T, bool ANG> struct PairKernel
     const R dx = xi - xj, dy = yi - yj, dz = zi - zj;
     return below4(fmaR(dx, dx, fmaR(dy, dy, dz * dz)));
   }
+  // The same with room for another rounding of r^2.
+  static __device__ __forceinline__ bool maybe_near(R xi, R yi, R zi, R xj, R yj, R zj) {
+    const R dx = xi - xj, dy = yi - yj, dz = zi - zj;
+    return below4(R(0.96875) * fmaR(dx, dx, fmaR(dy, dy, dz * dz)));
+  }
 
   // For a pair with r^2 < 4 already added in the fast form: adds
   // (exact - fast).  Both are O(1) there, so the difference is accurate.
@@ -211,7 +219,8 @@ template <class R, int GEOM, bool HAS_F, bool HAS_T, bool ANG> struct PairKernel
   }
 };
 
-template <class R, int GEOM, bool HAS_F, bool HAS_T, bool ANG, int TPT, int TILE, int SUB>
+template <class R, int GEOM, bool HAS_F, bool HAS_T, bool ANG, int TPT, int TILE, int SUB,
+          bool DENSE>
 __global__ void __launch_bounds__(TILE / SUB)
 mdot_kernel(const MdotArgs<R> a) {
   using PK = PairKernel<R, GEOM, HAS_F, HAS_T, ANG>;
@@ -235,6 +244,11 @@ mdot_kernel(const MdotArgs<R> a) {
   __shared__ Q4<R> sf[HAS_F && !SOA ? TILE : 1];
   __shared__ Q4<R> st[USE_T && !SOA ? TILE : 1];
   __shared__ __align__(16) float sv[NSV][SOA ? TILE : 4];
+  // packed wall pairs: events (lane, packed pair) closer than 2a and their values
+  constexpr bool EVENTS = DENSE && GEOM == kWall && (PACK || PACK_UF);
+  constexpr int kCloseCap = 64;
+  __shared__ unsigned short s_event[EVENTS ? THREADS / 32 : 1][EVENTS ? kCloseCap : 1];
+  __shared__ float2 s_close[EVENTS ? THREADS / 32 : 1][EVENTS ? NC : 1][EVENTS ? kCloseCap : 1];
   __shared__ int s_last;
 
   const int N = a.N;
@@ -325,58 +339,259 @@ mdot_kernel(const MdotArgs<R> a) {
     }
     __syncthreads();
     const int n_here = min(TILE, c_end - ts);
-    if constexpr (PACK) {
-      if (uniform && n_here == TILE) {
-        V3p u2[TPT], w2[TPT];
+    if (!(uniform && n_here == TILE)) {
+      // a ragged tile or one over a batch boundary: one source after another;
+      // two without branches where no target of the warp is close to either (not
+      // the block-by-block wall form, whose sums the compiler would contract
+      // another way there)
+      auto one = [&](int jj, auto near_tag) {
+        constexpr bool NEAR = decltype(near_tag)::value;
+        const int j = ts + jj;
+        Q4<R> p, fv = {0, 0, 0, 0}, tv = {0, 0, 0, 0};
+        if constexpr (SOA) {
+          p = {sv[0][jj], sv[1][jj], sv[2][jj], 0};
+          fv = {sv[3][jj], sv[4][jj], sv[5][jj], 0};
+          if constexpr (PACK) tv = {sv[6][jj], sv[7][jj], sv[8][jj], 0};
+        } else {
+          p = sp[jj];
+          if (HAS_F) fv = sf[jj];
+          if (USE_T) tv = st[jj];
+        }
 #pragma unroll
         for (int t = 0; t < TPT; t++) {
-          u2[t] = {bc(0.f), bc(0.f), bc(0.f)};
-          w2[t] = {bc(0.f), bc(0.f), bc(0.f)};
-        }
-#pragma unroll 1
-        for (int jj = 0; jj < TILE; jj += 4) {
-          float4 q[9];
-#pragma unroll
-          for (int c = 0; c < 9; c++) q[c] = *reinterpret_cast<const float4 *>(&sv[c][jj]);
-#pragma unroll
-          for (int h = 0; h < 2; h++) {
-            F2 v[9];
-#pragma unroll
-            for (int c = 0; c < 9; c++) v[c] = h ? mk2(q[c].z, q[c].w) : mk2(q[c].x, q[c].y);
-#pragma unroll
-            for (int t = 0; t < TPT; t++)
-              wall_pair_fused_x2(a.k, a.kw, bc(xi[t]), bc(yi[t]), bc(zi[t]), v[0], v[1], v[2],
-                                 v[3], v[4], v[5], v[6], v[7], v[8], u2[t], w2[t]);
+          if (!NEAR || (j >= lo[t] && j < hi[t])) {
+            if constexpr (PACK)
+              wall_pair_fused<NEAR>(a.k, a.kw, xi[t], yi[t], zi[t], p.x, p.y, p.z, fv.x, fv.y,
+                                    fv.z, tv.x, tv.y, tv.z, u[t], w[t]);
+            else
+              PK::template eval<true, NEAR>(a.k, a.kw, xi[t], yi[t], zi[t], p, fv, tv, u[t], w[t]);
           }
         }
+      };
+      auto close = [&](int jj) {
+        bool c = false;
 #pragma unroll
-        for (int t = 0; t < TPT; t++) {  // the two lanes hold even and odd sources
-          u[t].x += u2[t].x.v.x + u2[t].x.v.y;
-          u[t].y += u2[t].y.v.x + u2[t].y.v.y;
-          u[t].z += u2[t].z.v.x + u2[t].z.v.y;
+        for (int t = 0; t < TPT; t++) {
+          if constexpr (SOA) c = c || PK::maybe_near(xi[t], yi[t], zi[t], sv[0][jj], sv[1][jj], sv[2][jj]);
+          else c = c || PK::maybe_near(xi[t], yi[t], zi[t], sp[jj].x, sp[jj].y, sp[jj].z);
+        }
+        return c;
+      };
+      int jj = 0;
+      if ((PACK || GEOM == kOpen) && uniform) {
+#pragma unroll 1
+        for (; jj + 1 < n_here; jj += 2) {
+          const bool c = close(jj) || close(jj + 1);
+          if (__any_sync(0xffffffffu, c)) {
+            one(jj, std::true_type());
+            one(jj + 1, std::true_type());
+          } else {
+            one(jj, std::false_type());
+            one(jj + 1, std::false_type());
+          }
+        }
+      }
+#pragma unroll 1
+      for (; jj < n_here; jj++) one(jj, std::true_type());
+    } else if constexpr (EVENTS) {
+      // Two sources per instruction, 32 sources at a time.  Packed pairs with a
+      // lane closer than 2a are found first; their scalar evaluations are dealt
+      // out over the warp's lanes, and the sums then take every packed pair in
+      // source order.  (Evaluated in place, each cost the whole warp two scalar
+      // evaluations: most of the time of a few hundred particles.)
+      const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+      V3p u2[TPT], w2[TPT];
+#pragma unroll
+      for (int t = 0; t < TPT; t++) {
+        u2[t] = {bc(0.f), bc(0.f), bc(0.f)};
+        w2[t] = {bc(0.f), bc(0.f), bc(0.f)};
+      }
+      auto pick = [&](int c, int pp) {  // component c of packed sources 2 pp, 2 pp + 1
+        const float2 x = *reinterpret_cast<const float2 *>(&sv[c][2 * pp]);
+        return mk2(x.x, x.y);
+      };
+#pragma unroll 1
+      for (int p0 = 0; p0 < TILE / 2; p0 += 16) {
+        unsigned close[TPT], any[TPT];  // bit pp: packed pair p0 + pp
+#pragma unroll
+        for (int t = 0; t < TPT; t++) {
+          close[t] = 0u;
+#pragma unroll 8
+          for (int pp = 0; pp < 16; pp++)
+            close[t] |= (unsigned)wall_close(bc(xi[t]), bc(yi[t]), bc(zi[t]), pick(0, p0 + pp),
+                                             pick(1, p0 + pp), pick(2, p0 + pp)) << pp;
+          any[t] = __reduce_or_sync(0xffffffffu, close[t]);
+        }
+#pragma unroll
+        for (int t = 0; t < TPT; t++) {
+          int mine = 0, total = 0;  // this lane's first event, events of the warp
+          if (any[t]) {
+            int incl = __popc(close[t]);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+              const int up = __shfl_up_sync(0xffffffffu, incl, o);
+              if (lane >= o) incl += up;
+            }
+            mine = incl - __popc(close[t]);
+            total = __shfl_sync(0xffffffffu, incl, 31);
+            if (total <= kCloseCap) {
+              int e = mine;
+              for (unsigned c = close[t]; c != 0u; c &= c - 1u)
+                s_event[wid][e++] = (unsigned short)((lane << 4) | (__ffs(c) - 1));
+              __syncwarp();
+              for (int e0 = 0; e0 < total; e0 += 32) {
+                const int ev = e0 + lane < total ? s_event[wid][e0 + lane] : 0;
+                const float ox = __shfl_sync(0xffffffffu, xi[t], ev >> 4),
+                            oy = __shfl_sync(0xffffffffu, yi[t], ev >> 4),
+                            oz = __shfl_sync(0xffffffffu, zi[t], ev >> 4);
+                if (e0 + lane < total) {
+                  F2 v[9];
+#pragma unroll
+                  for (int c = 0; c < 9; c++) v[c] = c < NSV ? pick(c < NSV ? c : 0, p0 + (ev & 15)) : bc(0.f);
+                  V3p cu, cw;
+                  wall_close_x2(a.k, a.kw, ox, oy, oz, v, cu, cw);
+                  const F2 r[6] = {cu.x, cu.y, cu.z, cw.x, cw.y, cw.z};
+#pragma unroll
+                  for (int c = 0; c < NC; c++) s_close[wid][c][e0 + lane] = r[c].v;
+                }
+              }
+              __syncwarp();
+            }
+          }
+#pragma unroll 1
+          for (int pp = 0; pp < 16; pp += 2) {
+            auto far = [&](int q) {
+              F2 v[9];
+#pragma unroll
+              for (int c = 0; c < 9; c++) v[c] = c < NSV ? pick(c < NSV ? c : 0, p0 + q) : bc(0.f);
+              if constexpr (PACK)
+                wall_pair_far_x2(a.k, a.kw, bc(xi[t]), bc(yi[t]), bc(zi[t]), v[0], v[1], v[2],
+                                 v[3], v[4], v[5], v[6], v[7], v[8], u2[t], w2[t]);
+              else
+                wall_uf_far_x2(a.k, a.kw, bc(xi[t]), bc(yi[t]), bc(zi[t]), v[0], v[1], v[2],
+                               v[3], v[4], v[5], u2[t]);
+            };
+            if (((any[t] >> pp) & 3u) == 0u) {
+              far(pp);
+              far(pp + 1);
+              continue;
+            }
+#pragma unroll 1
+            for (int q = pp; q < pp + 2; q++) {
+              if ((close[t] >> q) & 1u) {
+                V3p cu, cw;
+                if (total <= kCloseCap) {
+                  F2 r[6];
+#pragma unroll
+                  for (int c = 0; c < 6; c++) r[c] = {s_close[wid][c < NC ? c : 0][mine]};
+                  cu = {r[0], r[1], r[2]};
+                  cw = {r[3], r[4], r[5]};
+                  mine++;
+                } else {
+                  F2 v[9];
+#pragma unroll
+                  for (int c = 0; c < 9; c++) v[c] = c < NSV ? pick(c < NSV ? c : 0, p0 + q) : bc(0.f);
+                  wall_close_x2(a.k, a.kw, xi[t], yi[t], zi[t], v, cu, cw);
+                }
+                u2[t].x = u2[t].x + cu.x;
+                u2[t].y = u2[t].y + cu.y;
+                u2[t].z = u2[t].z + cu.z;
+                if constexpr (PACK) {
+                  w2[t].x = w2[t].x + cw.x;
+                  w2[t].y = w2[t].y + cw.y;
+                  w2[t].z = w2[t].z + cw.z;
+                }
+              } else {
+                far(q);
+              }
+            }
+          }
+          __syncwarp();  // the events' place is used again
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < TPT; t++) {  // the two lanes hold even and odd sources
+        u[t].x += u2[t].x.v.x + u2[t].x.v.y;
+        u[t].y += u2[t].y.v.x + u2[t].y.v.y;
+        u[t].z += u2[t].z.v.x + u2[t].z.v.y;
+        if constexpr (PACK) {
           w[t].x += w2[t].x.v.x + w2[t].x.v.y;
           w[t].y += w2[t].y.v.x + w2[t].y.v.y;
           w[t].z += w2[t].z.v.x + w2[t].z.v.y;
         }
-      } else {
-        for (int jj = 0; jj < n_here; jj++) {
-          const int j = ts + jj;
+      }
+    } else if constexpr (PACK) {
+      V3p u2[TPT], w2[TPT];
+#pragma unroll
+      for (int t = 0; t < TPT; t++) {
+        u2[t] = {bc(0.f), bc(0.f), bc(0.f)};
+        w2[t] = {bc(0.f), bc(0.f), bc(0.f)};
+      }
+#pragma unroll 1
+      for (int jj = 0; jj < TILE; jj += 4) {
+        float4 q[9];
+#pragma unroll
+        for (int c = 0; c < 9; c++) q[c] = *reinterpret_cast<const float4 *>(&sv[c][jj]);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          F2 v[9];
+#pragma unroll
+          for (int c = 0; c < 9; c++) v[c] = h ? mk2(q[c].z, q[c].w) : mk2(q[c].x, q[c].y);
 #pragma unroll
           for (int t = 0; t < TPT; t++)
-            if (j >= lo[t] && j < hi[t])
-              wall_pair_fused(a.k, a.kw, xi[t], yi[t], zi[t], sv[0][jj], sv[1][jj], sv[2][jj],
-                              sv[3][jj], sv[4][jj], sv[5][jj], sv[6][jj], sv[7][jj], sv[8][jj],
-                              u[t], w[t]);
+            wall_pair_fused_x2(a.k, a.kw, xi[t], yi[t], zi[t], v, u2[t], w2[t]);
         }
       }
-    } else if constexpr (PACK_UF && GEOM == kWall) {
-      if (uniform && n_here == TILE) {
-        // two sources per instruction; close pairs fall back lane by lane
-        V3p u2[TPT];
 #pragma unroll
-        for (int t = 0; t < TPT; t++) u2[t] = {bc(0.f), bc(0.f), bc(0.f)};
+      for (int t = 0; t < TPT; t++) {  // the two lanes hold even and odd sources
+        u[t].x += u2[t].x.v.x + u2[t].x.v.y;
+        u[t].y += u2[t].y.v.x + u2[t].y.v.y;
+        u[t].z += u2[t].z.v.x + u2[t].z.v.y;
+        w[t].x += w2[t].x.v.x + w2[t].x.v.y;
+        w[t].y += w2[t].y.v.x + w2[t].y.v.y;
+        w[t].z += w2[t].z.v.x + w2[t].z.v.y;
+      }
+    } else if constexpr (PACK_UF && GEOM == kWall) {
+      // two sources per instruction; close pairs fall back lane by lane
+      V3p u2[TPT];
+#pragma unroll
+      for (int t = 0; t < TPT; t++) u2[t] = {bc(0.f), bc(0.f), bc(0.f)};
 #pragma unroll 1
-        for (int jj = 0; jj < TILE; jj += 4) {
+      for (int jj = 0; jj < TILE; jj += 4) {
+        float4 q[6];
+#pragma unroll
+        for (int c = 0; c < 6; c++) q[c] = *reinterpret_cast<const float4 *>(&sv[c][jj]);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          F2 v[9];
+#pragma unroll
+          for (int c = 0; c < 9; c++)
+            v[c] = c >= 6 ? bc(0.f)
+                          : (h ? mk2(q[c % 6].z, q[c % 6].w) : mk2(q[c % 6].x, q[c % 6].y));
+#pragma unroll
+          for (int t = 0; t < TPT; t++)
+            wall_uf_pair_x2(a.k, a.kw, xi[t], yi[t], zi[t], v, u2[t]);
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < TPT; t++) {  // the two lanes hold even and odd sources
+        u[t].x += u2[t].x.v.x + u2[t].x.v.y;
+        u[t].y += u2[t].y.v.x + u2[t].y.v.y;
+        u[t].z += u2[t].z.v.x + u2[t].z.v.y;
+      }
+    } else if constexpr (PACK_UF) {
+      // as the scalar full-tile path below, two sources per instruction
+#pragma unroll 1
+      for (int j0 = 0; j0 < TILE; j0 += 32) {
+        V3p u2[TPT];
+        float2 mr2[TPT];
+#pragma unroll
+        for (int t = 0; t < TPT; t++) {
+          u2[t] = {bc(0.f), bc(0.f), bc(0.f)};
+          mr2[t] = make_float2(4.f, 4.f);
+        }
+#pragma unroll 2
+        for (int jj = j0; jj < j0 + 32; jj += 4) {
           float4 q[6];
 #pragma unroll
           for (int c = 0; c < 6; c++) q[c] = *reinterpret_cast<const float4 *>(&sv[c][jj]);
@@ -387,90 +602,36 @@ mdot_kernel(const MdotArgs<R> a) {
             for (int c = 0; c < 6; c++) v[c] = h ? mk2(q[c].z, q[c].w) : mk2(q[c].x, q[c].y);
 #pragma unroll
             for (int t = 0; t < TPT; t++)
-              wall_uf_pair_x2(a.k, a.kw, bc(xi[t]), bc(yi[t]), bc(zi[t]), v[0], v[1], v[2],
-                              v[3], v[4], v[5], u2[t]);
+              open_uf_pair_x2(a.k, bc(xi[t]), bc(yi[t]), bc(zi[t]), v[0], v[1], v[2], v[3],
+                              v[4], v[5], u2[t], mr2[t]);
           }
         }
+        bool near = false;
 #pragma unroll
-        for (int t = 0; t < TPT; t++) {  // the two lanes hold even and odd sources
+        for (int t = 0; t < TPT; t++) {
           u[t].x += u2[t].x.v.x + u2[t].x.v.y;
           u[t].y += u2[t].y.v.x + u2[t].y.v.y;
           u[t].z += u2[t].z.v.x + u2[t].z.v.y;
+          near = near || fminf(mr2[t].x, mr2[t].y) < 4.f;
         }
-      } else {
-        for (int jj = 0; jj < n_here; jj++) {
-          const int j = ts + jj;
-          const Q4<R> p = {sv[0][jj], sv[1][jj], sv[2][jj], 0};
-          const Q4<R> fv = {sv[3][jj], sv[4][jj], sv[5][jj], 0};
-#pragma unroll
-          for (int t = 0; t < TPT; t++)
-            if (j >= lo[t] && j < hi[t]) PK::eval(a.k, a.kw, xi[t], yi[t], zi[t], p, fv, fv, u[t], w[t]);
-        }
-      }
-    } else if constexpr (PACK_UF) {
-      if (uniform && n_here == TILE) {
-        // as the scalar full-tile path below, two sources per instruction
-#pragma unroll 1
-        for (int j0 = 0; j0 < TILE; j0 += 32) {
-          V3p u2[TPT];
-          float2 mr2[TPT];
+        if (__any_sync(0xffffffffu, near)) {
 #pragma unroll
           for (int t = 0; t < TPT; t++) {
-            u2[t] = {bc(0.f), bc(0.f), bc(0.f)};
-            mr2[t] = make_float2(4.f, 4.f);
-          }
-#pragma unroll 2
-          for (int jj = j0; jj < j0 + 32; jj += 4) {
-            float4 q[6];
-#pragma unroll
-            for (int c = 0; c < 6; c++) q[c] = *reinterpret_cast<const float4 *>(&sv[c][jj]);
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-              F2 v[6];
-#pragma unroll
-              for (int c = 0; c < 6; c++) v[c] = h ? mk2(q[c].z, q[c].w) : mk2(q[c].x, q[c].y);
-#pragma unroll
-              for (int t = 0; t < TPT; t++)
-                open_uf_pair_x2(a.k, bc(xi[t]), bc(yi[t]), bc(zi[t]), v[0], v[1], v[2], v[3],
-                                v[4], v[5], u2[t], mr2[t]);
-            }
-          }
-          bool near = false;
-#pragma unroll
-          for (int t = 0; t < TPT; t++) {
-            u[t].x += u2[t].x.v.x + u2[t].x.v.y;
-            u[t].y += u2[t].y.v.x + u2[t].y.v.y;
-            u[t].z += u2[t].z.v.x + u2[t].z.v.y;
-            near = near || fminf(mr2[t].x, mr2[t].y) < 4.f;
-          }
-          if (__any_sync(0xffffffffu, near)) {
-#pragma unroll
-            for (int t = 0; t < TPT; t++) {
-              unsigned close = 0u;
+            unsigned close = 0u;
 #pragma unroll 8
-              for (int jj = 0; jj < 32; jj++)
-                close |= (unsigned)PK::near_pair(xi[t], yi[t], zi[t], sv[0][j0 + jj],
-                                                 sv[1][j0 + jj], sv[2][j0 + jj]) << jj;
-              for (; close != 0u; close &= close - 1u) {
-                const int jj = j0 + __ffs(close) - 1;
-                const Q4<R> p = {sv[0][jj], sv[1][jj], sv[2][jj], 0};
-                const Q4<R> fv = {sv[3][jj], sv[4][jj], sv[5][jj], 0};
-                PK::correct(a.k, a.kw, xi[t], yi[t], zi[t], p, fv, fv, u[t], w[t]);
-              }
+            for (int jj = 0; jj < 32; jj++)
+              close |= (unsigned)PK::near_pair(xi[t], yi[t], zi[t], sv[0][j0 + jj],
+                                               sv[1][j0 + jj], sv[2][j0 + jj]) << jj;
+            for (; close != 0u; close &= close - 1u) {
+              const int jj = j0 + __ffs(close) - 1;
+              const Q4<R> p = {sv[0][jj], sv[1][jj], sv[2][jj], 0};
+              const Q4<R> fv = {sv[3][jj], sv[4][jj], sv[5][jj], 0};
+              PK::correct(a.k, a.kw, xi[t], yi[t], zi[t], p, fv, fv, u[t], w[t]);
             }
           }
         }
-      } else {
-        for (int jj = 0; jj < n_here; jj++) {
-          const int j = ts + jj;
-          const Q4<R> p = {sv[0][jj], sv[1][jj], sv[2][jj], 0};
-          const Q4<R> fv = {sv[3][jj], sv[4][jj], sv[5][jj], 0};
-#pragma unroll
-          for (int t = 0; t < TPT; t++)
-            if (j >= lo[t] && j < hi[t]) PK::eval(a.k, a.kw, xi[t], yi[t], zi[t], p, fv, fv, u[t], w[t]);
-        }
       }
-    } else if (uniform && n_here == TILE) {
+    } else {
       // Fast form for every pair, 32 sources at a time; then, in a warp where
       // some target met a pair closer than 2a among those 32 (its self pair,
       // or an overlap), those targets swap the fast value of such pairs for
@@ -513,16 +674,6 @@ mdot_kernel(const MdotArgs<R> a) {
             }
           }
         }
-      }
-    } else {
-      for (int jj = 0; jj < n_here; jj++) {
-        const int j = ts + jj;
-        const Q4<R> p = sp[jj];
-        const Q4<R> fv = HAS_F ? sf[jj] : Q4<R>{0, 0, 0, 0};
-        const Q4<R> tv = USE_T ? st[jj] : Q4<R>{0, 0, 0, 0};
-#pragma unroll
-        for (int t = 0; t < TPT; t++)
-          if (j >= lo[t] && j < hi[t]) PK::eval(a.k, a.kw, xi[t], yi[t], zi[t], p, fv, tv, u[t], w[t]);
       }
     }
     // fold the tile's partial sums
@@ -589,9 +740,10 @@ mdot_kernel(const MdotArgs<R> a) {
   for (int t = 0; t < TPT; t++) {
     const int l = me + t * TILE;
     const int i = tgt0 + l;
-    R Ss[NC], Cs[NC];
+    R Ss[NC], Cs[NC], Sg[NC], Cg[NC];
 #pragma unroll
-    for (int c = 0; c < NC; c++) { Ss[c] = 0; Cs[c] = 0; }
+    for (int c = 0; c < NC; c++) { Ss[c] = 0; Cs[c] = 0; Sg[c] = 0; Cg[c] = 0; }
+    int left = a.group;
     // UNR splits' partials are loaded before any is folded, so that many L2
     // reads are in flight at once (the fold order stays the split order)
     constexpr int UNR = 24 / NC;
@@ -616,8 +768,18 @@ mdot_kernel(const MdotArgs<R> a) {
       for (int u = 0; u < UNR; u++) {
 #pragma unroll
         for (int c = 0; c < NC; c++) {
-          if (COMP) fold(Ss[c], Cs[c], sv[u][c]); else Ss[c] += sv[u][c];
-          Cs[c] += cv[u][c];
+          if (COMP) fold(Sg[c], Cg[c], sv[u][c]); else Sg[c] += sv[u][c];
+          Cg[c] += cv[u][c];
+        }
+        if (--left == 0 || s0 + u >= nsplit - 1) {
+          left = a.group;
+#pragma unroll
+          for (int c = 0; c < NC; c++) {
+            if (COMP) fold(Ss[c], Cs[c], Sg[c]); else Ss[c] += Sg[c];
+            Cs[c] += Cg[c];
+            Sg[c] = 0;
+            Cg[c] = 0;
+          }
         }
       }
     }
@@ -642,9 +804,11 @@ mdot_kernel(const MdotArgs<R> a) {
 struct MdotPlan {
   int threads = 128;  // targets of a tile per targets-per-thread; sources of one
   int sub = 1;        // CTAs that share a tile (threads / sub threads each)
+  bool dense = false; // close wall pairs dealt out beforehand (kDenseSpan)
   int tpt = 1;
   int nsplit = 1;
   int chunk = 0;
+  int group = 1;      // splits summed on their own first (MdotArgs::group)
   int tiles = 0;
   size_t part_elems = 0;  // scratch elements of R needed
   size_t tickets = 0;

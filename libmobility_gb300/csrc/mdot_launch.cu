@@ -19,17 +19,28 @@ constexpr int kThreads = 128;
 // tile is a CTA of its own (the sums of a target are the same, bit for bit).
 template <class R> constexpr int kSub = sizeof(R) == 8 ? 4 : 1;
 
+// Packed wall pairs (FP32): up to this many sources a batch, close pairs are
+// dealt out over the warp before the sums (DENSE); beyond, they are rare and
+// are evaluated where they are met, with fewer registers.  Above a wall at one
+// particle per unit area, dealt out and in place: N = 300 with torques 52 and
+// 64 us, 2048 41 and 45 us, 16384 1475 and 1397 us.
+constexpr int kDenseSpan = 4096;
+
 template <class R, int GEOM, bool HF, bool HT, bool ANG, int TPT>
-void *kernel_ptr() {
-  return (void *)mdot_kernel<R, GEOM, HF, HT, ANG, TPT, kThreads, TPT == 1 ? kSub<R> : 1>;
+void *kernel_ptr(bool dense) {
+  constexpr int S = TPT == 1 ? kSub<R> : 1;
+  if constexpr (sizeof(R) == 4 && GEOM == kWall && HF && HT == ANG && TPT == 1) {
+    if (dense) return (void *)mdot_kernel<R, GEOM, HF, HT, ANG, TPT, kThreads, S, true>;
+  }
+  return (void *)mdot_kernel<R, GEOM, HF, HT, ANG, TPT, kThreads, S, false>;
 }
 
 // kernel pointer for a shape; TPT in {1, 2}
 template <class R>
-void *select_kernel(const MdotShape &s, int tpt) {
+void *select_kernel(const MdotShape &s, int tpt, bool dense) {
 #define LMG_SEL(G, HF, HT, A)                                              \
   if (s.geom == G && s.has_f == HF && s.has_t == HT && s.ang == A)         \
-    return tpt == 2 ? kernel_ptr<R, G, HF, HT, A, 2>() : kernel_ptr<R, G, HF, HT, A, 1>();
+    return tpt == 2 ? kernel_ptr<R, G, HF, HT, A, 2>(dense) : kernel_ptr<R, G, HF, HT, A, 1>(dense);
   LMG_SEL(kOpen, true, false, false)
   LMG_SEL(kOpen, true, false, true)
   LMG_SEL(kOpen, false, true, true)
@@ -57,7 +68,8 @@ cudaError_t mdot_plan(const MdotShape &s, int N, int max_src_span, int num_sms, 
   plan.sub = tpt == 1 ? kSub<R> : 1;
   const int bt = kThreads * tpt;
   plan.tiles = (N + bt - 1) / bt;
-  void *k = select_kernel<R>(s, tpt);
+  // (the splits are planned for the kernel without it, whichever runs)
+  void *k = select_kernel<R>(s, tpt, false);
   if (!k) return cudaErrorInvalidValue;
   int per_sm = 0;
   cudaError_t e =
@@ -80,8 +92,19 @@ cudaError_t mdot_plan(const MdotShape &s, int N, int max_src_span, int num_sms, 
   if (chunk <= 0) chunk = kThreads;
   nsplit = (max_src_span + chunk - 1) / chunk;
   if (nsplit < 1) nsplit = 1;
+  // With few CTAs, a split of several source tiles is cut into one split per
+  // tile, and the reduction sums those of a former split first: the same sums
+  // bit for bit, on more SMs (a span of 2000 gave 8 splits of 256 sources, one
+  // of 2048 gave 16 of 128: N = 2000 wall with torques 54 us, N = 2048 47).
+  const long warps = (long)plan.tiles * nsplit * (kThreads / 32);
+  if (force_split <= 0 && chunk > kThreads && warps < 8L * num_sms) {
+    plan.group = chunk / kThreads;
+    chunk = kThreads;
+    nsplit = (max_src_span + chunk - 1) / chunk;
+  }
   plan.nsplit = nsplit;
   plan.chunk = chunk;
+  plan.dense = max_src_span <= kDenseSpan;
   const int nc = s.ang ? 6 : 3;
   plan.part_elems = nsplit > 1 ? (size_t)plan.tiles * nsplit * 2 * nc * bt : 0;
   plan.tickets = nsplit > 1 ? (size_t)plan.tiles * plan.sub : 0;
@@ -91,10 +114,11 @@ cudaError_t mdot_plan(const MdotShape &s, int N, int max_src_span, int num_sms, 
 template <class R>
 cudaError_t mdot_launch(const MdotShape &s, const MdotArgs<R> &args, const MdotPlan &plan,
                         cudaStream_t stream) {
-  void *k = select_kernel<R>(s, plan.tpt);
+  void *k = select_kernel<R>(s, plan.tpt, plan.dense);
   if (!k) return cudaErrorInvalidValue;
   MdotArgs<R> a = args;
   a.chunk = plan.chunk;
+  a.group = plan.group;
   a.part_cap = plan.part_elems;
   a.ticket_cap = plan.tickets;
   dim3 grid(plan.tiles * plan.sub, plan.nsplit);

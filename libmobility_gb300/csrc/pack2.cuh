@@ -39,32 +39,38 @@ struct V3p {
   F2 x, y, z;
 };
 
-// Packed version of wall_pair_fused (rpy_pair.cuh) for two targets (lanes of
-// xi, yi, hi) and one source whose values arrive already duplicated in both
-// lanes (Xj = {xj, xj}, ...).  Same formulas, same order of operations per
-// lane; pairs with r = 0 (self) or r < 2a (overlap) in either lane are
-// evaluated lane by lane with the scalar code.
-__device__ __forceinline__ void wall_pair_fused_x2(
+// Whether either lane's pair is closer than 2a (the self pair included): such a
+// packed pair is evaluated lane by lane with the scalar code
+// (wall_close_x2), the others with wall_pair_far_x2 / wall_uf_far_x2.
+__device__ __forceinline__ bool wall_close(F2 xi, F2 yi, F2 hi, F2 Xj, F2 Yj, F2 Hj) {
+  const F2 dx = xi - Xj, dy = yi - Yj, dz = hi - Hj;
+  const F2 r2 = fma2(dz, dz, fma2(dx, dx, dy * dy));
+  return r2.v.x < 4.0f || r2.v.y < 4.0f;
+}
+
+// The scalar evaluation of both lanes, summed from zero: (lane 0, lane 1) of u
+// and w.  v: X, Y, H, F and T of the two sources.
+__device__ __forceinline__ void wall_close_x2(const PairConst<float> &k, const WallConst &K,
+                                              float xi, float yi, float hi, const F2 (&v)[9],
+                                              V3p &u, V3p &w) {
+  Vec3<float> u0 = {0, 0, 0}, w0 = {0, 0, 0}, u1 = {0, 0, 0}, w1 = {0, 0, 0};
+  wall_pair_fused(k, K, xi, yi, hi, v[0].v.x, v[1].v.x, v[2].v.x, v[3].v.x, v[4].v.x, v[5].v.x,
+                  v[6].v.x, v[7].v.x, v[8].v.x, u0, w0);
+  wall_pair_fused(k, K, xi, yi, hi, v[0].v.y, v[1].v.y, v[2].v.y, v[3].v.y, v[4].v.y, v[5].v.y,
+                  v[6].v.y, v[7].v.y, v[8].v.y, u1, w1);
+  u = {mk2(u0.x, u1.x), mk2(u0.y, u1.y), mk2(u0.z, u1.z)};
+  w = {mk2(w0.x, w1.x), mk2(w0.y, w1.y), mk2(w0.z, w1.z)};
+}
+
+// Packed version of wall_pair_fused (rpy_pair.cuh) for one target (both lanes
+// of xi, yi, hi) and two sources, both at least 2a away.  Same formulas, same
+// order of operations per lane.
+__device__ __forceinline__ void wall_pair_far_x2(
     const PairConst<float> &k, const WallConst &K, F2 xi, F2 yi, F2 hi, F2 Xj, F2 Yj, F2 Hj,
     F2 Fx, F2 Fy, F2 Fz, F2 Tx, F2 Ty, F2 Tz, V3p &u, V3p &w) {
   const F2 dx = xi - Xj, dy = yi - Yj, dz = hi - Hj;
   const F2 sxy = fma2(dx, dx, dy * dy);
   const F2 r2 = fma2(dz, dz, sxy);
-  if (r2.v.x < 4.0f || r2.v.y < 4.0f) {
-    // rare: overlapping or self pair in a lane -> scalar evaluation per lane
-    Vec3<float> u0 = {0, 0, 0}, w0 = {0, 0, 0}, u1 = {0, 0, 0}, w1 = {0, 0, 0};
-    wall_pair_fused(k, K, xi.v.x, yi.v.x, hi.v.x, Xj.v.x, Yj.v.x, Hj.v.x, Fx.v.x, Fy.v.x,
-                    Fz.v.x, Tx.v.x, Ty.v.x, Tz.v.x, u0, w0);
-    wall_pair_fused(k, K, xi.v.y, yi.v.y, hi.v.y, Xj.v.y, Yj.v.y, Hj.v.y, Fx.v.y, Fy.v.y,
-                    Fz.v.y, Tx.v.y, Ty.v.y, Tz.v.y, u1, w1);
-    u.x = u.x + mk2(u0.x, u1.x);
-    u.y = u.y + mk2(u0.y, u1.y);
-    u.z = u.z + mk2(u0.z, u1.z);
-    w.x = w.x + mk2(w0.x, w1.x);
-    w.y = w.y + mk2(w0.y, w1.y);
-    w.z = w.z + mk2(w0.z, w1.z);
-    return;
-  }
   const F2 Rz = hi + Hj;
   // far-field RPY coefficients (rpy_coefficients, r >= 2a)
   const F2 ir = rsq2(r2);
@@ -139,28 +145,35 @@ __device__ __forceinline__ void wall_pair_fused_x2(
   u.z = fms2(k1, fma2(dy, Tx, neg2(dx * Ty)), fma2(mp, ez, fma2(pv, f2i, u.z)));
 }
 
+// The same for any pair: a close one in either lane is evaluated where it is met.
+__device__ __forceinline__ void wall_pair_fused_x2(const PairConst<float> &k, const WallConst &K,
+                                                   float xi, float yi, float hi,
+                                                   const F2 (&v)[9], V3p &u, V3p &w) {
+  if (wall_close(bc(xi), bc(yi), bc(hi), v[0], v[1], v[2])) {
+    V3p cu, cw;
+    wall_close_x2(k, K, xi, yi, hi, v, cu, cw);
+    u.x = u.x + cu.x;
+    u.y = u.y + cu.y;
+    u.z = u.z + cu.z;
+    w.x = w.x + cw.x;
+    w.y = w.y + cw.y;
+    w.z = w.z + cw.z;
+    return;
+  }
+  wall_pair_far_x2(k, K, bc(xi), bc(yi), bc(hi), v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7],
+                   v[8], u, w);
+}
+
 // Packed wall UF pair (forces only): the translational part of
-// wall_pair_fused_x2 above (RPY UF merged with the translational image C2),
-// same formulas and order of operations.  Pairs closer than 2a in either lane
-// (the self pair included) are evaluated lane by lane with the scalar
-// wall_pair_fused with zero torques, keeping its u.
-__device__ __forceinline__ void wall_uf_pair_x2(const PairConst<float> &k, const WallConst &K,
-                                                F2 xi, F2 yi, F2 hi, F2 Xj, F2 Yj, F2 Hj,
-                                                F2 Fx, F2 Fy, F2 Fz, V3p &u) {
+// wall_pair_far_x2 above (RPY UF merged with the translational image C2), same
+// formulas and order of operations.  (Close pairs: wall_close_x2 with zero
+// torques, keeping its u.)
+__device__ __forceinline__ void wall_uf_far_x2(const PairConst<float> &k, const WallConst &K,
+                                               F2 xi, F2 yi, F2 hi, F2 Xj, F2 Yj, F2 Hj,
+                                               F2 Fx, F2 Fy, F2 Fz, V3p &u) {
   const F2 dx = xi - Xj, dy = yi - Yj, dz = hi - Hj;
   const F2 sxy = fma2(dx, dx, dy * dy);
   const F2 r2 = fma2(dz, dz, sxy);
-  if (r2.v.x < 4.0f || r2.v.y < 4.0f) {
-    Vec3<float> u0 = {0, 0, 0}, w0 = {0, 0, 0}, u1 = {0, 0, 0}, w1 = {0, 0, 0};
-    wall_pair_fused(k, K, xi.v.x, yi.v.x, hi.v.x, Xj.v.x, Yj.v.x, Hj.v.x, Fx.v.x, Fy.v.x,
-                    Fz.v.x, 0.f, 0.f, 0.f, u0, w0);
-    wall_pair_fused(k, K, xi.v.y, yi.v.y, hi.v.y, Xj.v.y, Yj.v.y, Hj.v.y, Fx.v.y, Fy.v.y,
-                    Fz.v.y, 0.f, 0.f, 0.f, u1, w1);
-    u.x = u.x + mk2(u0.x, u1.x);
-    u.y = u.y + mk2(u0.y, u1.y);
-    u.z = u.z + mk2(u0.z, u1.z);
-    return;
-  }
   const F2 Rz = hi + Hj;
   const F2 ir = rsq2(r2);
   const F2 ir2 = ir * ir;
@@ -190,6 +203,21 @@ __device__ __forceinline__ void wall_uf_pair_x2(const PairConst<float> &k, const
   u.x = fma2(fA, Fx, fma2(g, dx, fma2(s, ex, u.x)));
   u.y = fma2(fA, Fy, fma2(g, dy, fma2(s, ey, u.y)));
   u.z = fma2(fA, Fz, fma2(g, dz, fma2(s, ez, fma2(D, ev, fma2(E, Fz, u.z)))));
+}
+
+// The same for any pair (v[6..8], the torques, are 0).
+__device__ __forceinline__ void wall_uf_pair_x2(const PairConst<float> &k, const WallConst &K,
+                                                float xi, float yi, float hi, const F2 (&v)[9],
+                                                V3p &u) {
+  if (wall_close(bc(xi), bc(yi), bc(hi), v[0], v[1], v[2])) {
+    V3p cu, cw;
+    wall_close_x2(k, K, xi, yi, hi, v, cu, cw);
+    u.x = u.x + cu.x;
+    u.y = u.y + cu.y;
+    u.z = u.z + cu.z;
+    return;
+  }
+  wall_uf_far_x2(k, K, bc(xi), bc(yi), bc(hi), v[0], v[1], v[2], v[3], v[4], v[5], u);
 }
 
 // Packed open-space UF pair (translational RPY, forces only) in the fast

@@ -314,7 +314,9 @@ inline WallConst make_wall_const(double t0, double r0, double rt0) {
 }
 
 // Adds the UF+UT contribution to u and WT+WF to w for target (xi, yi, hi) and
-// source p = (xj, yj, hj, .), F, T (scaled units, FP32).
+// source p = (xj, yj, hj, .), F, T (scaled units, FP32).  CLOSE = false is for
+// pairs known to be at least 2a apart: the same operations without branches.
+template <bool CLOSE = true>
 __device__ __forceinline__ void wall_pair_fused(const PairConst<float> &k, const WallConst &K,
                                                 float xi, float yi, float hi, float xj, float yj,
                                                 float hj, float Fx, float Fy, float Fz, float Tx,
@@ -324,10 +326,10 @@ __device__ __forceinline__ void wall_pair_fused(const PairConst<float> &k, const
   const float sxy = fmaf(dx, dx, dy * dy);
   const float r2 = fmaf(dz, dz, sxy);
   const float Rz = hi + hj;
-  if (r2 > 0.0f) {
+  if (!CLOSE || r2 > 0.0f) {
     const float ir = rsqrtf(r2);
     float f, G, fw, Gw, c;
-    rpy_coefficients<float, true, true, true>(k, r2, ir, f, G, fw, Gw, c);
+    rpy_coefficients<float, true, true, true, CLOSE>(k, r2, ir, f, G, fw, Gw, c);
     const float iR = rsqrtf(fmaf(Rz, Rz, sxy));
     const float ex = dx * iR, ey = dy * iR, ez = Rz * iR;
     const float iRz = __fdividef(1.0f, Rz);
@@ -346,7 +348,7 @@ __device__ __forceinline__ void wall_pair_fused(const PairConst<float> &k, const
     const float E = fmaf(K.e1 * q, fmaf(hhj * hhj, iR, iR3), iR5 * fmaf(K.e51, q, K.e50));
     const float ev = fmaf(ex, Fx, fmaf(ey, Fy, ez * Fz));
     const float dF = fmaf(dx, Fx, fmaf(dy, Fy, dz * Fz));
-    const float fA = f + A;
+    const float fA = __fadd_rn(f, A);  // not contracted with f's last product
     const float g = G * dF;
     const float s = fmaf(B, ev, C * Fz);
     u.x = fmaf(fA, Fx, fmaf(g, dx, fmaf(s, ex, u.x)));
