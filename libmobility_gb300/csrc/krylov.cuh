@@ -1008,16 +1008,16 @@ __global__ void krylov_check_kernel(const R *V, size_t ldv, int m, const double 
     if (ok) {
       // eight loads in flight per thread ahead of their products, which are
       // summed in the same order as one at a time
+      // (the last, partial batch too: its loads are clamped, its terms dropped)
       const R *col = V + e;
-      int k = part;
-      for (; k + 7 * TPE < m; k += 8 * TPE) {
+      for (int k = part; k < m; k += 8 * TPE) {
         R x[8];
 #pragma unroll
-        for (int u = 0; u < 8; u++) x[u] = col[(size_t)(k + u * TPE) * ldv];
+        for (int u = 0; u < 8; u++) x[u] = col[(size_t)min(k + u * TPE, m - 1) * ldv];
 #pragma unroll
-        for (int u = 0; u < 8; u++) acc += cs[k + u * TPE] * x[u];
+        for (int u = 0; u < 8; u++)
+          if (k + u * TPE < m) acc += cs[k + u * TPE] * x[u];
       }
-      for (; k < m; k += TPE) acc += cs[k] * col[(size_t)k * ldv];
     }
 #pragma unroll
     for (int o = 1; o < TPE; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);

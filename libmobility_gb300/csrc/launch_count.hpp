@@ -21,7 +21,7 @@ extern std::atomic<size_t> g_pairs_max_part;
 // the device by quadrature; 2 (default) on the host by quadrature; the host
 // QL wherever a quadrature falls back
 extern std::atomic<int> g_lanczos_device_sqrt;
-// iterations issued ahead of a check (0 = by batch size: 3 up to 8192 particles, else 1)
+// iterations issued ahead of a check (0 = 2 where a product is short, else 1)
 extern std::atomic<int> g_lanczos_lookahead;
 // what the check kernel of iteration i waits for on the side stream: 0 the
 // end of iteration i; 1 the end of iteration i + 1's matrix-vector product

@@ -223,8 +223,8 @@ int lmg_internal_lanczos_device_sqrt(int on) {
 }
 
 // Iterations the single-system Lanczos issues ahead of the check it is
-// evaluating: 1..4, or 0 for the default (3 for batches of up to 8192
-// particles, else 1).
+// evaluating: 1..4, or 0 for the default (2 for FP32 forces in open space up to
+// 4096 particles a batch, else 1).
 int lmg_internal_lanczos_lookahead(int n) {
   if (n < 0 || n > 4) return 1;
   lmg::g_lanczos_lookahead.store(n);

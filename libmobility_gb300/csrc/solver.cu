@@ -734,9 +734,9 @@ cudaError_t launch_step_cluster(int ctas, int cta_threads, R *w, const R *vi, co
 //
 // Schedule per iteration i on the solver stream S: matvec, alpha, beta (which
 // also writes alpha_i, beta_i to mapped host memory), next -> event I_i.  The
-// GPU is kept ahead of the host: iterations up to i+3 (batches of up to 8192
-// particles, else i+1) are issued before the host handles the convergence
-// check of iteration i.  A check (every i >= k, the adaptive start of
+// GPU is kept ahead of the host: iterations up to i+2 (short products,
+// else i+1) are issued before the host handles the convergence check of
+// iteration i.  A check (every i >= k, the adaptive start of
 // LanczosAlgorithm.cu:179-184, or every i with a callback) waits for I_i,
 // takes the FP64 T^{1/2} e1 on the host while the GPU runs ahead, then on
 // the high-priority side stream P computes y_i = |z| V c_i and
@@ -820,15 +820,19 @@ int Solver<R>::lanczos(const R *z, R *y_out, size_t n, double tol, double *resid
   auto nper_lookahead = [&]() {
     const int forced = g_lanczos_lookahead.load();
     if (forced > 0) return std::min(forced, (int)kMaxLookahead);
-    // one matrix-vector product of a batch of up to 8192 particles takes
-    // tens of microseconds, less than a check
-    return batch_size() <= 8192 ? 3 : 1;
+    // one iteration ahead covers a check (about 30 us from the end of its
+    // iteration to its verdict), and every further one is work thrown away at
+    // the end (N = 2048 wall with torques, 50 us an iteration: 3.15 ms a step
+    // with one ahead, 3.22 with two, 3.27 with three).  FP32 forces in open
+    // space up to 4096 particles take 20 to 30 us an iteration: two ahead
+    // (N = 2000 1.05 ms, 1.06 with one or three)
+    return sizeof(R) == 4 && !wall_ && !ang_ && !prec_active() && batch_size() <= 4096 ? 2 : 1;
   };
   auto issue = [&](int j) {
     R *vj = V + (size_t)j * n;
     if (timing_) LMG_CUDA(cudaEventRecord(ev_phase_[5 * j], st));
     apply_operator(vj, w);
-    LMG_CUDA(cudaEventRecord(ev_prod_[j % kIterEvents], st));
+    if (g_lanczos_check_wait.load() == 1) LMG_CUDA(cudaEventRecord(ev_prod_[j % kIterEvents], st));
     if (timing_) LMG_CUDA(cudaEventRecord(ev_phase_[5 * j + 1], st));
     const R *vprev = j > 0 ? vj - n : vj;
     R *vnext = vj + n;
