@@ -458,6 +458,7 @@ krylov_step_cluster_kernel(R *w, const R *vi, const R *vprev, R *vnext, size_t n
                            KrylovScalars *sc, double *host_ab) {
   __shared__ ClusterRed<R> red;
   constexpr int E = EPT > 0 ? EPT : 1;
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the product is complete
   const unsigned nct = cluster_nctarank(), rank = cluster_ctarank();
   const size_t stride = (size_t)nct * blockDim.x;
   const size_t e0 = (size_t)rank * blockDim.x + threadIdx.x;

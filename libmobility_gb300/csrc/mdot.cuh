@@ -294,6 +294,7 @@ mdot_kernel(const MdotArgs<R> a) {
     for (int q = s_first; q <= s_lastb; q++) any |= __ldg(a.sys_active + q);
     if (!any) return;
   }
+  asm volatile("griddepcontrol.launch_dependents;");
   const int c_begin = src_lo + split * a.chunk;
   const int c_end = min(src_hi, c_begin + a.chunk);
 

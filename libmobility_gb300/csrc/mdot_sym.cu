@@ -457,6 +457,7 @@ __global__ void __launch_bounds__(kSymThreads, MINB) mdot_sym_kernel(const SymAr
   }
   if (a.trace && lane == 0) a.trace[2 * gw + 1] = global_ns();
 
+  asm volatile("griddepcontrol.launch_dependents;");
   // ---- every partial is written: fold them into U ----
   if (!grid_barrier_mono(a.bar)) {
     if (threadIdx.x == 0) *a.err = 1;

@@ -721,8 +721,11 @@ cudaError_t launch_step_cluster(int ctas, int cta_threads, R *w, const R *vi, co
   int ept = 0;
   for (int e : {1, 2, 4, 8})
     if (ept == 0 && e <= max_ept && per <= (size_t)e) ept = e;
-  cudaLaunchAttribute at[1];
-  const cudaLaunchConfig_t cfg = cluster_config(ctas, cta_threads, st, at);
+  cudaLaunchAttribute at[2];
+  cudaLaunchConfig_t cfg = cluster_config(ctas, cta_threads, st, at);
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   void *args[] = {&w, (void *)&vi, (void *)&vprev, &vnext, &n, &i, &sc, &host_ab};
   count_launch();
   return cudaLaunchKernelExC(&cfg, step_cluster_fn<R>(ept), args);
