@@ -531,6 +531,7 @@ krylov_step_cluster_kernel(R *w, const R *vi, const R *vprev, R *vnext, size_t n
       red.inv_beta = sizeof(R) == 4 ? (R)rsqrt(t.value()) : (R)(1.0 / sqrt(t.value()));
   }
   __syncthreads();
+  asm volatile("griddepcontrol.launch_dependents;");  // the next product
   const bool broke = !(red.beta > 0.0);
   if (rank == 0 && threadIdx.x == 0) {
     sc->alpha[i] = red.alpha;

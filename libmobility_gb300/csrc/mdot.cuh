@@ -251,6 +251,7 @@ mdot_kernel(const MdotArgs<R> a) {
   __shared__ float2 s_close[EVENTS ? THREADS / 32 : 1][EVENTS ? NC : 1][EVENTS ? kCloseCap : 1];
   __shared__ int s_last;
 
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // a step ahead of it is complete
   const int N = a.N;
   const int t_lo = a.tgt_begin, t_hi = a.tgt_end > 0 ? a.tgt_end : N;
   const int tile = blockIdx.x / SUB;

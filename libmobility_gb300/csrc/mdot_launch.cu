@@ -113,7 +113,7 @@ cudaError_t mdot_plan(const MdotShape &s, int N, int max_src_span, int num_sms, 
 
 template <class R>
 cudaError_t mdot_launch(const MdotShape &s, const MdotArgs<R> &args, const MdotPlan &plan,
-                        cudaStream_t stream) {
+                        cudaStream_t stream, bool early) {
   void *k = select_kernel<R>(s, plan.tpt, plan.dense);
   if (!k) return cudaErrorInvalidValue;
   MdotArgs<R> a = args;
@@ -124,7 +124,16 @@ cudaError_t mdot_launch(const MdotShape &s, const MdotArgs<R> &args, const MdotP
   dim3 grid(plan.tiles * plan.sub, plan.nsplit);
   void *params[] = {(void *)&a};
   count_launch();
-  return cudaLaunchKernel(k, grid, dim3(plan.threads / plan.sub), params, 0, stream);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(plan.threads / plan.sub);
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelExC(&cfg, k, params);
 }
 
 // this translation unit's bounds status (the checked build; 0 otherwise)
@@ -134,6 +143,6 @@ unsigned long long LMG_STATUS_NAME(LMG_REAL)(bool reset) { return bounds_status_
 
 template cudaError_t mdot_plan<LMG_REAL>(const MdotShape &, int, int, int, int, int, MdotPlan &);
 template cudaError_t mdot_launch<LMG_REAL>(const MdotShape &, const MdotArgs<LMG_REAL> &,
-                                           const MdotPlan &, cudaStream_t);
+                                           const MdotPlan &, cudaStream_t, bool);
 
 }  // namespace lmg
