@@ -18,6 +18,7 @@
 #pragma once
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 #include "grid_sync.cuh"
@@ -1002,6 +1003,13 @@ __global__ void krylov_check_kernel(const R *V, size_t ldv, int m, const double 
   const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const int part = (int)(tid % TPE);
   const size_t per_pass = (size_t)gridDim.x * blockDim.x / TPE;
+  // The sums are taken over y / 2^k, 2^k about |z| c_0 <= |y|: the scale is
+  // exact, and FP32 squares neither overflow nor vanish for any size of z.
+  R scale = R(1);
+  if constexpr (std::is_same<R, float>::value) {
+    const double top = fabs(nz * c[0]);
+    if (top > 0.0 && top < 3e38) scale = ldexpf(1.0f, -max(-126, min(126, ilogb(top))));
+  }
   DotAcc<R> v[2];  // |yprev|^2, |y - yprev|^2
   for (size_t e0 = 0; e0 < n; e0 += per_pass) {
     const size_t e = e0 + tid / TPE;
@@ -1026,9 +1034,9 @@ __global__ void krylov_check_kernel(const R *V, size_t ldv, int m, const double 
     if (ok && part == 0) {
       y[e] = acc;
       if (yprev) {
-        const R a = yprev[e];
+        const R a = scale * yprev[e];
         v[0].add_prod(a, a);
-        v[1].add_diff2(acc, a);
+        v[1].add_diff2(scale * acc, a);
       }
     }
   }
@@ -1042,70 +1050,137 @@ __global__ void krylov_check_kernel(const R *V, size_t ldv, int m, const double 
 }
 
 // ---------------------------------------------------------------------------
-// BiCGSTAB pieces for solving P x = b with the sparse preconditioner (the
-// last step of the preconditioned square root).  Each reduction writes its
-// FP64 results to mapped host memory (out[0], out[1]).
+// BiCGSTAB (van der Vorst 1992) for P x = b with the sparse preconditioner,
+// the last step of the preconditioned square root.  The scalars live on the
+// device: the last block of a reduction works out what the next kernel needs,
+// so an iteration is seven launches that nothing waits between; the host looks
+// at `done` an iteration late.  Once done (or broken down) the kernels of a
+// further iteration return at once.
 // ---------------------------------------------------------------------------
+struct BicgScalars {
+  double tol2, rho, alpha, omega;  // |r|^2 to reach; the recurrence (FP64 throughout)
+  float alpha_f, omega_f, beta_f;  // as the vectors use them
+  int last;                        // |s|^2 is small enough: this half step ends it
+  int done;                        // 0 going on, 1 converged, 2 broken down
+  int iterations;
+};
+
+// x = p = v = 0, r = rhat = b; the first scalars
 template <class R>
-__global__ void dot2_kernel(const R *a, const R *b, const R *c, const R *d, size_t n,
-                            double *partials, unsigned *ticket, double *out) {
-  double v[2] = {0.0, 0.0};
+__global__ void bicg_init_kernel(const R *b, R *x, R *p, R *v, R *r, R *rhat, size_t n,
+                                 double *partials, unsigned *ticket, BicgScalars *sc,
+                                 BicgScalars *host) {
+  double d[1] = {0.0};
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n;
        e += (size_t)gridDim.x * blockDim.x) {
-    v[0] += (double)a[e] * (double)b[e];
-    v[1] += (double)c[e] * (double)d[e];
+    const R y = b[e];
+    x[e] = p[e] = v[e] = R(0);
+    r[e] = rhat[e] = y;
+    d[0] += (double)y * (double)y;
   }
-  double tot[2];
-  if (grid_sum<2>(v, partials, ticket, tot)) {
-    out[0] = tot[0];
-    out[1] = tot[1];
+  double tot[1];
+  if (grid_sum<1>(d, partials, ticket, tot)) {
+    BicgScalars z{};
+    z.tol2 = 1e-14 * tot[0];
+    z.rho = tot[0];
+    z.alpha = z.omega = 1.0;
+    z.done = tot[0] > 0.0 ? 0 : 1;  // b = 0: x = 0
+    *sc = z;
+    host->iterations = 0;
+    host->done = z.done;
   }
 }
 
 // p = r + beta (p - omega v)
 template <class R>
-__global__ void bicg_p_kernel(R *p, const R *r, const R *v, double beta, double omega, size_t n) {
-  const R b = (R)beta, o = (R)omega;
+__global__ void bicg_p_kernel(R *p, const R *r, const R *v, size_t n, const BicgScalars *sc) {
+  if (sc->done) return;
+  const R b = sc->beta_f, o = sc->omega_f;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n;
        e += (size_t)gridDim.x * blockDim.x)
     p[e] = r[e] + b * (p[e] - o * v[e]);
 }
 
-// s = r - alpha v ; out[0] = |s|^2
+// alpha = rho / (rhat . v)
 template <class R>
-__global__ void bicg_s_kernel(R *s, const R *r, const R *v, double alpha, size_t n,
-                              double *partials, unsigned *ticket, double *out) {
-  const R a = (R)alpha;
-  double acc[1] = {0.0};
+__global__ void bicg_alpha_kernel(const R *rhat, const R *v, size_t n, double *partials,
+                                  unsigned *ticket, BicgScalars *sc) {
+  if (sc->done) return;
+  double d[1] = {0.0};
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n;
+       e += (size_t)gridDim.x * blockDim.x)
+    d[0] += (double)rhat[e] * (double)v[e];
+  double tot[1];
+  if (grid_sum<1>(d, partials, ticket, tot)) {
+    if (tot[0] == 0.0 || isnan(tot[0])) sc->done = 2;
+    sc->alpha = sc->rho / tot[0];
+    sc->alpha_f = (float)sc->alpha;
+  }
+}
+
+// s = r - alpha v
+template <class R>
+__global__ void bicg_s_kernel(R *s, const R *r, const R *v, size_t n, double *partials,
+                              unsigned *ticket, BicgScalars *sc) {
+  if (sc->done) return;
+  const R a = sc->alpha_f;
+  double d[1] = {0.0};
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n;
        e += (size_t)gridDim.x * blockDim.x) {
     const R x = r[e] - a * v[e];
     s[e] = x;
-    acc[0] += (double)x * (double)x;
+    d[0] += (double)x * (double)x;
   }
   double tot[1];
-  if (grid_sum<1>(acc, partials, ticket, tot)) out[0] = tot[0];
+  if (grid_sum<1>(d, partials, ticket, tot)) sc->last = tot[0] <= sc->tol2;
 }
 
-// x += alpha p + omega s ; r = s - omega t ; out = (|r|^2, rhat . r)
+// omega = (t . s) / (t . t), or 0 in the last half step
+template <class R>
+__global__ void bicg_omega_kernel(const R *t, const R *s, size_t n, double *partials,
+                                  unsigned *ticket, BicgScalars *sc) {
+  if (sc->done) return;
+  double d[2] = {0.0, 0.0};
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n;
+       e += (size_t)gridDim.x * blockDim.x) {
+    d[0] += (double)t[e] * (double)s[e];
+    d[1] += (double)t[e] * (double)t[e];
+  }
+  double tot[2];
+  if (grid_sum<2>(d, partials, ticket, tot)) {
+    sc->omega = sc->last ? 0.0 : tot[0] / tot[1];
+    sc->omega_f = (float)sc->omega;
+  }
+}
+
+// x += alpha p + omega s ; r = s - omega t ; the next beta, and whether it ends
 template <class R>
 __global__ void bicg_xr_kernel(R *x, const R *p, const R *s, const R *t, R *r, const R *rhat,
-                               double alpha, double omega, size_t n, double *partials,
-                               unsigned *ticket, double *out) {
-  const R a = (R)alpha, o = (R)omega;
-  double acc[2] = {0.0, 0.0};
+                               size_t n, double *partials, unsigned *ticket, BicgScalars *sc,
+                               BicgScalars *host) {
+  if (sc->done) return;
+  const R a = sc->alpha_f, o = sc->omega_f;
+  double d[2] = {0.0, 0.0};
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n;
        e += (size_t)gridDim.x * blockDim.x) {
     x[e] += a * p[e] + o * s[e];
     const R re = s[e] - o * t[e];
     r[e] = re;
-    acc[0] += (double)re * (double)re;
-    acc[1] += (double)rhat[e] * (double)re;
+    d[0] += (double)re * (double)re;
+    d[1] += (double)rhat[e] * (double)re;
   }
   double tot[2];
-  if (grid_sum<2>(acc, partials, ticket, tot)) {
-    out[0] = tot[0];
-    out[1] = tot[1];
+  if (grid_sum<2>(d, partials, ticket, tot)) {
+    sc->iterations += 1;
+    sc->beta_f = (float)((tot[1] / sc->rho) * (sc->alpha / sc->omega));
+    sc->rho = tot[1];
+    if (sc->last || tot[0] <= sc->tol2)
+      sc->done = 1;
+    else if (isnan(tot[0]))
+      sc->done = 2;
+    host->iterations = sc->iterations;
+    __threadfence_system();
+    host->done = sc->done;
   }
 }
 

@@ -97,6 +97,8 @@ template <class R> class Solver final : public SolverBase {
     for (auto &e : ev_check_)
       if (e) cudaEventDestroy(e);
     if (ev_side_) cudaEventDestroy(ev_side_);
+    for (auto &e : ev_bicg_)
+      if (e) cudaEventDestroy(e);
     for (auto &e : ev_phase_)
       if (e) cudaEventDestroy(e);
     for (auto &e : ev_pre_)
@@ -167,7 +169,10 @@ template <class R> class Solver final : public SolverBase {
   DeviceBuffer<int> prec_nb_;
   KnnScratch knn_scratch_;
   DeviceBuffer<R> pt_, pu_, bx_, br_, brh_, bp_, bv_, bs_, bt_;  // operator and BiCGSTAB vectors
-  DeviceBuffer<float> ppad_;  // float4-padded work array of the P^T product
+  PrecRows prec_rows_;                // P and P^T as the products read them
+  DeviceBuffer<BicgScalars> bsc_;
+  MappedBuffer<BicgScalars> bsc_host_;
+  cudaEvent_t ev_bicg_[2] = {nullptr, nullptr};
   int num_sms_ = 0;
   int step_per_sm_ = 0;  // resident krylov_step_kernel blocks per SM
   int step_ctas_ = -1;   // CTAs of the cluster of krylov_step_cluster_kernel (0: none fits)
@@ -1261,6 +1266,7 @@ template <class R> void Solver<R>::prec_build() {
     // products apply t0^{-1/2} (prec_scale)
     LMG_CUDA(precond_build_launch(prec_layout_, pos_.ptr, nb, N, prec_params_.ptr, (float)(1.0 / a_),
                                   1.0f, blocks, true, &prec_work_, stream()));
+    LMG_CUDA(precond_pack_launch(prec_k_, blocks, nb, N, &prec_rows_, stream()));
     prec_dirty_ = false;
   }
 }
@@ -1277,15 +1283,15 @@ template <class R> void Solver<R>::apply_operator(const R *v, R *out) {
     R *t = pt_.ensure(n);
     R *u = pu_.ensure(n);
     const R s = (R)(1.0 / std::sqrt(r0_));  // angular part: scalar r0^{-1/2}
-    float4 *pad = reinterpret_cast<float4 *>(ppad_.ensure(4 * (size_t)N));
-    LMG_CUDA(precond_apply_t_launch(prec_k_, prec_blocks_.ptr, true, prec_scale(), prec_nb_.ptr, N,
-                                    v, t, pad, stream()));
+    LMG_CUDA(precond_rows_launch(prec_k_, prec_rows_, true, prec_scale(), N, v, t, nullptr,
+                                 stream(), true));
     if (ang_) {
       scale_kernel<R><<<vec_blocks(n3), kRedThreads, 0, stream()>>>(t + n3, v + n3, n3, s);
       count_launch();
     }
     mdot_device(pos_.ptr, t, ang_ ? t + n3 : nullptr, u, ang_ ? u + n3 : nullptr, true);
-    LMG_CUDA(precond_apply_launch(prec_k_, prec_blocks_.ptr, true, prec_scale(), prec_nb_.ptr, N, u, out, stream()));
+    LMG_CUDA(precond_rows_launch(prec_k_, prec_rows_, false, prec_scale(), N, u, out, nullptr,
+                                 stream(), true));
     if (ang_) {
       scale_kernel<R><<<vec_blocks(n3), kRedThreads, 0, stream()>>>(out + n3, u + n3, n3, s);
       count_launch();
@@ -1293,10 +1299,8 @@ template <class R> void Solver<R>::apply_operator(const R *v, R *out) {
   }
 }
 
-// BiCGSTAB (van der Vorst 1992) for P x = b on the translational part,
-// relative residual 1e-7 (the Lanczos tolerance is at least 1e-6 on single
-// precision vectors).  Scalars in FP64 on the host; each reduction is read
-// back through mapped memory.
+// P x = b on the translational part (BiCGSTAB, krylov.cuh), relative residual
+// 1e-7 (the Lanczos tolerance is at least 1e-6 on single precision vectors).
 template <class R> int Solver<R>::solve_p(const R *b, R *x) {
   NvtxRange nvtx_range_("lmg preconditioner solve");
   if constexpr (!std::is_same<R, float>::value) {
@@ -1310,61 +1314,41 @@ template <class R> int Solver<R>::solve_p(const R *b, R *x) {
     ensure_reduction(blocks);
     unsigned *tk = red_ticket_.ptr;
     double *rp = red_part_.ptr;
-    double *mir = mirror_.ensure(2 * 256 + 8);
-    double *out = mirror_.device_ptr() + 514;
-    double *hout = mir + 514;
     R *r = br_.ensure(n), *rh = brh_.ensure(n), *p = bp_.ensure(n), *v = bv_.ensure(n);
     R *s = bs_.ensure(n), *t = bt_.ensure(n);
-    auto sync = [&]() { LMG_CUDA(cudaStreamSynchronize(st)); };
-    LMG_CUDA(cudaMemsetAsync(x, 0, n * sizeof(R), st));
-    LMG_CUDA(cudaMemsetAsync(p, 0, n * sizeof(R), st));
-    LMG_CUDA(cudaMemsetAsync(v, 0, n * sizeof(R), st));
-    LMG_CUDA(cudaMemcpyAsync(r, b, n * sizeof(R), cudaMemcpyDeviceToDevice, st));
-    LMG_CUDA(cudaMemcpyAsync(rh, b, n * sizeof(R), cudaMemcpyDeviceToDevice, st));
-    dot2_kernel<R><<<blocks, kRedThreads, 0, st>>>(b, b, b, b, n, rp, tk, out);
+    BicgScalars *sc = bsc_.ensure(1);
+    volatile BicgScalars *host = bsc_host_.ensure(1);
+    BicgScalars *host_dev = bsc_host_.device_ptr();
+    for (auto &e : ev_bicg_)
+      if (!e) LMG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    host->done = host->iterations = 0;
+    bicg_init_kernel<R><<<blocks, kRedThreads, 0, st>>>(b, x, p, v, r, rh, n, rp, tk, sc,
+                                                        host_dev);
     count_launch();
-    sync();
-    const double bnorm2 = hout[0];
-    if (!(bnorm2 > 0)) return 0;
-    const double tol2 = 1e-14 * bnorm2;
-    double rho = 1, alpha = 1, omega = 1, rho1 = bnorm2;
+    auto product = [&](const R *in, R *out) {
+      LMG_CUDA(precond_rows_launch(prec_k_, prec_rows_, false, prec_scale(), N, in, out,
+                                   &sc->done, st));
+    };
     const int max_it = 500;
-    for (int it = 1; it <= max_it; it++) {
-      const double beta = (rho1 / rho) * (alpha / omega);
-      bicg_p_kernel<R><<<blocks, kRedThreads, 0, st>>>(p, r, v, it == 1 ? 0.0 : beta,
-                                                       omega, n);
-      count_launch();
-      LMG_CUDA(precond_apply_launch(prec_k_, prec_blocks_.ptr, true, prec_scale(), prec_nb_.ptr, N, p, v, st));
-      dot2_kernel<R><<<blocks, kRedThreads, 0, st>>>(rh, v, rh, v, n, rp, tk, out);
-      count_launch();
-      sync();
-      const double rv = hout[0];
-      if (rv == 0 || std::isnan(rv))
-        throw Error(LMG_ERR_NAN, "[libmobility_gb300] preconditioner solve broke down");
-      alpha = rho1 / rv;
-      bicg_s_kernel<R><<<blocks, kRedThreads, 0, st>>>(s, r, v, alpha, n, rp, tk, out);
-      count_launch();
-      sync();
-      if (hout[0] <= tol2) {  // x += alpha p
-        bicg_xr_kernel<R><<<blocks, kRedThreads, 0, st>>>(x, p, s, s, r, rh, alpha, 0.0, n,
-                                                          rp, tk, out);
-        count_launch();
-        sync();
-        return it;
+    for (int it = 1; it <= max_it + 1; it++) {
+      if (it <= max_it) {
+        bicg_p_kernel<R><<<blocks, kRedThreads, 0, st>>>(p, r, v, n, sc);
+        product(p, v);
+        bicg_alpha_kernel<R><<<blocks, kRedThreads, 0, st>>>(rh, v, n, rp, tk, sc);
+        bicg_s_kernel<R><<<blocks, kRedThreads, 0, st>>>(s, r, v, n, rp, tk, sc);
+        product(s, t);
+        bicg_omega_kernel<R><<<blocks, kRedThreads, 0, st>>>(t, s, n, rp, tk, sc);
+        bicg_xr_kernel<R><<<blocks, kRedThreads, 0, st>>>(x, p, s, t, r, rh, n, rp, tk, sc,
+                                                          host_dev);
+        for (int k = 0; k < 5; k++) count_launch();
+        LMG_CUDA(cudaGetLastError());
+        LMG_CUDA(cudaEventRecord(ev_bicg_[it & 1], st));
       }
-      LMG_CUDA(precond_apply_launch(prec_k_, prec_blocks_.ptr, true, prec_scale(), prec_nb_.ptr, N, s, t, st));
-      dot2_kernel<R><<<blocks, kRedThreads, 0, st>>>(t, s, t, t, n, rp, tk, out);
-      count_launch();
-      sync();
-      omega = hout[0] / hout[1];
-      bicg_xr_kernel<R><<<blocks, kRedThreads, 0, st>>>(x, p, s, t, r, rh, alpha, omega, n, rp,
-                                                        tk, out);
-      count_launch();
-      sync();
-      rho = rho1;
-      rho1 = hout[1];
-      if (hout[0] <= tol2) return it;
-      if (std::isnan(hout[0]))
+      if (it == 1) continue;
+      // the verdict of the iteration before
+      LMG_CUDA(cudaEventSynchronize(ev_bicg_[(it - 1) & 1]));
+      if (host->done == 1) return host->iterations;
+      if (host->done == 2 || host->iterations < it - 1)
         throw Error(LMG_ERR_NAN, "[libmobility_gb300] preconditioner solve broke down");
     }
     throw Error(LMG_ERR_NO_CONVERGENCE,
