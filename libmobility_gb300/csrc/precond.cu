@@ -675,24 +675,28 @@ precond_pack_kernel(const uint16_t *__restrict__ B, const int *__restrict__ nb, 
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       const uint16_t v = B[((size_t)n * 9 + 3 * r + c) * N + i];
-      e.b[3 * r + c] = v;
-      f.b[3 * c + r] = v;
+      e.col[c][r] = v;
+      f.col[r][c] = v;
     }
   }
-  e.pad = f.pad = 0;
-  e.col = j;
-  f.col = i;
+  e.col[0][3] = (uint16_t)j;
+  e.col[1][3] = (uint16_t)((unsigned)j >> 16);
+  f.col[0][3] = (uint16_t)i;
+  f.col[1][3] = (uint16_t)((unsigned)i >> 16);
+  e.col[2][3] = f.col[2][3] = 0;
   rows[(size_t)i * KB + n] = e;
   cols[start[j] + atomicAdd(fill + j, 1)] = f;
 }
 
-// Latency-bound (two dependent loads, N x (K+1) x 24 bytes from L2): both
-// entries of a lane are loaded before either is used.  N = 16384, K = 48:
-// 223 -> 199 us for P M P^T x with a 183 us product in it.
-constexpr int kRowWarps = 8;
+// Bound by the cache lines touched in gathering x.  Three lanes take an entry,
+// one a column and a component of x: the components of a particle are then read
+// by one load (a lane an entry takes three, each touching every particle's line
+// again), and ten entries of a row are adjacent words.  The loads of five such
+// groups, a whole row for K = 48, are issued before any is used.
+constexpr int kRowWarps = 8, kRowGroups = 5;
 __global__ void __launch_bounds__(32 * kRowWarps)
-precond_rows_kernel(const PrecEntry *__restrict__ E, const int64_t *__restrict__ start, int KB, int N,
-                    const float *x, float *out, float scale, const int *skip) {
+precond_rows_kernel(const PrecEntry *__restrict__ E, const int64_t *__restrict__ start, int KB,
+                    int N, const float *x, float *out, float scale, const int *skip) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
   if (skip && *skip) return;
@@ -703,42 +707,34 @@ precond_rows_kernel(const PrecEntry *__restrict__ E, const int64_t *__restrict__
     b0 = start[row];
     b1 = start[row + 1];
   }
-  E += b0;
+  const uint2 *q0 = reinterpret_cast<const uint2 *>(E + b0);
   const int len = (int)(b1 - b0);
+  const int sub = lane / 3, c = lane - 3 * sub;  // lanes 30 and 31 take no entry
   float o[3] = {0.f, 0.f, 0.f};
-  for (int b = lane; b < len; b += 64) {
-    uint2 q[2][3];
-    float v[2][3];
+  for (int b = 0; b < len; b += 10 * kRowGroups) {
+    uint2 q[kRowGroups];
+    float v[kRowGroups];
 #pragma unroll
-    for (int u = 0; u < 2; u++) {
-      const bool in = b + 32 * u < len;
-      const uint2 *p = reinterpret_cast<const uint2 *>(E + (in ? b + 32 * u : b));
-#pragma unroll
-      for (int c = 0; c < 3; c++) q[u][c] = __ldg(p + c);
-      if (!in) {  // a zero block
-        q[u][0] = q[u][1] = make_uint2(0u, 0u);
-        q[u][2].x = 0u;
-      }
+    for (int u = 0; u < kRowGroups; u++) {
+      const int k = b + 10 * u + sub;
+      q[u] = make_uint2(0u, 0u);
+      if (sub < 10 && k < len) q[u] = __ldg(q0 + 3 * (size_t)k + c);
     }
 #pragma unroll
-    for (int u = 0; u < 2; u++) {
-      const size_t j = 3 * (size_t)(int)q[u][2].y;
-#pragma unroll
-      for (int c = 0; c < 3; c++) v[u][c] = x[j + c];
+    for (int u = 0; u < kRowGroups; u++) {
+      const unsigned part = q[u].y >> 16;
+      const unsigned j = __shfl_sync(0xffffffffu, part, 3 * sub) |
+                         (__shfl_sync(0xffffffffu, part, 3 * sub + 1) << 16);
+      v[u] = 0.f;
+      if (sub < 10 && b + 10 * u + sub < len) v[u] = x[3 * (size_t)j + c];
     }
 #pragma unroll
-    for (int u = 0; u < 2; u++) {
-      const unsigned w[5] = {q[u][0].x, q[u][0].y, q[u][1].x, q[u][1].y, q[u][2].x};
-      float h[10];
-#pragma unroll
-      for (int k = 0; k < 5; k++) {
-        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[k]));
-        h[2 * k] = f.x;
-        h[2 * k + 1] = f.y;
-      }
-#pragma unroll
-      for (int r = 0; r < 3; r++)
-        o[r] = fmaf(h[3 * r], v[u][0], fmaf(h[3 * r + 1], v[u][1], fmaf(h[3 * r + 2], v[u][2], o[r])));
+    for (int u = 0; u < kRowGroups; u++) {
+      const float2 h = __half22float2(*reinterpret_cast<const __half2 *>(&q[u].x));
+      const float2 g = __half22float2(*reinterpret_cast<const __half2 *>(&q[u].y));
+      o[0] = fmaf(h.x, v[u], o[0]);
+      o[1] = fmaf(h.y, v[u], o[1]);
+      o[2] = fmaf(g.x, v[u], o[2]);
     }
   }
 #pragma unroll

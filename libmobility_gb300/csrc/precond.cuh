@@ -114,15 +114,16 @@ cudaError_t precond_build_launch(const PrecLayout &L, const float *pos, const in
 // the products get 1).
 //
 // The solver's products: P and P^T, both as rows of packed half blocks.  An
-// entry holds its block and the particle it multiplies; row i of P is its K+1
-// entries, row j of P^T the entries (transposed) of the rows that have j as a
-// neighbour, found by counting and a scan.  A warp takes a row, so its entries
-// are read side by side and nothing is scattered (adding each row's products
-// with vector atomics took 22 us at N = 16384 and gave sums in no fixed order
-// from one product to the next).
+// entry holds its block by columns and the particle it multiplies; row i of P
+// is its K+1 entries, row j of P^T the entries (transposed) of the rows that
+// have j as a neighbour, found by counting and a scan.  A warp takes a row, so
+// its entries are read side by side and nothing is scattered (adding each row's
+// products with vector atomics took 22 us at N = 16384 and gave sums in no
+// fixed order from one product to the next).
 struct alignas(8) PrecEntry {
-  uint16_t b[9], pad;  // element 3 r + c, half precision
-  int col;
+  // column c: elements (0, c), (1, c), (2, c) in half precision, then a part of
+  // the particle's index (c = 0: low 16 bits, 1: high 16 bits)
+  uint16_t col[3][4];
 };
 struct PrecRows {
   DeviceBuffer<PrecEntry> rows, cols;  // P: K+1 entries a row; P^T: start[j] .. start[j+1]
