@@ -128,79 +128,191 @@ __global__ void knn_scatter_kernel(const float *__restrict__ pos, int N, const i
   spos[slot] = make_float4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], 0.f);
 }
 
-// Particles are taken in cell order (thread t -> sidx[t]), so the lanes of a
-// warp search the same cells: their loops stay in step and share cached reads.
-// Each thread's sorted list of the KB nearest lives in shared memory
-// (entry q of thread t at [q][t]: the lanes of a warp use distinct banks);
-// a candidate is placed by binary search and only the tail moves.
-constexpr int kSearchThreads = 64;
+// A warp takes a particle (in cell order, so that neighbouring warps share
+// cached reads).  Its lanes take the runs of cells of a shell (cells that
+// follow one another in z are one run of particles), then the candidates of
+// the runs, 32 at a time; those nearer than the K-th so far are appended to a
+// list in shared memory, which is cut back to the KB nearest by bisecting on
+// the distance (its bits order as whole numbers) when it is full and after a
+// shell.  The last list is put in order by counting.  One thread a particle
+// (a sorted list each, one candidate after the other) left the chip with a
+// few long chains: the whole build took 1.17 ms at N = 16384 and 0.71 at
+// N = 4000 (K = 48), 0.81 and 0.32 with a warp.
+constexpr int kSearchWarps = 8, kSearchCap = 256;
+
+// Cuts the warp's list (keys in any order, count >= KB) to KB entries with the
+// smallest keys; lo: fewer than KB keys are <= lo.  Returns a key below which
+// later candidates have to lie to matter.
+template <int KB>
+__device__ __forceinline__ unsigned knn_cut(unsigned *key, int *slot, int &count, unsigned lo) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  unsigned top = 0u;
+  for (int k = lane; k < count; k += 32) top = max(top, key[k]);
+  unsigned hi = __reduce_max_sync(0xffffffffu, top);
+  while (hi - lo > 1u) {  // count(<= lo) < KB <= count(<= hi)
+    const unsigned mid = lo + (hi - lo) / 2;
+    int c = 0;
+    for (int k = lane; k < count; k += 32) c += key[k] <= mid;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (c < KB) {
+      lo = mid;
+    } else {
+      hi = mid;
+      if (c == KB) break;
+    }
+  }
+  // all below hi, and of those equal to it as many as there is room for
+  int below = 0;
+  for (int k = lane; k < count; k += 32) below += key[k] < hi;
+  int room = KB - __reduce_add_sync(0xffffffffu, below);
+  int out = 0;
+  for (int k0 = 0; k0 < count; k0 += 32) {
+    const int k = k0 + lane;
+    const unsigned v = k < count ? key[k] : 0xffffffffu;
+    const int s = k < count ? slot[k] : 0;
+    const unsigned lower = (1u << lane) - 1u;
+    const unsigned eq = __ballot_sync(0xffffffffu, v == hi && k < count);
+    const bool keep = k < count && (v < hi || (v == hi && __popc(eq & lower) < room));
+    const unsigned kept = __ballot_sync(0xffffffffu, keep);
+    __syncwarp();  // all have read before any writes
+    if (keep) {
+      const int o = out + __popc(kept & lower);
+      key[o] = v;
+      slot[o] = s;
+    }
+    out += __popc(kept);
+    room -= min(room, __popc(eq));
+    __syncwarp();
+  }
+  count = out;
+  return hi;
+}
 
 template <int KB>
-__global__ void __launch_bounds__(kSearchThreads)
+__global__ void __launch_bounds__(32 * kSearchWarps)
 knn_search_kernel(int N, KnnGridShape g, const int *__restrict__ start,
                   const int *__restrict__ sidx, const float4 *__restrict__ spos,
                   int *__restrict__ nb) {
-  __shared__ float ld[KB][kSearchThreads];
-  __shared__ int lj[KB][kSearchThreads];
-  const int tl = threadIdx.x;
-  const int t0 = blockIdx.x * kSearchThreads + tl;
+  static_assert(KB + 32 <= kSearchCap, "room for a batch after a cut");
+  __shared__ unsigned keys[kSearchWarps][kSearchCap];
+  __shared__ int slots[kSearchWarps][kSearchCap];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t0 = blockIdx.x * kSearchWarps + wid;
   if (t0 >= N) return;
+  unsigned *key = keys[wid];
+  int *slot = slots[wid];
   const int i = sidx[t0];
   const float4 pi = spos[t0];
-  const float xi = pi.x, yi = pi.y, zi = pi.z;
-  const int ix = cell_coord(xi, g.x0, g.inv_h, g.nx);
-  const int iy = cell_coord(yi, g.y0, g.inv_h, g.ny);
-  const int iz = cell_coord(zi, g.z0, g.inv_h, g.nz);
+  const int ix = cell_coord(pi.x, g.x0, g.inv_h, g.nx);
+  const int iy = cell_coord(pi.y, g.y0, g.inv_h, g.ny);
+  const int iz = cell_coord(pi.z, g.z0, g.inv_h, g.nz);
   const int base = (i / g.nper) * g.cells;
-  int len = 0;
-  float worst = FLT_MAX;  // ld[KB-1] once the list is full
-  auto scan_cell = [&](int cx, int cy, int cz) {
-    const int k = base + (cx * g.ny + cy) * g.nz + cz;
-    const int e = start[k + 1];
-    for (int t = start[k]; t < e; t++) {
-      const float4 p = spos[t];
-      const float dx = p.x - xi, dy = p.y - yi, dz = p.z - zi;
-      float cd = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-      if (cd < worst) {
-        const int j = sidx[t];
-        if (j == i) cd = -1.0f;  // the particle itself goes first
-        int lo = 0, hi = len;    // first entry greater than cd
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (ld[mid][tl] > cd) hi = mid; else lo = mid + 1;
-        }
-        const int last = len < KB ? len : KB - 1;
-        for (int q = last; q > lo; q--) {
-          ld[q][tl] = ld[q - 1][tl];
-          lj[q][tl] = lj[q - 1][tl];
-        }
-        ld[lo][tl] = cd;
-        lj[lo][tl] = j;
-        if (len < KB) len++;
-        if (len == KB) worst = ld[KB - 1][tl];
-      }
-    }
-  };
+  int count = 0;
+  // a distance's bits + 1; the particle itself goes first, with 0
+  unsigned worst = __float_as_uint(FLT_MAX) + 1u;
   const int smax = max(g.nx, max(g.ny, g.nz));
-  for (int s = 0; s <= smax; s++) {
-    // the cells at Chebyshev distance exactly s
-    for (int dx = -s; dx <= s; dx++) {
-      const int cx = ix + dx;
-      if (cx < 0 || cx >= g.nx) continue;
-      for (int dy = -s; dy <= s; dy++) {
-        const int cy = iy + dy;
-        if (cy < 0 || cy >= g.ny) continue;
-        const bool face = (dx == -s || dx == s || dy == -s || dy == s);
-        for (int dz = -s; dz <= s; dz += face ? 1 : (s > 0 ? 2 * s : 1)) {
-          const int cz = iz + dz;
-          if (cz >= 0 && cz < g.nz) scan_cell(cx, cy, cz);
+  for (int s = 1; s <= smax; s++) {
+    // runs of cells: the columns on the shell's four sides (s = 1: all nine,
+    // shell 0 with them), then of the columns between them the cells at the
+    // lower and the upper end, as far as the grid reaches
+    const int w = 2 * s + 1, sides = s == 1 ? 9 : 8 * s;
+    const int x0 = max(ix - s + 1, 0), wx = min(ix + s - 1, g.nx - 1) - x0 + 1;
+    const int y0 = max(iy - s + 1, 0), wy = min(iy + s - 1, g.ny - 1) - y0 + 1;
+    const int low = s > 1 && iz - s >= 0 ? wx * wy : 0;
+    const int high = s > 1 && iz + s < g.nz ? wx * wy : 0;
+    const int runs = sides + low + high;
+    for (int r0 = 0; r0 < runs; r0 += 32) {
+      const int r = r0 + lane;
+      int b = 0, len = 0;
+      if (r < runs) {
+        int cx, cy, z0, z1;
+        if (r < sides) {
+          if (s == 1) {
+            cx = ix - 1 + r / 3;
+            cy = iy - 1 + r % 3;
+          } else if (r < 2 * w) {
+            cx = r < w ? ix - s : ix + s;
+            cy = iy - s + (r < w ? r : r - w);
+          } else {
+            const int m = r - 2 * w, in = w - 2;
+            cx = ix - s + 1 + (m < in ? m : m - in);
+            cy = m < in ? iy - s : iy + s;
+          }
+          z0 = max(iz - s, 0);
+          z1 = min(iz + s, g.nz - 1);
+        } else {
+          const int m = r - sides, c = m < low ? m : m - low;
+          cx = x0 + c / wy;
+          cy = y0 + c % wy;
+          z0 = z1 = m < low ? iz - s : iz + s;
+        }
+        if (cx >= 0 && cx < g.nx && cy >= 0 && cy < g.ny) {
+          const int k = base + (cx * g.ny + cy) * g.nz;
+          b = start[k + z0];
+          len = start[k + z1 + 1] - b;
         }
       }
+      int incl = len;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const int total = __shfl_sync(0xffffffffu, incl, 31);
+      const int off = b - (incl - len);
+      for (int c0 = 0; c0 < total; c0 += 32) {
+        const int t = c0 + lane;
+        int run = 0;  // the first run that ends after t
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+          if (__shfl_sync(0xffffffffu, incl, run + o - 1) <= t) run += o;
+        const int q = t + __shfl_sync(0xffffffffu, off, run);
+        unsigned kq = 0xffffffffu;
+        if (t < total) {
+          const float4 p = spos[q];
+          const float dx = p.x - pi.x, dy = p.y - pi.y, dz = p.z - pi.z;
+          kq = __float_as_uint(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) + 1u;
+          if (q == t0 && kq < worst) kq = 0u;
+        }
+        const bool add = kq < worst;
+        const unsigned in = __ballot_sync(0xffffffffu, add);
+        if (add) {
+          const int o = count + __popc(in & ((1u << lane) - 1u));
+          key[o] = kq;
+          slot[o] = q;
+        }
+        count += __popc(in);
+        if (count > kSearchCap - 32) worst = knn_cut<KB>(key, slot, count, 0u);
+      }
     }
-    const float r = s * g.h;
-    if (len == KB && worst <= r * r) break;
+    if (count < KB) continue;
+    // done once KB of them are no further than s h (every cell that reaches
+    // that far has been searched)
+    const float rs = s * g.h;
+    const unsigned kr = __float_as_uint(rs * rs) + 1u;
+    __syncwarp();
+    int c = 0;
+    for (int k = lane; k < count; k += 32) c += key[k] <= kr;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (c >= KB) break;
+    worst = knn_cut<KB>(key, slot, count, kr);
   }
-  for (int q = 0; q < KB; q++) nb[(size_t)q * N + i] = q < len ? lj[q][tl] : i;
+  if (count > KB) knn_cut<KB>(key, slot, count, 0u);
+  __syncwarp();
+  for (int k = lane; k < KB; k += 32) {
+    int rank = k, j = i;  // fewer than KB found: the particle itself
+    if (k < count) {
+      const unsigned v = key[k];
+      rank = 0;
+      for (int l = 0; l < count; l++) {
+        const unsigned u = key[l];
+        rank += u < v || (u == v && l < k);
+      }
+      j = sidx[slot[k]];
+    }
+    nb[(size_t)rank * N + i] = j;
+  }
 }
 
 cudaError_t knn_launch(int K, const float *pos, int N, int nper, int *nb, cudaStream_t stream,
@@ -274,12 +386,12 @@ cudaError_t knn_launch(int K, const float *pos, int N, int nper, int *nb, cudaSt
   if (e != cudaSuccess) return e;
   count_launch();
   knn_scatter_kernel<<<grid, 256, 0, stream>>>(pos, N, key, start, cnt, sidx, spos);
-  const int sg = (N + kSearchThreads - 1) / kSearchThreads;
+  const int sg = (N + kSearchWarps - 1) / kSearchWarps;
   count_launch();
-  if (K == 16) knn_search_kernel<17><<<sg, kSearchThreads, 0, stream>>>(N, g, start, sidx, spos, nb);
-  if (K == 32) knn_search_kernel<33><<<sg, kSearchThreads, 0, stream>>>(N, g, start, sidx, spos, nb);
-  if (K == 48) knn_search_kernel<49><<<sg, kSearchThreads, 0, stream>>>(N, g, start, sidx, spos, nb);
-  if (K == 64) knn_search_kernel<65><<<sg, kSearchThreads, 0, stream>>>(N, g, start, sidx, spos, nb);
+  if (K == 16) knn_search_kernel<17><<<sg, 32 * kSearchWarps, 0, stream>>>(N, g, start, sidx, spos, nb);
+  if (K == 32) knn_search_kernel<33><<<sg, 32 * kSearchWarps, 0, stream>>>(N, g, start, sidx, spos, nb);
+  if (K == 48) knn_search_kernel<49><<<sg, 32 * kSearchWarps, 0, stream>>>(N, g, start, sidx, spos, nb);
+  if (K == 64) knn_search_kernel<65><<<sg, 32 * kSearchWarps, 0, stream>>>(N, g, start, sidx, spos, nb);
   e = cudaGetLastError();
   if (e == cudaSuccess && !scratch) e = cudaStreamSynchronize(stream);  // before `local` goes
   return e;
