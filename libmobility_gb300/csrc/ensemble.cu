@@ -159,7 +159,7 @@ __global__ void ens_first(const R *z, R *V0, R *vcur, const int *off3, const int
   }
 }
 
-// One Lanczos iteration i = *iter for every active system, after w = M v_i
+// One Lanczos iteration i = iter[s] for every active system, after w = M v_i
 // (KrylovSubspace, LanczosAlgorithm.cu:131-152), split over CTAs (s, c), c a
 // chunk of kEstChunk elements of system s, in three launches (one CTA per
 // system took a fifth of an iteration for the largest systems).  Each
@@ -195,7 +195,7 @@ __global__ void ens_step_alpha(R *w, const R *V, size_t ldv, const int *iter, co
   if (!active[s]) return;
   const int n = nn[s], nch = (n + kEstChunk - 1) / kEstChunk, c = blockIdx.y;
   if (c >= nch) return;
-  const int i = *iter, o = off3[s];
+  const int i = iter[s], o = off3[s];
   R *ws = w + o;
   const R *vi = V + (size_t)i * ldv + o;
   const R *vp = i > 0 ? vi - ldv : vi;
@@ -222,7 +222,7 @@ __global__ void ens_step_beta(R *w, const R *V, size_t ldv, const int *iter, con
   if (!active[s]) return;
   const int n = nn[s], nch = (n + kEstChunk - 1) / kEstChunk, c = blockIdx.y;
   if (c >= nch) return;
-  const int i = *iter, o = off3[s];
+  const int i = iter[s], o = off3[s];
   R *ws = w + o;
   const R *vi = V + (size_t)i * ldv + o;
   const double al = alpha[s * lim + i];
@@ -252,7 +252,7 @@ __global__ void ens_step_next(const R *w, R *V, R *vcur, size_t ldv, const int *
   if (!active[s]) return;
   const int n = nn[s], nch = (n + kEstChunk - 1) / kEstChunk, c = blockIdx.y;
   if (c >= nch) return;
-  const int i = *iter, o = off3[s];
+  const int i = iter[s], o = off3[s];
   const double b = beta[s * lim + i];
   const R inv = b > 0.0 ? (R)(1.0 / b) : R(0);
   R *vn = V + (size_t)(i + 1) * ldv + o;
@@ -263,7 +263,116 @@ __global__ void ens_step_next(const R *w, R *V, R *vcur, size_t ldv, const int *
   }
 }
 
-__global__ void ens_iter_inc(int *iter) { *iter += 1; }
+__global__ void ens_iter_inc(int *iter, int nsys) {
+  for (int s = threadIdx.x; s < nsys; s += blockDim.x) iter[s] += 1;
+}
+
+// The whole iteration in one launch where every system has at most
+// kStepCluster chunks: one thread-block cluster per system, one CTA per chunk
+// with its elements in registers, and the two sums over the chunks through
+// distributed shared memory.  Element for element and sum for sum the
+// arithmetic of the three kernels above (block and chunk sums in the same
+// order), so the results are the same bits.  Latency-bound: 48 systems of 1000
+// to 2000 particles took 15 us in four launches, 6 in one.  A larger system
+// would give the CTAs of its cluster several chunks each while the rest of the
+// chip idles; ensembles with one keep the kernels above.
+constexpr int kStepCluster = 8;  // the portable cluster size
+
+template <class R>
+__global__ void __launch_bounds__(kEnsThreads)
+ens_step_cluster(const R *__restrict__ w, R *V, R *vcur, size_t ldv, int *iter, const int *off3,
+                 const int *nn, const int *active, const double *normz, double *beta, int lim,
+                 double *host_ab) {
+  __shared__ double warp_sum_[kEnsThreads / 32];
+  __shared__ double part[2];
+  __shared__ double sc;
+  const int c = (int)cluster_ctarank(), s = blockIdx.x / cluster_nctarank();
+  if (!active[s]) return;  // the whole cluster
+  constexpr int kPer = kEstChunk / kEnsThreads;
+  const int n = nn[s], nch = (n + kEstChunk - 1) / kEstChunk;
+  const int i = iter[s], o = off3[s];
+  const R *vi = V + (size_t)i * ldv + o;
+  const R *vp = i > 0 ? vi - ldv : vi;
+  const R bprev = i > 0 ? (R)beta[s * lim + i - 1] : R(0);
+  const int e0 = c * kEstChunk + threadIdx.x;
+  // sum of every thread's value over the system, in thread 0 of each CTA
+  auto system_sum = [&](double v, int slot) {
+#pragma unroll
+    for (int q = 16; q > 0; q >>= 1) v += __shfl_xor_sync(0xffffffffu, v, q);
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) warp_sum_[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = 0.0;
+      for (int q = 0; q < kEnsThreads / 32; q++) t += warp_sum_[q];
+      part[slot] = t;
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    double t = 0.0;
+    if (threadIdx.x < 32) {
+      const double p = lane < nch ? ld_dsmem(&part[slot], (unsigned)lane) : 0.0;
+      for (int q = 0; q < nch; q++) t += __shfl_sync(0xffffffffu, p, q);
+    }
+    return t;
+  };
+  R x[kPer], v[kPer];
+  double acc = 0.0;
+#pragma unroll
+  for (int u = 0; u < kPer; u++) {
+    const int e = e0 + u * kEnsThreads;
+    x[u] = v[u] = R(0);
+    if (e < n) {
+      R y = w[o + e];
+      v[u] = vi[e];
+      if (i > 0) y -= bprev * vp[e];
+      x[u] = y;
+      acc += (double)y * (double)v[u];
+    }
+  }
+  const double ta = system_sum(acc, 0);
+  if (threadIdx.x == 0) sc = ta;
+  __syncthreads();
+  const double al = sc;
+  const R alr = (R)al;
+  acc = 0.0;
+#pragma unroll
+  for (int u = 0; u < kPer; u++) {
+    if (e0 + u * kEnsThreads < n) {
+      const R y = x[u] - alr * v[u];
+      x[u] = y;
+      acc += (double)y * (double)y;
+    }
+  }
+  const double tb = system_sum(acc, 1);
+  if (threadIdx.x == 0) {
+    double b = sqrt(tb);
+    if (b < 1e-3 * al / normz[s]) b = 0.0;
+    sc = b > 0.0 ? 1.0 / b : -1.0;
+    if (c == 0) {
+      beta[s * lim + i] = b;
+      host_ab[2 * (s * lim + i)] = al;
+      host_ab[2 * (s * lim + i) + 1] = b;
+      iter[s] = i + 1;  // read by all before the first sum
+    }
+  }
+  __syncthreads();
+  cluster_arrive();  // this CTA has read the others' sums
+  const double invd = sc;
+  const R inv = (R)invd;
+  R *vn = V + (size_t)(i + 1) * ldv + o;
+#pragma unroll
+  for (int u = 0; u < kPer; u++) {
+    const int e = e0 + u * kEnsThreads;
+    if (e < n) {
+      const R y = invd >= 0.0 ? x[u] * inv : (e == 0 ? R(1) : R(0));
+      vn[e] = y;
+      vcur[o + e] = y;
+    }
+  }
+  cluster_wait();  // nobody reads this CTA's shared memory any more
+}
 
 // Result estimate y_s = |z_s| V_s c_s (m basis vectors) for the systems due
 // for a check, written to ynew, and err_s = |y_s - yold_s| / |yold_s|
@@ -901,18 +1010,35 @@ template <class R> void Ensemble<R>::build_graph(R *V, size_t ldv) {
   LMG_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   try {
     launch_groups(vcur_.ptr, w_.ptr, active_.ptr, st);
-    const dim3 cg(nsys_, est_chunks_);
-    ens_step_alpha<R><<<cg, kEnsThreads, 0, st>>>(w_.ptr, V, ldv, iter_.ptr, off3_.ptr, nn_.ptr,
-                                                  active_.ptr, beta_.ptr, alpha_.ptr, kEnsLimit,
-                                                  step_part_.ptr, step_ticket_.ptr);
-    ens_step_beta<R><<<cg, kEnsThreads, 0, st>>>(w_.ptr, V, ldv, iter_.ptr, off3_.ptr, nn_.ptr,
-                                                 active_.ptr, normz_.ptr, alpha_.ptr, beta_.ptr,
-                                                 kEnsLimit, hab_.device_ptr(), step_part_.ptr,
-                                                 step_ticket_.ptr);
-    ens_step_next<R><<<cg, kEnsThreads, 0, st>>>(w_.ptr, V, vcur_.ptr, ldv, iter_.ptr,
-                                                 off3_.ptr, nn_.ptr, active_.ptr, beta_.ptr,
-                                                 kEnsLimit);
-    ens_iter_inc<<<1, 1, 0, st>>>(iter_.ptr);
+    if (est_chunks_ <= kStepCluster) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)est_chunks_ * (unsigned)nsys_);
+      cfg.blockDim = dim3(kEnsThreads);
+      cfg.stream = st;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = est_chunks_;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      LMG_CUDA(cudaLaunchKernelEx(&cfg, ens_step_cluster<R>, (const R *)w_.ptr, V, vcur_.ptr, ldv,
+                                  iter_.ptr, (const int *)off3_.ptr, (const int *)nn_.ptr,
+                                  (const int *)active_.ptr, (const double *)normz_.ptr,
+                                  beta_.ptr, kEnsLimit, hab_.device_ptr()));
+    } else {
+      const dim3 cg(nsys_, est_chunks_);
+      ens_step_alpha<R><<<cg, kEnsThreads, 0, st>>>(w_.ptr, V, ldv, iter_.ptr, off3_.ptr, nn_.ptr,
+                                                    active_.ptr, beta_.ptr, alpha_.ptr, kEnsLimit,
+                                                    step_part_.ptr, step_ticket_.ptr);
+      ens_step_beta<R><<<cg, kEnsThreads, 0, st>>>(w_.ptr, V, ldv, iter_.ptr, off3_.ptr, nn_.ptr,
+                                                   active_.ptr, normz_.ptr, alpha_.ptr, beta_.ptr,
+                                                   kEnsLimit, hab_.device_ptr(), step_part_.ptr,
+                                                   step_ticket_.ptr);
+      ens_step_next<R><<<cg, kEnsThreads, 0, st>>>(w_.ptr, V, vcur_.ptr, ldv, iter_.ptr,
+                                                   off3_.ptr, nn_.ptr, active_.ptr, beta_.ptr,
+                                                   kEnsLimit);
+      ens_iter_inc<<<1, 256, 0, st>>>(iter_.ptr, nsys_);
+    }
     LMG_CUDA(cudaGetLastError());
   } catch (...) {
     cudaStreamEndCapture(st, &g);
@@ -1004,7 +1130,7 @@ void Ensemble<R>::sqrt_mdot_w(const void *dW, size_t ndW, void *U, size_t nU, do
   int *due = due_.ensure(nsys_);
   int *act = active_.ensure(nsys_);
   int *par = parity_.ensure(nsys_);
-  int *iter = iter_.ensure(1);
+  int *iter = iter_.ensure(nsys_);
   // pinned flags: two slots for active-flag uploads used in turn (an upload
   // issued at one check has run before its slot is reused two checks later:
   // the host has waited meanwhile for an event recorded after it), and one
@@ -1029,12 +1155,13 @@ void Ensemble<R>::sqrt_mdot_w(const void *dW, size_t ndW, void *U, size_t nU, do
   // all systems active, iteration 0
   for (int q = 0; q < nsys_; q++) hf[q] = 1;
   LMG_CUDA(cudaMemcpyAsync(act, hf, nsys_ * sizeof(int), cudaMemcpyHostToDevice, st));
-  LMG_CUDA(cudaMemsetAsync(iter, 0, sizeof(int), st));
+  LMG_CUDA(cudaMemsetAsync(iter, 0, nsys_ * sizeof(int), st));
   ens_first<R><<<nsys_, kEnsThreads, 0, st>>>(z, V, vc, off3_.ptr, nn_.ptr, nz);
   count_launch();
   LMG_CUDA(cudaGetLastError());
   build_graph(V, ld);
-  const int per_iter = (int)groups_.size() + 4;  // groups, three step kernels, counter
+  // groups, then one step kernel or three and the counters
+  const int per_iter = (int)groups_.size() + (est_chunks_ <= kStepCluster ? 1 : 4);
   auto issue = [&](int i) {
     LMG_CUDA(cudaGraphLaunch(graph_, st));
     for (int k = 0; k < per_iter; k++) count_launch();

@@ -35,3 +35,31 @@ def test_tuned_plans_sum_every_source(cuda, oracle, sizes, repeat):
                             viscosity=1.0, wall=g != "open", include_angular=0)
         assert np.abs(U[b:b + len(p)] - Uo).max() <= 1e-5 * np.abs(Uo).max(), (len(p), g)
         b += len(p)
+
+
+@pytest.mark.parametrize("precision", ["float", "double"])
+@pytest.mark.parametrize("sizes", [[1, 2, 100, 341], [341, 342, 500], [300, 700, 1365, 1366],
+                                   [2049, 2730, 60]])
+def test_one_launch_step_is_the_three_kernel_step(cuda, sizes, precision):
+    """Systems of up to 8 chunks of 1024 values take one cluster launch a step.
+    With one larger system beside them (4100 particles, its own group, so the
+    others' products stay the same) the step goes through three kernels: same
+    arithmetic in the same order, so the same bits."""
+    from libmobility_gb300.ensemble import Ensemble
+    rng = np.random.default_rng(sum(sizes))
+    sizes = sizes + [4100]
+    pos = np.concatenate([rng.uniform(0, 2.5 * n ** (1 / 3), (n, 3)) for n in sizes])
+    dW = rng.normal(size=(sum(sizes), 3))
+    dtype = np.float32 if precision == "float" else np.float64
+    out = []
+    for k in (len(sizes) - 1, len(sizes)):
+        m = sum(sizes[:k])
+        e = Ensemble(precision=precision)
+        e.setSystems(sizes[:k], ["open"] * k, [0.0] * k)
+        e.initialize(1.0, 1.0, tolerance=1e-4, seed=1, autotune=False)
+        e.setPositions(pos[:m].astype(dtype))
+        r = e.sqrtMdotW(dW[:m].astype(dtype))
+        out.append((np.asarray(r[0]), np.asarray(r[1])))
+    m = sum(sizes[:-1])
+    assert (out[0][1] == out[1][1][:-1]).all()
+    assert np.array_equal(out[0][0][:m], out[1][0][:m])
