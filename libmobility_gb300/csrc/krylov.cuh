@@ -103,6 +103,13 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // Sums `v` over the block; result valid in thread 0.
+// In a kernel launched ahead of its predecessor's end: waits for that end, then
+// lets the next one be launched.
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+}
+
 template <int NV>
 __device__ __forceinline__ void block_sum(double (&v)[NV]) {
   __shared__ double red[NV][kRedThreads / 32];
@@ -1055,7 +1062,8 @@ __global__ void krylov_check_kernel(const R *V, size_t ldv, int m, const double 
 // device: the last block of a reduction works out what the next kernel needs,
 // so an iteration is seven launches that nothing waits between; the host looks
 // at `done` an iteration late.  Once done (or broken down) the kernels of a
-// further iteration return at once.
+// further iteration return at once.  All but the first are launched while the
+// kernel before them ends (programmatic dependent launch) and wait in pdl_wait.
 // ---------------------------------------------------------------------------
 struct BicgScalars {
   double tol2, rho, alpha, omega;  // |r|^2 to reach; the recurrence (FP64 throughout)
@@ -1094,6 +1102,7 @@ __global__ void bicg_init_kernel(const R *b, R *x, R *p, R *v, R *r, R *rhat, si
 // p = r + beta (p - omega v)
 template <class R>
 __global__ void bicg_p_kernel(R *p, const R *r, const R *v, size_t n, const BicgScalars *sc) {
+  pdl_wait();
   if (sc->done) return;
   const R b = sc->beta_f, o = sc->omega_f;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n;
@@ -1105,6 +1114,7 @@ __global__ void bicg_p_kernel(R *p, const R *r, const R *v, size_t n, const Bicg
 template <class R>
 __global__ void bicg_alpha_kernel(const R *rhat, const R *v, size_t n, double *partials,
                                   unsigned *ticket, BicgScalars *sc) {
+  pdl_wait();
   if (sc->done) return;
   double d[1] = {0.0};
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n;
@@ -1122,6 +1132,7 @@ __global__ void bicg_alpha_kernel(const R *rhat, const R *v, size_t n, double *p
 template <class R>
 __global__ void bicg_s_kernel(R *s, const R *r, const R *v, size_t n, double *partials,
                               unsigned *ticket, BicgScalars *sc) {
+  pdl_wait();
   if (sc->done) return;
   const R a = sc->alpha_f;
   double d[1] = {0.0};
@@ -1139,6 +1150,7 @@ __global__ void bicg_s_kernel(R *s, const R *r, const R *v, size_t n, double *pa
 template <class R>
 __global__ void bicg_omega_kernel(const R *t, const R *s, size_t n, double *partials,
                                   unsigned *ticket, BicgScalars *sc) {
+  pdl_wait();
   if (sc->done) return;
   double d[2] = {0.0, 0.0};
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n;
@@ -1158,6 +1170,7 @@ template <class R>
 __global__ void bicg_xr_kernel(R *x, const R *p, const R *s, const R *t, R *r, const R *rhat,
                                size_t n, double *partials, unsigned *ticket, BicgScalars *sc,
                                BicgScalars *host) {
+  pdl_wait();
   if (sc->done) return;
   const R a = sc->alpha_f, o = sc->omega_f;
   double d[2] = {0.0, 0.0};

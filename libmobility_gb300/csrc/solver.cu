@@ -1325,23 +1325,35 @@ template <class R> int Solver<R>::solve_p(const R *b, R *x) {
     bicg_init_kernel<R><<<blocks, kRedThreads, 0, st>>>(b, x, p, v, r, rh, n, rp, tk, sc,
                                                         host_dev);
     count_launch();
+    auto launch = [&](auto kernel, auto... args) {
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at[0].val.programmaticStreamSerializationAllowed = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(blocks);
+      cfg.blockDim = dim3(kRedThreads);
+      cfg.stream = st;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      LMG_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+      count_launch();
+    };
     auto product = [&](const R *in, R *out) {
       LMG_CUDA(precond_rows_launch(prec_k_, prec_rows_, false, prec_scale(), N, in, out,
-                                   &sc->done, st));
+                                   &sc->done, st, true));
     };
+    const R *cr = r, *crh = rh, *cp = p, *cv = v, *cs = s, *ct = t;
+    const BicgScalars *csc = sc;
     const int max_it = 500;
     for (int it = 1; it <= max_it + 1; it++) {
       if (it <= max_it) {
-        bicg_p_kernel<R><<<blocks, kRedThreads, 0, st>>>(p, r, v, n, sc);
+        launch(bicg_p_kernel<R>, p, cr, cv, n, csc);
         product(p, v);
-        bicg_alpha_kernel<R><<<blocks, kRedThreads, 0, st>>>(rh, v, n, rp, tk, sc);
-        bicg_s_kernel<R><<<blocks, kRedThreads, 0, st>>>(s, r, v, n, rp, tk, sc);
+        launch(bicg_alpha_kernel<R>, crh, cv, n, rp, tk, sc);
+        launch(bicg_s_kernel<R>, s, cr, cv, n, rp, tk, sc);
         product(s, t);
-        bicg_omega_kernel<R><<<blocks, kRedThreads, 0, st>>>(t, s, n, rp, tk, sc);
-        bicg_xr_kernel<R><<<blocks, kRedThreads, 0, st>>>(x, p, s, t, r, rh, n, rp, tk, sc,
-                                                          host_dev);
-        for (int k = 0; k < 5; k++) count_launch();
-        LMG_CUDA(cudaGetLastError());
+        launch(bicg_omega_kernel<R>, ct, cs, n, rp, tk, sc);
+        launch(bicg_xr_kernel<R>, x, cp, cs, ct, r, crh, n, rp, tk, sc, host_dev);
         LMG_CUDA(cudaEventRecord(ev_bicg_[it & 1], st));
       }
       if (it == 1) continue;
