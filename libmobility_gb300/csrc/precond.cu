@@ -11,6 +11,7 @@
 #include <cuda_fp16.h>
 
 #include "launch_count.hpp"
+#include "pack2.cuh"
 #include "precond.cuh"
 #include "tc_gemm.cuh"
 
@@ -1008,52 +1009,76 @@ __global__ void adam_kernel(size_t n, float *w, const float *g, float *m, float 
 // slabs of A and B in shared memory, 8 x 8 outputs per thread in two 4-wide
 // groups per dimension (rows 4 ty + r and 64 + 4 ty + r, columns likewise
 // with tx), so the inner loop reads shared memory as float4 without bank
-// conflicts and does 64 FMAs per 4 vector loads.  Tile loads put consecutive
-// threads on consecutive addresses for every transposition.
+// conflicts and does 64 FMAs per 4 vector loads, two columns at a time
+// (fma.rn.f32x2: the same rounding).  Tile loads put consecutive threads on
+// consecutive addresses for every transposition.  Bound by the FMA pipe's
+// operand reads (three register pairs an instruction): the next slab's loads
+// are in flight while a slab is multiplied, into the other half of the shared
+// memory, one barrier a slab.  M = 16384, N = K = 512: 224 us with single FMAs
+// and loads between the slabs, 207 us; M = 65536: 814 and 715 us.
 constexpr int kGT2 = 128, kGK2 = 16;
 
 template <bool TA, bool TB>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 gemm_kernel2(int M, int N, int K, const float *__restrict__ A, int lda,
              const float *__restrict__ B, int ldb, float *__restrict__ C, int ldc,
              const float *__restrict__ bias, int act, float beta) {
-  __shared__ __align__(16) float sa[kGK2][kGT2 + 4];
-  __shared__ __align__(16) float sb[kGK2][kGT2 + 4];
+  constexpr int kLoads = (kGK2 * kGT2) / 256;
+  __shared__ __align__(16) float sa[2][kGK2][kGT2 + 4];
+  __shared__ __align__(16) float sb[2][kGK2][kGT2 + 4];
   const int tid = threadIdx.x;
   const int tx = tid % 16, ty = tid / 16;
   const int row0 = blockIdx.y * kGT2, col0 = blockIdx.x * kGT2;
-  float acc[8][8] = {};
-  for (int k0 = 0; k0 < K; k0 += kGK2) {
+  // element q of this thread: (mm, kk) of the A tile, (kk, nn) of the B tile
+  auto a_mm = [&](int q) { return TA ? tid % kGT2 : (tid + 256 * q) / kGK2; };
+  auto a_kk = [&](int q) { return TA ? (tid + 256 * q) / kGT2 : tid % kGK2; };
+  auto b_nn = [&](int q) { return TB ? (tid + 256 * q) / kGK2 : tid % kGT2; };
+  auto b_kk = [&](int q) { return TB ? tid % kGK2 : (tid + 256 * q) / kGT2; };
+  float va[kLoads], vb[kLoads];
+  auto load = [&](int k0) {
 #pragma unroll
-    for (int q = 0; q < (kGK2 * kGT2) / 256; q++) {
-      const int t = tid + 256 * q;
-      // A tile: element (mm, kk) = op(A)[row0 + mm][k0 + kk]
-      const int amm = TA ? t % kGT2 : t / kGK2, akk = TA ? t / kGT2 : t % kGK2;
-      const int gi = row0 + amm, gk = k0 + akk;
-      float va = 0.f;
-      if (gi < M && gk < K) va = TA ? A[(size_t)gk * lda + gi] : A[(size_t)gi * lda + gk];
-      sa[akk][amm] = va;
-      // B tile: element (kk, nn) = op(B)[k0 + kk][col0 + nn]
-      const int bnn = TB ? t / kGK2 : t % kGT2, bkk = TB ? t % kGK2 : t / kGT2;
-      const int gj = col0 + bnn, gk2 = k0 + bkk;
-      float vb = 0.f;
-      if (gj < N && gk2 < K) vb = TB ? B[(size_t)gj * ldb + gk2] : B[(size_t)gk2 * ldb + gj];
-      sb[bkk][bnn] = vb;
+    for (int q = 0; q < kLoads; q++) {
+      const int gi = row0 + a_mm(q), gk = k0 + a_kk(q);
+      va[q] = 0.f;
+      if (gi < M && gk < K) va[q] = TA ? A[(size_t)gk * lda + gi] : A[(size_t)gi * lda + gk];
+      const int gj = col0 + b_nn(q), gk2 = k0 + b_kk(q);
+      vb[q] = 0.f;
+      if (gj < N && gk2 < K) vb[q] = TB ? B[(size_t)gj * ldb + gk2] : B[(size_t)gk2 * ldb + gj];
     }
-    __syncthreads();
+  };
+  auto stage = [&](int h) {
+#pragma unroll
+    for (int q = 0; q < kLoads; q++) {
+      sa[h][a_kk(q)][a_mm(q)] = va[q];
+      sb[h][b_kk(q)][b_nn(q)] = vb[q];
+    }
+  };
+  F2 acc[8][4];
+#pragma unroll
+  for (int r = 0; r < 8; r++)
+#pragma unroll
+    for (int c = 0; c < 4; c++) acc[r][c] = bc(0.f);
+  load(0);
+  stage(0);
+  __syncthreads();
+  int h = 0;
+  for (int k0 = 0; k0 < K; k0 += kGK2, h ^= 1) {
+    const bool more = k0 + kGK2 < K;
+    if (more) load(k0 + kGK2);
 #pragma unroll
     for (int kk = 0; kk < kGK2; kk++) {
-      const float4 a0 = *reinterpret_cast<const float4 *>(&sa[kk][4 * ty]);
-      const float4 a1 = *reinterpret_cast<const float4 *>(&sa[kk][64 + 4 * ty]);
-      const float4 b0 = *reinterpret_cast<const float4 *>(&sb[kk][4 * tx]);
-      const float4 b1 = *reinterpret_cast<const float4 *>(&sb[kk][64 + 4 * tx]);
+      const float4 a0 = *reinterpret_cast<const float4 *>(&sa[h][kk][4 * ty]);
+      const float4 a1 = *reinterpret_cast<const float4 *>(&sa[h][kk][64 + 4 * ty]);
+      const float4 b0 = *reinterpret_cast<const float4 *>(&sb[h][kk][4 * tx]);
+      const float4 b1 = *reinterpret_cast<const float4 *>(&sb[h][kk][64 + 4 * tx]);
       const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+      const F2 b[4] = {mk2(b0.x, b0.y), mk2(b0.z, b0.w), mk2(b1.x, b1.y), mk2(b1.z, b1.w)};
 #pragma unroll
       for (int r = 0; r < 8; r++)
 #pragma unroll
-        for (int c = 0; c < 8; c++) acc[r][c] = fmaf(a[r], b[c], acc[r][c]);
+        for (int c = 0; c < 4; c++) acc[r][c] = fma2(bc(a[r]), b[c], acc[r][c]);
     }
+    if (more) stage(h ^ 1);  // read last before the barrier of the slab before
     __syncthreads();
   }
 #pragma unroll
@@ -1064,7 +1089,7 @@ gemm_kernel2(int M, int N, int K, const float *__restrict__ A, int lda,
     for (int c = 0; c < 8; c++) {
       const int gj = col0 + (c < 4 ? 4 * tx + c : 64 + 4 * tx + c - 4);
       if (gj >= N) continue;
-      float v = acc[r][c];
+      float v = c & 1 ? acc[r][c / 2].v.y : acc[r][c / 2].v.x;
       if (bias) v += bias[gj];
       if (beta != 0.f) v += beta * C[(size_t)gi * ldc + gj];
       if (act == 1) v = tanhf(v);
