@@ -2,6 +2,7 @@
 // is described in mdot_pairs.cuh.  Compiled once per precision (LMG_REAL).
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "bounds.cuh"
 #include "grid_sync.cuh"
@@ -33,6 +34,8 @@ template <> struct LaneTypes<float> { using V = F2; using L = float2; };
 template <> struct LaneTypes<double> { using V = double; using L = double; };
 __device__ __forceinline__ float lane_value(float2 v, int q) { return q ? v.y : v.x; }
 __device__ __forceinline__ double lane_value(double v, int) { return v; }
+__device__ __forceinline__ float lane_of(F2 v, int q) { return q ? v.v.y : v.v.x; }
+__device__ __forceinline__ double lane_of(double v, int) { return v; }
 
 __device__ __forceinline__ F2 splat(float x, F2) { return bc(x); }
 __device__ __forceinline__ double splat(double x, double) { return x; }
@@ -65,6 +68,7 @@ template <class R> struct PairsArgs {
   int warps;
   bool first, last;   // of the passes
   bool wide;          // a slot of any tile is 8-byte aligned in pos, F and T
+  int share;          // warps that fold a component of a tile together (1 or 4)
   R inv_a;
   PairScale<R> k;
   R *part;
@@ -185,9 +189,16 @@ template <class R, bool WALL, bool ANG> constexpr int pairs_min_blocks() {
 // With fewer than this many steps a warp, two blocks per SM are launched: the
 // ranges are longer, their partials fewer, and a warp alone on its scheduler
 // still runs at seven eighths of its rate (N = 2048 wall with torques, 9 steps
-// a warp with three blocks: 24.4 us with three, 22.0 us with two; N = 3000 open
-// with torques, 15 steps: 26.2 and 24.5 us; N = 6001, 59 steps: 69.9 and 71.0).
-constexpr long long kPairsFewSteps = 24;
+// a warp with three blocks: 23.4 us with three, 21.1 us with two; N = 3000 open
+// with torques, 20 steps: 25.2 and 23.9 us; N = 6001, 78 steps: 69.6 and 71).
+// The line is lower with torques in small batches, whose sums have few partials
+// either way: 64 batches of 333 above a wall, 24 steps, 48.4 us with three and
+// 51.0 with two, 32 of 500 in open space, 20 steps, 27.5 and 29.1 us (one batch
+// of 3000, 20 steps, 25.2 and 23.9).  Not with forces alone: 64 batches of 333,
+// 18 steps, 18.4 us with four blocks and 17.6 with two.
+constexpr long long pairs_few_steps(bool ang, long long tpb) {
+  return ang && tpb <= 32 ? 16 : 24;
+}
 
 // A warp's shared memory: tiles I and J, the next ones as they arrive, the J
 // sums, the row's I sums (sum, compensation).
@@ -368,8 +379,24 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
       const int k = __ffs(st) - 1;
       if ((near >> k) & 1u) {
         const int s = (lane + k) & 31;
+        // which of the slots' pairs (NS q + h); FP32 takes the distances of all
+        // four first, which spares most of the loads below
+        unsigned which = (1u << (NS * NS)) - 1u;
+        if constexpr (NS == 2) {
+          which = 0u;
+#pragma unroll
+          for (int q = 0; q < NS; q++) {
+            V d[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) d[c] = vi[q][c] - reinterpret_cast<const V *>(w.J[c])[s];
+            const V r2 = vfma(d[2], d[2], vfma(d[0], d[0], d[1] * d[1]));
+#pragma unroll
+            for (int h = 0; h < NS; h++) which |= below4(lane_of(r2, h)) ? 1u << (NS * q + h) : 0u;
+          }
+        }
 #pragma unroll 1
-        for (int qh = 0; qh < NS * NS; qh++) {
+        for (; which != 0u; which &= which - 1u) {
+          const int qh = __ffs(which) - 1;
           const int li = NS * lane + qh / NS, lj = NS * s + qh % NS;
           R pi[9], pj[9];
 #pragma unroll
@@ -379,7 +406,7 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
           }
           const R dx = pi[0] - pj[0], dy = pi[1] - pj[1], dz = pi[2] - pj[2];
           const R r2 = vfma(dz, dz, vfma(dx, dx, dy * dy));
-          if (!below4(r2)) continue;
+          if (NS == 1 && !below4(r2)) continue;
           Vec6<R> o = {0, 0, 0, 0, 0, 0};
           pair_correct<R, WALL, ANG>(pi, pj, r2, o);
           const R ai[6] = {o.ux, o.uy, o.uz, o.wx, o.wy, o.wz};
@@ -418,100 +445,116 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
     return;
   }
 
-  // ---- fold the partials: a block takes 32 slots of one component of a tile at
-  // a time, each warp every fourth partial, sixteen loads ahead ----
+  // ---- fold the partials: one component of a tile at a time, by a warp or by
+  // the block's four warps, each taking every fourth partial, sixteen loads ahead ----
   R (*red)[2][TS] = reinterpret_cast<R (*)[2][TS]>(&sm[0]);  // [warp][S, C][particle]
   using L = typename LaneTypes<R>::L;
   const int *cut_begin = a.cuts, *cut_warp = a.cuts + a.tiles + 1;
   // (a pass over a band of rows still touches every tile of its batch)
   const int t_lo = a.row0 / a.tpb * a.tpb, t_hi = ((a.row1 - 1) / a.tpb + 1) * a.tpb;
-  for (int unit = blockIdx.x; unit < (t_hi - t_lo) * NC; unit += gridDim.x) {
-    const int t = t_lo + unit / NC, comp = unit % NC;
-    const int tb = t / a.tpb, tl = t - tb * a.tpb;  // batch, tile in it
-    const L *src = reinterpret_cast<const L *>(a.part + comp * TS) + lane;
-    R S[NS], C[NS];
+  auto fold_units = [&](auto share) {
+    constexpr bool alone = decltype(share)::value == 1;
+    constexpr int step = alone ? 1 : NW;
+    const int sub = alone ? 0 : warp;
+    const int stride = alone ? (int)gridDim.x * NW : (int)gridDim.x;
+    for (int unit = alone ? gw : (int)blockIdx.x; unit < (t_hi - t_lo) * NC; unit += stride) {
+      const int t = t_lo + unit / NC, comp = unit % NC;
+      const int tb = t / a.tpb, tl = t - tb * a.tpb;  // batch, tile in it
+      const L *src = reinterpret_cast<const L *>(a.part + comp * TS) + lane;
+      R S[NS], C[NS];
 #pragma unroll
-    for (int q = 0; q < NS; q++) S[q] = C[q] = R(0);
-    constexpr int UN = 16;
-    // adds the partials slot(e), e = warp, warp + 4, ... < n
-    auto gather = [&](int n, auto slot) {
-      for (int e0 = warp; e0 < n; e0 += UN * NW) {
-        L v[UN];
+      for (int q = 0; q < NS; q++) S[q] = C[q] = R(0);
+      constexpr int UN = 16;
+      // adds the partials slot(e), e = sub, sub + step, ... < n
+      auto gather = [&](int n, auto slot) {
+        for (int e0 = sub; e0 < n; e0 += UN * step) {
+          L v[UN];
 #pragma unroll
-        for (int u = 0; u < UN; u++) {
-          const int e = e0 + u * NW;
-          v[u] = L();
-          if (e < n) {
-            const size_t sl = slot(e);
-            if (LMG_IN_BOUNDS((sl + 1) * EL <= a.part_elems, 23, sl))
-              v[u] = __ldcg(src + sl * (EL / NS));
+          for (int u = 0; u < UN; u++) {
+            const int e = e0 + u * step;
+            v[u] = L();
+            if (e < n) {
+              const size_t sl = slot(e);
+              if (LMG_IN_BOUNDS((sl + 1) * EL <= a.part_elems, 23, sl))
+                v[u] = __ldcg(src + sl * (EL / NS));
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < UN; u++) {
+#pragma unroll
+            for (int q = 0; q < NS; q++) fold_in(S[q], C[q], lane_value(v[u], q));
           }
         }
-#pragma unroll
-        for (int u = 0; u < UN; u++) {
-#pragma unroll
-          for (int q = 0; q < NS; q++) fold_in(S[q], C[q], lane_value(v[u], q));
-        }
-      }
-    };
-    // J side: rows I < tl of its batch in this pass
-    const int I_lo = max(0, a.row0 - tb * a.tpb), I_hi = min(tl, a.row1 - tb * a.tpb);
-    const int base = tb * ppb - P0 + tl;
-    gather(I_hi - I_lo, [&](int e) {
-      const int I = I_lo + e;
-      return (size_t)(base + local_before(a.tpb, I) - I);
-    });
-    // I side: the row's own partial, then those of warps that began in it
-    if (t >= a.row0 && t < a.row1) {
-      const unsigned xs = 32u * (unsigned)(tb * ppb + local_before(a.tpb, tl) - P0);
-      const unsigned xe = xs + 32u * (unsigned)(a.tpb - tl);
-      const int w_lo = (int)(xs / a.per_warp), w_hi = (int)((xe - 1u) / a.per_warp);
-      gather(w_hi - w_lo + 1, [&](int e) {
-        return e == 0 ? slot_row + (t - a.row0) : slot_irow + w_lo + e;
+      };
+      // J side: rows I < tl of its batch in this pass
+      const int I_lo = max(0, a.row0 - tb * a.tpb), I_hi = min(tl, a.row1 - tb * a.tpb);
+      const int base = tb * ppb - P0 + tl;
+      gather(I_hi - I_lo, [&](int e) {
+        const int I = I_lo + e;
+        return (size_t)(base + local_before(a.tpb, I) - I);
       });
-    }
-    // J side of tile pairs that a warp began in
-    const int q_lo = __ldg(cut_begin + t);
-    gather(__ldg(cut_begin + t + 1) - q_lo,
-           [&](int e) { return slot_cut + __ldg(cut_warp + q_lo + e); });
+      // I side: the row's own partial, then those of warps that began in it
+      if (t >= a.row0 && t < a.row1) {
+        const unsigned xs = 32u * (unsigned)(tb * ppb + local_before(a.tpb, tl) - P0);
+        const unsigned xe = xs + 32u * (unsigned)(a.tpb - tl);
+        const int w_lo = (int)(xs / a.per_warp), w_hi = (int)((xe - 1u) / a.per_warp);
+        gather(w_hi - w_lo + 1, [&](int e) {
+          return e == 0 ? slot_row + (t - a.row0) : slot_irow + w_lo + e;
+        });
+      }
+      // J side of tile pairs that a warp began in
+      const int q_lo = __ldg(cut_begin + t);
+      gather(__ldg(cut_begin + t + 1) - q_lo,
+             [&](int e) { return slot_cut + __ldg(cut_warp + q_lo + e); });
+      auto finish = [&](int p, R s, R c) {
+        const size_t o = ((size_t)t * NC + comp) * TS + p;
+        if (!a.first) {
+          fold_in(s, c, a.acc[2 * o]);
+          c += a.acc[2 * o + 1];
+        }
+        if constexpr (!alone) {
 #pragma unroll
-    for (int q = 0; q < NS; q++) {
-      red[warp][0][NS * lane + q] = S[q];
-      red[warp][1][NS * lane + q] = C[q];
-    }
-    __syncthreads();
-    for (int p = threadIdx.x; p < TS; p += kPairsThreads) {
-      R s = red[0][0][p], c = red[0][1][p];
-      const size_t o = ((size_t)t * NC + comp) * TS + p;
-      if (!a.first) {
-        fold_in(s, c, a.acc[2 * o]);
-        c += a.acc[2 * o + 1];
-      }
+          for (int q = 1; q < NW; q++) {
+            fold_in(s, c, red[q][0][p]);
+            c += red[q][1][p];
+          }
+        }
+        if (!a.last) {
+          a.acc[2 * o] = s;
+          a.acc[2 * o + 1] = c;
+          return;
+        }
+        const int l = tl * TS + p, i = tb * a.nper + l;
+        if (l >= a.nper || !LMG_IN_BOUNDS(i < a.N, 24, i)) return;
+        s += c;
+        if (WALL) {
+          const R z = mul_rn(a.pos[3 * (size_t)i + 2], a.inv_a);
+          s *= z < R(0) ? R(0) : (z > R(1) ? R(1) : z);
+        }
+        if (comp < 3) {
+          if (a.U) a.U[3 * (size_t)i + comp] = s;
+        } else if (a.W) {
+          a.W[3 * (size_t)i + (comp - 3)] = a.k.sW * s;
+        }
+      };
+      if constexpr (alone) {
 #pragma unroll
-      for (int q = 1; q < NW; q++) {
-        fold_in(s, c, red[q][0][p]);
-        c += red[q][1][p];
-      }
-      if (!a.last) {
-        a.acc[2 * o] = s;
-        a.acc[2 * o + 1] = c;
-        continue;
-      }
-      const int l = tl * TS + p, i = tb * a.nper + l;
-      if (l >= a.nper || !LMG_IN_BOUNDS(i < a.N, 24, i)) continue;
-      s += c;
-      if (WALL) {
-        const R z = mul_rn(a.pos[3 * (size_t)i + 2], a.inv_a);
-        s *= z < R(0) ? R(0) : (z > R(1) ? R(1) : z);
-      }
-      if (comp < 3) {
-        if (a.U) a.U[3 * (size_t)i + comp] = s;
-      } else if (a.W) {
-        a.W[3 * (size_t)i + (comp - 3)] = a.k.sW * s;
+        for (int q = 0; q < NS; q++) finish(NS * lane + q, S[q], C[q]);
+      } else {
+#pragma unroll
+        for (int q = 0; q < NS; q++) {
+          red[warp][0][NS * lane + q] = S[q];
+          red[warp][1][NS * lane + q] = C[q];
+        }
+        __syncthreads();
+        for (int p = threadIdx.x; p < TS; p += kPairsThreads)
+          finish(p, red[0][0][p], red[0][1][p]);
+        __syncthreads();
       }
     }
-    __syncthreads();
-  }
+  };
+  if (a.share == 1) fold_units(std::integral_constant<int, 1>());
+  else fold_units(std::integral_constant<int, NW>());
 }
 
 template <class R> size_t pairs_smem(bool ang) {
@@ -621,7 +664,7 @@ cudaError_t mdot_pairs_plan(int N, int nper, bool wall, bool ang, int num_sms, i
   if (e != cudaSuccess) return e;
   const long long tpb = (nper + kPairsTile<R> - 1) / kPairsTile<R>;
   const long long steps = 16 * tpb * (tpb + 1) * (N / nper);
-  if (steps < kPairsFewSteps * per_sm * num_sms * (kPairsThreads / 32)) per_sm = std::min(per_sm, 2);
+  if (steps < pairs_few_steps(ang, tpb) * per_sm * num_sms * (kPairsThreads / 32)) per_sm = std::min(per_sm, 2);
   mdot_pairs_plan_tables<R>(N, nper, ang, (long long)per_sm * num_sms, force_warps, max_part, p);
   p.wall = wall;
   return cudaSuccess;
@@ -663,6 +706,21 @@ cudaError_t mdot_pairs_launch(const PairsPlan &p, const int *cuts, const R *pos,
                reinterpret_cast<uintptr_t>(T)) & 7) == 0;
     a.bar = bar + q;
     a.err = err;
+    // Folding: rounds of loads one after the other (16 partials a warp, about
+    // as much again to start and finish a component of a tile) with four warps
+    // on each, or one.  64 batches of 333 (10 partials a tile): 24.0 us with
+    // four, 17.9 with one, wall with torques 63.7 and 51.2.  With many partials
+    // four are as good or better (N = 16384 wall forces, 272 a tile: 326.9
+    // and 328.5 us).
+    {
+      const long long NW = kPairsThreads / 32, nc = p.ang ? 6 : 3;
+      const long long tiles = ((s.row1 - 1) / p.tpb + 1 - s.row0 / p.tpb) * (long long)p.tpb;
+      const long long n = p.tpb + 1 + 2LL * s.warps / tiles, units = tiles * nc;
+      auto up = [](long long x, long long y) { return (x + y - 1) / y; };
+      const long long four = up(units, s.grid) * (up(n, 16 * NW) + 1);
+      const long long one = up(units, NW * s.grid) * (up(n, 16) + 1);
+      a.share = n <= 64 && one < four ? 1 : (int)NW;
+    }
     void *params[] = {(void *)&a};
     count_launch();
     const cudaError_t e =
