@@ -2,6 +2,7 @@
 // and launch.  The scheme is described in mdot_sym.cuh.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "bounds.cuh"
 #include "grid_sync.cuh"
@@ -471,79 +472,108 @@ __global__ void __launch_bounds__(kSymThreads, MINB) mdot_sym_kernel(const SymAr
     a.trace[2 * (size_t)gridDim.x * (kSymThreads / 32) + 2 * gridDim.x + blockIdx.x] = smid;
   }
   // kFoldH pairs of adjacent output elements per thread and pass, sixteen
-  // float2 loads of each in flight: a warp's lanes read 8 consecutive elements
-  // of each of rt slots (whole 32-byte sectors); at N = 4096 one pass covers
-  // every element
+  // float2 loads of each in flight; at N = 4096 one pass covers every element.
+  // The slots of an element are summed in rt shares (share u: u, u + rt, ...),
+  // which meet in an xor tree, bit 0 first.  At most 8 lanes take the shares of
+  // an element, in turn where there are more, so that a warp always reads 8
+  // consecutive elements (a whole 32-byte sector) of a slot: with 16 lanes half
+  // of every sector was read in vain and the fold of N = 16384 took 18 us.
   const int rt = 1 << a.lg_rt;
+  const int lg_lanes = min(a.lg_rt, 3), lanes = 1 << lg_lanes, turns = rt >> lg_lanes;
   constexpr int kPairs = kElems / 2;
-  const unsigned total = (unsigned)a.ntiles * kPairs * rt;
+  const unsigned total = (unsigned)a.ntiles * kPairs * lanes;
   const unsigned stride = gridDim.x * blockDim.x;
-  for (unsigned base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total;
-       base += kFoldH * stride) {
-    float S[kFoldH][2], C[kFoldH][2];
-    int t[kFoldH], e[kFoldH], sub[kFoldH], cnt[kFoldH];
-    bool in[kFoldH];
-    const float2 *src[kFoldH];
-    int cmx = 0;
+  // (S, C) += (S2, C2); the same bits for either order of the operands
+  auto merge = [](float &S, float &C, float S2, float C2) {
+    const float sm = S + S2;
+    const float bp = sm - S;
+    const float err = (S - (sm - bp)) + (S2 - bp);  // exact, symmetric in (S, S2)
+    C = (C + C2) + err;
+    S = sm;
+  };
+  // (two copies of the code: one turn, in a small system, is mostly the time to
+  // fetch it)
+  auto fold_all = [&](auto one) {
+    constexpr bool single = decltype(one)::value;
+    for (unsigned base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total;
+         base += kFoldH * stride) {
+      float S[kFoldH][2], C[kFoldH][2];
+      int t[kFoldH], e[kFoldH], sub[kFoldH], cnt[kFoldH];
+      bool in[kFoldH];
+      const float2 *src[kFoldH];
+      int cmx = 0;
 #pragma unroll
-    for (int h = 0; h < kFoldH; h++) {
-      S[h][0] = S[h][1] = C[h][0] = C[h][1] = 0.f;
-      const unsigned g = base + h * stride + lane;
-      in[h] = g < total;
-      const unsigned el = in[h] ? g >> a.lg_rt : 0u;  // pair of elements (2 el, 2 el + 1)
-      sub[h] = (int)(g & (unsigned)(rt - 1));
-      t[h] = (int)(el / kPairs);
-      e[h] = 2 * (int)(el - (unsigned)t[h] * kPairs);
-      src[h] = reinterpret_cast<const float2 *>(a.part + (size_t)t[h] * a.cmax * kElems + e[h]);
-      cnt[h] = in[h] ? a.cmax : 0;
-      cmx = max(cmx, cnt[h]);
-    }
-    // each tile's slot range, in slot order (share `sub` of every rt)
-    for (int m0 = 0; m0 < cmx; m0 += 16 * rt) {
-      float2 v[kFoldH][16];
+      for (int h = 0; h < kFoldH; h++) {
+        const unsigned g = base + h * stride + lane;
+        in[h] = g < total;
+        const unsigned el = in[h] ? g >> lg_lanes : 0u;  // pair of elements (2 el, 2 el + 1)
+        sub[h] = (int)(g & (unsigned)(lanes - 1));
+        t[h] = (int)(el / kPairs);
+        e[h] = 2 * (int)(el - (unsigned)t[h] * kPairs);
+        src[h] = reinterpret_cast<const float2 *>(a.part + (size_t)t[h] * a.cmax * kElems + e[h]);
+        cnt[h] = in[h] ? a.cmax : 0;
+        cmx = max(cmx, cnt[h]);
+      }
+      float S1[kFoldH][2], C1[kFoldH][2], S2[kFoldH][2], C2[kFoldH][2];  // of earlier turns
+      for (int turn = 0; turn < (single ? 1 : turns); turn++) {
 #pragma unroll
-      for (int h = 0; h < kFoldH; h++)
+        for (int h = 0; h < kFoldH; h++) S[h][0] = S[h][1] = C[h][0] = C[h][1] = 0.f;
+        // each tile's slot range, in slot order (every rt-th from the share's)
+        for (int m0 = turn * lanes; m0 < cmx; m0 += 16 * rt) {
+          float2 v[kFoldH][16];
 #pragma unroll
-        for (int m = 0; m < 16; m++) {
-          const int j = m0 + sub[h] + m * rt;
-          v[h][m] = (j < cnt[h] &&
-                     LMG_IN_BOUNDS(((size_t)t[h] * a.cmax + j + 1) * kElems <= a.part_elems, 13,
-                                   t[h]))
-                        ? __ldcg(src[h] + (size_t)j * kPairs) : make_float2(0.f, 0.f);
+          for (int h = 0; h < kFoldH; h++)
+#pragma unroll
+            for (int m = 0; m < 16; m++) {
+              const int j = m0 + sub[h] + m * rt;
+              v[h][m] = (j < cnt[h] &&
+                         LMG_IN_BOUNDS(((size_t)t[h] * a.cmax + j + 1) * kElems <= a.part_elems, 13,
+                                       t[h]))
+                            ? __ldcg(src[h] + (size_t)j * kPairs) : make_float2(0.f, 0.f);
+            }
+#pragma unroll
+          for (int h = 0; h < kFoldH; h++)
+#pragma unroll
+            for (int m = 0; m < 16; m++) {
+              fold(S[h][0], C[h][0], v[h][m].x);
+              fold(S[h][1], C[h][1], v[h][m].y);
+            }
         }
 #pragma unroll
-      for (int h = 0; h < kFoldH; h++)
+        for (int h = 0; h < kFoldH; h++) {
 #pragma unroll
-        for (int m = 0; m < 16; m++) {
-          fold(S[h][0], C[h][0], v[h][m].x);
-          fold(S[h][1], C[h][1], v[h][m].y);
-        }
-    }
-#pragma unroll
-    for (int h = 0; h < kFoldH; h++) {
-#pragma unroll
-      for (int c = 0; c < 2; c++) {
-        // combine the rt shares (the same value lands in every lane of a group)
-        for (int o = 1; o < rt; o <<= 1) {
-          const float S2 = __shfl_xor_sync(0xffffffffu, S[h][c], o);
-          const float C2 = __shfl_xor_sync(0xffffffffu, C[h][c], o);
-          const float sm = S[h][c] + S2;
-          const float bp = sm - S[h][c];
-          const float err = (S[h][c] - (sm - bp)) + (S2 - bp);  // exact, symmetric in (S, S2)
-          C[h][c] = (C[h][c] + C2) + err;
-          S[h][c] = sm;
+          for (int c = 0; c < 2; c++) {
+            // the lanes' shares (the same value lands in every lane of a group)
+            for (int o = 1; o < lanes; o <<= 1) {
+              const float So = __shfl_xor_sync(0xffffffffu, S[h][c], o);
+              const float Co = __shfl_xor_sync(0xffffffffu, C[h][c], o);
+              merge(S[h][c], C[h][c], So, Co);
+            }
+            // and the turns': 0 and 1, 2 and 3, then those two (rt <= 32: four)
+            if (single) continue;
+            if (turn & 1) merge(S[h][c], C[h][c], S1[h][c], C1[h][c]);
+            if (turn == 3) merge(S[h][c], C[h][c], S2[h][c], C2[h][c]);
+            if (turn == 1) S2[h][c] = S[h][c], C2[h][c] = C[h][c];
+            S1[h][c] = S[h][c];
+            C1[h][c] = C[h][c];
+          }
         }
       }
-      if (in[h] && sub[h] == 0) {
-        const int2 td = tile_desc(a, t[h]);
 #pragma unroll
-        for (int c = 0; c < 2; c++)
-          if (e[h] + c < 3 * td.y &&
-              LMG_IN_BOUNDS(3 * (size_t)td.x + e[h] + c < 3 * (size_t)a.N, 14, td.x))
-            a.U[3 * (size_t)td.x + e[h] + c] = S[h][c] + C[h][c];
+      for (int h = 0; h < kFoldH; h++) {
+        if (in[h] && sub[h] == 0) {
+          const int2 td = tile_desc(a, t[h]);
+#pragma unroll
+          for (int c = 0; c < 2; c++)
+            if (e[h] + c < 3 * td.y &&
+                LMG_IN_BOUNDS(3 * (size_t)td.x + e[h] + c < 3 * (size_t)a.N, 14, td.x))
+              a.U[3 * (size_t)td.x + e[h] + c] = S[h][c] + C[h][c];
+        }
       }
     }
-  }
+  };
+  if (turns == 1) fold_all(std::true_type());
+  else fold_all(std::false_type());
   if (a.trace) {
     __syncthreads();
     if (threadIdx.x == 0) a.trace[tb + 1] = global_ns();

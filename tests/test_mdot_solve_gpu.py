@@ -51,3 +51,19 @@ def test_matches_oracle(tiled, oracle, precision, wall, N, nper, dense):
         assert rel_err(U, Uo) <= TOL[precision], ang
         if ang:
             assert rel_err(W, Wo) <= TOL[precision]
+
+
+@pytest.mark.parametrize("N", [5000, 16384, 33001, 70000])
+def test_symmetric_fold(cuda, N):
+    """The symmetric product's fold with 8, 16 and 32 shares an element (one, two
+    and four turns of 8 lanes) and more slots than one pass over them, against
+    the FP64 product of the same (single precision) inputs."""
+    rng = np.random.default_rng(N)
+    p = rng.uniform(0, (N * 4 * np.pi / 3 / 0.1) ** (1 / 3), (N, 3)).astype(np.float32)
+    F = rng.normal(size=(N, 3)).astype(np.float32)
+    out = {}
+    for precision, dtype in (("float", np.float32), ("double", np.float64)):
+        s = make_solver(0, 0, 1.0, 1.0, precision, N, N)
+        s.setPositions(p.astype(dtype))
+        out[precision] = s.Mdot(F.astype(dtype))[0]
+    assert rel_err(out["float"], out["double"]) <= TOL["float"]
