@@ -141,9 +141,10 @@ __global__ void knn_scatter_kernel(const float *__restrict__ pos, int N, const i
 // N = 4000 (K = 48), 0.81 and 0.32 with a warp.
 constexpr int kSearchWarps = 8, kSearchCap = 256;
 
-// Cuts the warp's list (keys in any order, count >= KB) to KB entries with the
-// smallest keys; lo: fewer than KB keys are <= lo.  Returns a key below which
-// later candidates have to lie to matter.
+// Cuts the warp's list (keys in any order, count >= KB) to the KB entries with
+// the smallest keys and those that tie with the last, as far as they leave room
+// for a batch; lo: fewer than KB keys are <= lo.  Returns the largest key that
+// still matters.
 template <int KB>
 __device__ __forceinline__ unsigned knn_cut(unsigned *key, int *slot, int &count, unsigned lo) {
   const int lane = threadIdx.x & 31;
@@ -163,10 +164,15 @@ __device__ __forceinline__ unsigned knn_cut(unsigned *key, int *slot, int &count
       if (c == KB) break;
     }
   }
-  // all below hi, and of those equal to it as many as there is room for
-  int below = 0;
-  for (int k = lane; k < count; k += 32) below += key[k] < hi;
-  int room = KB - __reduce_add_sync(0xffffffffu, below);
+  // all below hi, and those equal to it
+  int below = 0, level = 0;
+  for (int k = lane; k < count; k += 32) {
+    below += key[k] < hi;
+    level += key[k] == hi;
+  }
+  below = __reduce_add_sync(0xffffffffu, below);
+  level = __reduce_add_sync(0xffffffffu, level);
+  int room = below + level <= kSearchCap - 32 ? level : KB - below;
   int out = 0;
   for (int k0 = 0; k0 < count; k0 += 32) {
     const int k = k0 + lane;
@@ -211,7 +217,7 @@ knn_search_kernel(int N, KnnGridShape g, const int *__restrict__ start,
   const int base = (i / g.nper) * g.cells;
   int count = 0;
   // a distance's bits + 1; the particle itself goes first, with 0
-  unsigned worst = __float_as_uint(FLT_MAX) + 1u;
+  unsigned worst = __float_as_uint(FLT_MAX);  // the largest finite distance but one
   const int smax = max(g.nx, max(g.ny, g.nz));
   for (int s = 1; s <= smax; s++) {
     // runs of cells: the columns on the shell's four sides (s = 1: all nine,
@@ -274,9 +280,9 @@ knn_search_kernel(int N, KnnGridShape g, const int *__restrict__ start,
           const float4 p = spos[q];
           const float dx = p.x - pi.x, dy = p.y - pi.y, dz = p.z - pi.z;
           kq = __float_as_uint(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) + 1u;
-          if (q == t0 && kq < worst) kq = 0u;
+          if (q == t0 && kq <= worst) kq = 0u;
         }
-        const bool add = kq < worst;
+        const bool add = kq <= worst;
         const unsigned in = __ballot_sync(0xffffffffu, add);
         if (add) {
           const int o = count + __popc(in & ((1u << lane) - 1u));
@@ -301,18 +307,36 @@ knn_search_kernel(int N, KnnGridShape g, const int *__restrict__ start,
   }
   if (count > KB) knn_cut<KB>(key, slot, count, 0u);
   __syncwarp();
-  for (int k = lane; k < KB; k += 32) {
+  // equal distances: shell by shell, in the order of the cells, then as stored
+  auto before = [&](int qa, int qb) {
+    int o[2][4];
+    const int q[2] = {qa, qb};
+#pragma unroll 1
+    for (int h = 0; h < 2; h++) {
+      const float4 p = spos[q[h]];
+      o[h][1] = cell_coord(p.x, g.x0, g.inv_h, g.nx) - ix;
+      o[h][2] = cell_coord(p.y, g.y0, g.inv_h, g.ny) - iy;
+      o[h][3] = cell_coord(p.z, g.z0, g.inv_h, g.nz) - iz;
+      o[h][0] = max(abs(o[h][1]), max(abs(o[h][2]), abs(o[h][3])));
+    }
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+      if (o[0][c] != o[1][c]) return o[0][c] < o[1][c];
+    return qa < qb;
+  };
+  for (int k = lane; k < max(KB, count); k += 32) {
     int rank = k, j = i;  // fewer than KB found: the particle itself
     if (k < count) {
       const unsigned v = key[k];
+      const int q = slot[k];
       rank = 0;
       for (int l = 0; l < count; l++) {
         const unsigned u = key[l];
-        rank += u < v || (u == v && l < k);
+        rank += u < v || (u == v && l != k && before(slot[l], q));
       }
-      j = sidx[slot[k]];
+      j = sidx[q];
     }
-    nb[(size_t)rank * N + i] = j;
+    if (rank < KB) nb[(size_t)rank * N + i] = j;
   }
 }
 

@@ -54,3 +54,36 @@ def test_nearest_neighbours(cuda, system, K):
         ref = np.sort(((q[b:b + nper] - q[i]) ** 2).sum(1))[:K + 1]
         d = ((q[got[i]] - q[i]) ** 2).sum(1)
         assert np.allclose(d, ref, rtol=1e-6, atol=0), i
+
+
+def test_order_of_equal_distances(cuda):
+    """On a perfect lattice most distances tie: equal ones come shell by shell of
+    the search grid (Chebyshev distance in cells), in the order of the cells'
+    coordinates.  The preconditioner's network takes them in this order.  Cells
+    are half the expected distance of the 16th neighbour wide, here less than
+    the lattice constant, so that no two particles share one."""
+    import torch
+    from libmobility_gb300 import _capi
+    lib = _capi.load()
+    K, m = 16, 11
+    rng = np.random.default_rng(3)
+    p = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3) * 2.5
+    p = p[rng.permutation(m ** 3)].astype(np.float32)
+    N = len(p)
+    dp = torch.tensor(p, device="cuda")
+    nb = torch.empty((K + 1, N), dtype=torch.int32, device="cuda")
+    assert lib.lmg_internal_knn_k(K, ctypes.c_void_p(dp.data_ptr()), N, N,
+                                  ctypes.c_void_p(nb.data_ptr()), None) == 0
+    torch.cuda.synchronize()
+    got = nb.cpu().numpy().T
+    extent = np.float64(2.5 * (m - 1))
+    h = 0.5 * np.cbrt(3 * (K + 1) / (4 * np.pi * N / extent ** 3))
+    assert h < 2.5 and np.ceil(extent / h) ** 3 <= 8 * N + 64
+    n = int(np.ceil(extent / h))
+    cell = np.minimum((p * np.float32(1 / h)).astype(int), n - 1)
+    for i in range(N):
+        d2 = ((p - p[i]).astype(np.float64) ** 2).sum(1)
+        d2[i] = -1
+        o = cell - cell[i]
+        order = np.lexsort((o[:, 2], o[:, 1], o[:, 0], np.abs(o).max(1), d2))
+        assert np.array_equal(got[i], order[:K + 1]), i
