@@ -67,3 +67,25 @@ def test_symmetric_fold(cuda, N):
         s.setPositions(p.astype(dtype))
         out[precision] = s.Mdot(F.astype(dtype))[0]
     assert rel_err(out["float"], out["double"]) <= TOL["float"]
+
+
+@pytest.mark.parametrize("power", [60, 100])
+@pytest.mark.parametrize("N", [200, 3000])
+def test_large_noise(cuda, N, power):
+    """The convergence check sums FP32 squares at a scale of its own, so noise whose
+    squares are out of range stops at the same iteration, and the result is that
+    of ordinary noise times the same power of two, bit for bit.  (Not for small
+    noise: the recurrence takes beta < 1e-3 alpha / |z| for a breakdown, as the
+    reference does, LanczosAlgorithm.cu:144, and ends early below |z| of about
+    0.01.)"""
+    rng = np.random.default_rng(N)
+    p = rng.uniform(0, (N * 4 * np.pi / 3 / 0.1) ** (1 / 3), (N, 3)).astype(np.float32)
+    z = rng.normal(size=(N, 3)).astype(np.float32)
+    out = []
+    for scale in (0, power):
+        s = make_solver(0, 0, 1.0, 1.0, "float", N, N)
+        s.setPositions(p)
+        y, _, iterations, _ = s.sqrtMdotW_noise(np.ldexp(z, scale).astype(np.float32))
+        out.append((np.asarray(y), iterations))
+    assert out[0][1] == out[1][1]
+    assert np.array_equal(np.ldexp(out[0][0], power).astype(np.float32), out[1][0])
