@@ -374,10 +374,21 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
 #pragma unroll
       for (int q = 0; q < NS; q++) ui[q] = {zero, zero, zero, zero, zero, zero};
     }
-    // exact - fast for the close pairs, in step order
-    for (unsigned st = __reduce_or_sync(0xffffffffu, near); st != 0u; st &= st - 1u) {
-      const int k = __ffs(st) - 1;
-      if ((near >> k) & 1u) {
+    // exact - fast for the close pairs: usually no two flagged steps share a slot,
+    // and each lane takes its own in turn, all side by side; else step by step.
+    // Either way every sum gets its corrections in step order.  (Always step by
+    // step: 500 batches of 60 13.3 us, 11.8 side by side; N = 200 in FP64 17.7,
+    // 16.0.)
+    unsigned st = __reduce_or_sync(0xffffffffu, near);
+    const unsigned slots = __funnelshift_l(near, near, lane);
+    const bool apart =
+        st == 0u || diag ||
+        (int)__reduce_add_sync(0xffffffffu, (unsigned)__popc(near)) ==
+            __popc(__reduce_or_sync(0xffffffffu, slots));
+    while (st != 0u) {
+      const unsigned from = apart ? near : st;
+      const int k = __ffs(from) - 1;
+      if (from != 0u && ((near >> k) & 1u)) {
         const int s = (lane + k) & 31;
         // which of the slots' pairs (NS q + h); FP32 takes the distances of all
         // four first, which spares most of the loads below
@@ -422,8 +433,15 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
           }
         }
       }
-      __syncwarp();
+      if (apart) {
+        near &= near - 1u;
+        st = __any_sync(0xffffffffu, near != 0u) ? 1u : 0u;
+      } else {
+        st &= st - 1u;
+        __syncwarp();
+      }
     }
+    __syncwarp();
     if (!diag) put(cur.k == 0 ? (size_t)cur.p : slot_cut + gw, w.A);
     if (flush) {
       if (sizeof(R) == 4) {

@@ -406,14 +406,31 @@ __global__ void __launch_bounds__(kSymThreads, MINB) mdot_sym_kernel(const SymAr
         if (rotation_step(a, I, ui, J4, A4, (lane + k) & 31)) near |= 1u << (k - k0);
         __syncwarp();
       }
-      // the flagged steps of any lane, in step order (at one step the lanes'
-      // slots are all different)
-      for (unsigned steps = __reduce_or_sync(0xffffffffu, near); steps != 0u;
-           steps &= steps - 1u) {
-        const int kk = __ffs(steps) - 1;
-        if ((near >> kk) & 1u) {
-          const int kabs = k0 + kk;
-          correct_step(a, I, ui, J4, A4, (lane + (diag && kabs == 0 ? 16 : kabs)) & 31);
+      // The flagged steps.  Usually no two of them share a slot, and each lane
+      // then takes its own in turn, all lanes side by side; else step by step
+      // (at one step the lanes' slots are all different).  Either way every sum
+      // gets its corrections in step order.  (Always step by step: N = 2000 at
+      // volume fraction 0.05 10.6 us, 10.0 side by side; N = 4096 19.1, 18.9.)
+      if (unsigned steps = __reduce_or_sync(0xffffffffu, near)) {
+        unsigned at = near << k0;  // by distance; 16 for the first of a diagonal tile
+        if (diag && (at & 1u)) at ^= 0x10001u;
+        const unsigned slots = __funnelshift_l(at, at, lane);
+        const bool apart = (int)__reduce_add_sync(0xffffffffu, (unsigned)__popc(slots)) ==
+                           __popc(__reduce_or_sync(0xffffffffu, slots));
+        while (steps != 0u) {
+          const unsigned from = apart ? near : steps;
+          const int kk = __ffs(from) - 1;
+          if (from != 0u && ((near >> kk) & 1u)) {
+            const int kabs = k0 + kk;
+            correct_step(a, I, ui, J4, A4, (lane + (diag && kabs == 0 ? 16 : kabs)) & 31);
+          }
+          if (apart) {
+            near &= near - 1u;
+            steps = __any_sync(0xffffffffu, near != 0u) ? 1u : 0u;
+          } else {
+            steps &= steps - 1u;
+            __syncwarp();
+          }
         }
         __syncwarp();
       }
