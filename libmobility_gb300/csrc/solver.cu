@@ -585,6 +585,18 @@ bool Solver<R>::mdot_pairs(const R *pos, const R *F, const R *T, R *U, R *W) {
   const int warps = g_sym_warps.load();
   const auto key = std::make_tuple(N, batch_size(), (int)ang_, warps);
   auto it = pairs_plans_.find(key);
+  // nothing can be allocated while the stream is captured: a first call then
+  // takes mdot_kernel, which needs no scratch for the smallest systems
+  if (it == pairs_plans_.end() || (it->second->plan.ok &&
+                                   (pairs_part_.count < it->second->plan.part_elems ||
+                                    pairs_acc_.count < it->second->plan.acc_elems))) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream(), &capture) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return false;
+    }
+    if (capture != cudaStreamCaptureStatusNone) return false;
+  }
   if (it == pairs_plans_.end()) {
     auto st = std::make_unique<PairsState>();
     LMG_CUDA(mdot_pairs_plan<R>(N, batch_size(), wall_, ang_, sms(), warps,
@@ -601,8 +613,14 @@ bool Solver<R>::mdot_pairs(const R *pos, const R *F, const R *T, R *U, R *W) {
   const PairsState &st = *it->second;
   if (!st.plan.ok) return false;
   check_barriers();
-  pairs_part_.ensure(st.plan.part_elems);
-  if (st.plan.acc_elems) pairs_acc_.ensure(st.plan.acc_elems);
+  try {
+    pairs_part_.ensure(st.plan.part_elems);
+    if (st.plan.acc_elems) pairs_acc_.ensure(st.plan.acc_elems);
+  } catch (const Error &) {  // no memory left for the partial sums (at most 1 GiB)
+    (void)cudaGetLastError();
+    pairs_part_.release();
+    return false;
+  }
   unsigned long long *bars = st.bars_and_cuts.ptr;
   LMG_CUDA(mdot_pairs_launch<R>(st.plan,
                                 reinterpret_cast<const int *>(bars + st.plan.passes.size()), pos,

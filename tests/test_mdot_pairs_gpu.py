@@ -57,3 +57,33 @@ def test_matches_oracle(lib, oracle, precision, wall, N, nper, warps, part):
         if ang:
             assert rel_err(W, Wo) <= TOL[precision], (f is None, t is None)
             assert np.array_equal(W, W2)
+
+
+@pytest.mark.parametrize("precision", ["float", "double"])
+@pytest.mark.parametrize("N,warm", [(100, False), (100, True), (3000, True)])
+def test_captured(lib, precision, N, warm):
+    """Mdot in a CUDA graph: after a first call, and for a small system without one
+    (nothing can be allocated then: another kernel that needs no scratch)."""
+    import torch
+    rng = np.random.default_rng(N)
+    dt = torch.float32 if precision == "float" else torch.float64
+    p = rng.uniform(0, (N * 4 * np.pi / 3 / 0.15) ** (1 / 3), (N, 3)) + 0.5
+    p, F, T = (torch.tensor(x, dtype=dt, device="cuda")
+               for x in (p, rng.normal(size=(N, 3)), rng.normal(size=(N, 3))))
+    s = make_solver(1, 1, 1.0, 1.0, precision, N, N)
+    s.setPositions(p)
+    if warm:
+        s.Mdot(F, T)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        U, W = s.Mdot(F, T)
+    F2 = F.clone()
+    F.copy_(T)  # read at replay
+    g.replay()
+    torch.cuda.synchronize()
+    got = U.cpu().numpy(), W.cpu().numpy()
+    U, W = s.Mdot(T, T)
+    assert rel_err(got[0], U.cpu().numpy()) <= TOL[precision]
+    assert rel_err(got[1], W.cpu().numpy()) <= TOL[precision]
+    F.copy_(F2)
