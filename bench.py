@@ -43,6 +43,11 @@ METRIC = ("sqrtMdotW solves/s at 1e-6 residual (learned-precond vs plain); "
 # rsqrt/rcp/div/sqrt = 1): open UF 36, open 6x6 89, wall UF 160, wall 6x6 380
 FLOPS_PER_PAIR = {("open", False): 36, ("open", True): 89, ("wall", False): 160,
                   ("wall", True): 380}
+# Mdot takes each unordered pair once: the coefficients and both particles' velocities
+# are 53, 153, 130 and 270 flops, counted here per ordered pair.  (The products inside
+# a solve above a wall or with torques are over ordered pairs, with the figures above.)
+MDOT_FLOPS_PER_PAIR = {("open", False): 26.5, ("open", True): 76.5, ("wall", False): 65,
+                       ("wall", True): 135}
 WORKLOADS = {
     "wall16k": dict(N=16384, wall=True, ang=True, tol=1e-6,
                     desc="single-wall RPY, N=16384, forces+torques, includeAngular, "
@@ -56,10 +61,10 @@ WORKLOADS = {
 }
 
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the Mdot kernel
-# from one ncu capture of each workload (profiles/mdot_kernel_*.md); the
+# from one ncu capture (profiles/mdot_pairs_kernel_wall6x6_N16384.md); the
 # kernel reads its inputs once (positions, forces, torques) and writes the
-# split partials, which stay in L2
-MDOT_TRAFFIC = {"wall16k": 633.3e3, "open16k": 417.8e3}
+# partial sums, which stay in L2
+MDOT_TRAFFIC = {"wall16k": 3.64e6}
 
 
 def make_inputs(w, seed):
@@ -286,7 +291,7 @@ def open4k_mdot(torch, lib, peak32, peak64, flush):
     pairs = float(N) * N
     out = {"workload": "open RPY (UF), N=4096, cube at phi=0.05, a=1, viscosity 1/(6 pi), "
                        "F ~ N(0,1), seed 1234",
-           "pairs": pairs, "flops_per_pair": FLOPS_PER_PAIR[("open", False)]}
+           "pairs": pairs, "flops_per_pair": MDOT_FLOPS_PER_PAIR[("open", False)]}
     results = {}
     for prec, dt, peak in (("float", torch.float32, peak32), ("double", torch.float64, peak64)):
         s = NBody("open", "open", "open", precision=prec)
@@ -317,7 +322,7 @@ def open4k_mdot(torch, lib, peak32, peak64, flush):
             e["tiled_kernel_ms"] = t_tiled * 1e3
             e["speedup_vs_tiled_kernel"] = t_tiled / t
         else:
-            e["kernel"] = "mdot_kernel<double>"
+            e["kernel"] = "mdot_pairs_kernel<double> (each unordered pair once)"
         out[prec] = e
     return out, pos, F, results
 
@@ -741,7 +746,7 @@ def large_wall_mdot(torch, rank, reps=3):
     return {"workload": "single wall, N=262144, x,y ~ U[0,1024), z ~ U[1.5,40], forces + "
                         "torques, includeAngular, FP32",
             "mdot_ms": t * 1e3, "mdot_pair_interactions_per_s": pairs / t,
-            "achieved_tflops": pairs * FLOPS_PER_PAIR[("wall", True)] / t / 1e12}
+            "achieved_tflops": pairs * MDOT_FLOPS_PER_PAIR[("wall", True)] / t / 1e12}
 
 
 def large_wall_sqrt(torch, rank):
@@ -790,7 +795,7 @@ def hbm_peak_gbs():
         return None
 
 
-def krylov_phases(torch, s, ddW, t_mdot, solves=3):
+def krylov_phases(torch, s, ddW, solves=3):
     """Device time of the Lanczos work outside the matvec on the main
     workload: the vector updates after each matvec (alpha, beta, next basis
     vector: 4 n s algorithmic bytes per iteration) and the convergence checks
@@ -821,9 +826,8 @@ def krylov_phases(torch, s, ddW, t_mdot, solves=3):
         "hbm_peak_gbs": peak, "peak_source": "MEASURED_PEAKS.json hbm_gbs (copy)",
         "vector_update_frac": vec_gbs / peak if peak else None,
         "check_frac": chk_gbs / peak if peak else None,
-        "matvec_us": t_mdot * 1e6,
-        "vector_share_of_iteration": (t["vector_ms"] / t["iterations"])
-        / (t["vector_ms"] / t["iterations"] + t_mdot * 1e3),
+        "matvec_us": 1e3 * t["operator_ms"] / t["iterations"],
+        "vector_share_of_iteration": t["vector_ms"] / (t["vector_ms"] + t["operator_ms"]),
         "note": "checks run on a high-priority side stream, overlapping the next matvec",
     }
 
@@ -963,7 +967,7 @@ def run_ours(args, w, ws, rank, local):
         s.sqrtMdotW_noise(ddW)
     torch.cuda.synchronize()
     t_sqrt = (time.perf_counter() - t0) / 3
-    krylov = krylov_phases(torch, s, ddW, t_mdot)
+    krylov = krylov_phases(torch, s, ddW)
     peak = fp32_peak_tflops(lib, torch)
     peak64 = fp64_peak_tflops(lib, torch)
     open4k, pos1, F1, res1 = open4k_mdot(torch, lib, peak, peak64, flush)
@@ -971,7 +975,7 @@ def run_ours(args, w, ws, rank, local):
     ref_gpu = None
     if not args.skip_reference_gpu:
         ref_gpu = reference_gpu_mdot(torch, (pos, F, T, dW))
-    fpp = FLOPS_PER_PAIR[("wall" if w["wall"] else "open", w["ang"])]
+    fpp = MDOT_FLOPS_PER_PAIR[("wall" if w["wall"] else "open", w["ang"])]
     achieved = pairs * fpp / t_mdot / 1e12
 
     # --- e2e through the public API with host buffers ---
@@ -1049,7 +1053,8 @@ def run_ours(args, w, ws, rank, local):
         "mdot_pair_interactions_per_s": pairs / t_mdot,
         "e2e": {"value": e2e_value, "unit": "pair-interactions/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "ms_per_step": t_e2e * 1e3},
-        "roofline": {"bound": "fp32", "kernel": "mdot_kernel (pair interactions)",
+        "roofline": {"bound": "fp32", "kernel": "Mdot (mdot_pairs_kernel, or mdot_sym_kernel for open "
+                                               "forces): pair interactions",
                      "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak, "traffic": MDOT_TRAFFIC.get(args.workload),
                      "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of one "
