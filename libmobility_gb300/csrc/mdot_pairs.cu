@@ -62,6 +62,7 @@ template <class R> struct PairsArgs {
   const R *pos, *F, *T;
   R *U, *W;
   int N, nper, tpb;   // tpb: tiles per batch
+  int slots;          // of a tile in use
   int row0, row1;
   int tiles;          // tiles of all batches
   unsigned steps, per_warp;
@@ -103,10 +104,11 @@ __device__ __forceinline__ void copies_done() {
 // at particle b0) to raw[positions, F, T][3 * particle + component]; only that
 // lane reads them back (scale_slot).
 template <class R, bool ANG, int NA, int TE>
-__device__ __forceinline__ void fetch_slot(const PairsArgs<R> &a, int b0, int t, int lane,
+__device__ __forceinline__ void fetch_slot(const PairsArgs<R> &a, int S, int b0, int t, int lane,
                                            R (&raw)[NA][TE]) {
-  constexpr int NS = kPairsSlot<R>, TS = kPairsTile<R>;
-  const int l = t * TS + NS * lane;
+  constexpr int NS = kPairsSlot<R>;
+  const int l = NS * (t * S + lane);
+  if (lane >= S) return;
   const size_t g = 3 * (size_t)(b0 + l);
   const R *src[3] = {a.pos + g, a.F + g, a.T + g};
   const bool use[3] = {true, a.F != nullptr, ANG && a.T != nullptr};
@@ -133,7 +135,7 @@ __device__ __forceinline__ void fetch_slot(const PairsArgs<R> &a, int b0, int t,
 
 // The lane's particles, scaled: out = x, y, z, F, T.
 template <class R, bool WALL, bool ANG, int NA, int TE, int NV, int TS>
-__device__ __forceinline__ void scale_slot(const PairsArgs<R> &a, int t, int lane,
+__device__ __forceinline__ void scale_slot(const PairsArgs<R> &a, int S, int t, int lane,
                                            const R (&raw)[NA][TE], R (&out)[NV][TS]) {
   constexpr int NS = kPairsSlot<R>;
   using L = typename LaneTypes<R>::L;
@@ -150,7 +152,7 @@ __device__ __forceinline__ void scale_slot(const PairsArgs<R> &a, int t, int lan
   }
 #pragma unroll
   for (int q = 0; q < NS; q++) {
-    const bool in = t * TS + NS * lane + q < a.nper;
+    const bool in = lane < S && NS * (t * S + lane) + q < a.nper;
     // no contraction with the differences: a particle meets itself at d = 0
     v[q][0] = in ? mul_rn(r[0][3 * q], a.inv_a) : R(kPadX) + R(4 * (NS * lane + q));
     v[q][1] = in ? mul_rn(r[0][3 * q + 1], a.inv_a) : R(0);
@@ -216,7 +218,8 @@ struct Segment {
   bool new_row, new_tile;  // the row begins here; tile I is not the last segment's
 };
 
-template <class R, bool WALL, bool ANG>
+// FULL: all 32 slots of a tile are in use.
+template <class R, bool WALL, bool ANG, bool FULL>
 __global__ void __launch_bounds__(kPairsThreads, (pairs_min_blocks<R, WALL, ANG>()))
 mdot_pairs_kernel(const PairsArgs<R> a) {
   using V = typename LaneTypes<R>::V;
@@ -231,6 +234,7 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gw = blockIdx.x * NW + warp;
   Warp &w = sm[warp];
+  const int nsl = FULL ? 32 : a.slots;
 
   const int ppb = a.tpb * (a.tpb + 1) / 2;
   const int P0 = (int)pairs_before(a.tpb, a.row0);
@@ -257,9 +261,9 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
   cur.left = 0;
   if (gw < a.warps) {
     cur.left = (int)min(a.per_warp, a.steps - x0);
-    cur.p = (int)(x0 >> 5);
-    cur.k = (int)(x0 & 31);
-    cur.n = min(32 - cur.k, cur.left);
+    cur.p = (int)(x0 / (unsigned)nsl);
+    cur.k = (int)(x0 - (unsigned)cur.p * (unsigned)nsl);
+    cur.n = min(nsl - cur.k, cur.left);
     const int g = P0 + cur.p;
     cur.batch = a.tpb == a.tiles ? 0 : g / ppb;
     const int rem = g - cur.batch * ppb;
@@ -279,7 +283,7 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
     s.p++;
     s.J++;
     s.k = 0;
-    s.n = min(32, s.left);
+    s.n = min(nsl, s.left);
     s.new_row = s.new_tile = s.J == a.tpb;
     if (s.new_tile) {
       if (++s.I == a.tpb) {
@@ -293,11 +297,19 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
   auto fetch = [&](const Segment &s) {
     if (s.left == 0) return;
     const int b0 = s.batch * a.nper;
-    if (s.new_tile) fetch_slot<R, ANG>(a, b0, s.I, lane, w.next_I);
-    fetch_slot<R, ANG>(a, b0, s.J, lane, w.next_J);
+    if (s.new_tile) fetch_slot<R, ANG>(a, nsl, b0, s.I, lane, w.next_I);
+    fetch_slot<R, ANG>(a, nsl, b0, s.J, lane, w.next_J);
   };
 
   fetch(cur);
+  // the slot that a lane meets at step k; lanes past the slots keep to their own,
+  // which is padding in every tile
+  const bool idle = !FULL && lane >= nsl;
+  auto met = [&](int k) {
+    if (FULL) return (lane + k) & 31;
+    const int s = lane + k;
+    return idle ? lane : (s >= nsl ? s - nsl : s);
+  };
   const V zero = splat(R(0), V());
   bool row_begun = false;  // the I sums are those of the row's first partial
   int held = 0;            // tile pairs whose I sums are still in registers
@@ -306,7 +318,7 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
   while (cur.left > 0) {
     copies_done();
     if (cur.new_tile) {
-      scale_slot<R, WALL, ANG>(a, cur.I, lane, w.next_I, w.I);
+      scale_slot<R, WALL, ANG>(a, nsl, cur.I, lane, w.next_I, w.I);
       row_begun = cur.new_row;
       held = 0;
 #pragma unroll
@@ -322,7 +334,7 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
         ui[q] = {zero, zero, zero, zero, zero, zero};
       }
     }
-    scale_slot<R, WALL, ANG>(a, cur.J, lane, w.next_J, w.J);
+    scale_slot<R, WALL, ANG>(a, nsl, cur.J, lane, w.next_J, w.J);
 #pragma unroll
     for (int c = 0; c < NC; c++) reinterpret_cast<V *>(w.A[c])[lane] = zero;
     __syncwarp();
@@ -333,7 +345,7 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
     unsigned near = 0u;  // steps with a pair closer than 2a
 #pragma unroll 1
     for (int k = cur.k; k < k_end; k++) {
-      const int s = (lane + k) & 31;
+      const int s = met(k);
       V vj[9], A[6];
 #pragma unroll
       for (int c = 0; c < 9; c++)
@@ -347,7 +359,7 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
 #pragma unroll
       for (int q = 0; q < NS; q++)
         close |= any_below4(pair_both<V, WALL, ANG>(vi[q], vj, ui[q], aj));
-      near |= close ? 1u << k : 0u;
+      near |= close && !idle ? 1u << k : 0u;
       if (!diag) {
         const V sum[6] = {aj.ux, aj.uy, aj.uz, aj.wx, aj.wy, aj.wz};
 #pragma unroll
@@ -380,16 +392,17 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
     // step: 500 batches of 60 13.3 us, 11.8 side by side; N = 200 in FP64 17.7,
     // 16.0.)
     unsigned st = __reduce_or_sync(0xffffffffu, near);
-    const unsigned slots = __funnelshift_l(near, near, lane);
+    const unsigned long long at = (unsigned long long)near << lane;  // bit k to k + lane
+    const unsigned slots = (unsigned)at | (unsigned)(at >> nsl);
     const bool apart =
         st == 0u || diag ||
         (int)__reduce_add_sync(0xffffffffu, (unsigned)__popc(near)) ==
-            __popc(__reduce_or_sync(0xffffffffu, slots));
+            __popc(__reduce_or_sync(0xffffffffu, slots & (0xffffffffu >> (32 - nsl))));
     while (st != 0u) {
       const unsigned from = apart ? near : st;
       const int k = __ffs(from) - 1;
       if (from != 0u && ((near >> k) & 1u)) {
-        const int s = (lane + k) & 31;
+        const int s = met(k);
         // which of the slots' pairs (NS q + h); FP32 takes the distances of all
         // four first, which spares most of the loads below
         unsigned which = (1u << (NS * NS)) - 1u;
@@ -513,8 +526,8 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
       });
       // I side: the row's own partial, then those of warps that began in it
       if (t >= a.row0 && t < a.row1) {
-        const unsigned xs = 32u * (unsigned)(tb * ppb + local_before(a.tpb, tl) - P0);
-        const unsigned xe = xs + 32u * (unsigned)(a.tpb - tl);
+        const unsigned xs = (unsigned)nsl * (unsigned)(tb * ppb + local_before(a.tpb, tl) - P0);
+        const unsigned xe = xs + (unsigned)nsl * (unsigned)(a.tpb - tl);
         const int w_lo = (int)(xs / a.per_warp), w_hi = (int)((xe - 1u) / a.per_warp);
         gather(w_hi - w_lo + 1, [&](int e) {
           return e == 0 ? slot_row + (t - a.row0) : slot_irow + w_lo + e;
@@ -542,8 +555,8 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
           a.acc[2 * o + 1] = c;
           return;
         }
-        const int l = tl * TS + p, i = tb * a.nper + l;
-        if (l >= a.nper || !LMG_IN_BOUNDS(i < a.N, 24, i)) return;
+        const int l = tl * NS * nsl + p, i = tb * a.nper + l;
+        if (p >= NS * nsl || l >= a.nper || !LMG_IN_BOUNDS(i < a.N, 24, i)) return;
         s += c;
         if (WALL) {
           const R z = mul_rn(a.pos[3 * (size_t)i + 2], a.inv_a);
@@ -579,11 +592,14 @@ template <class R> size_t pairs_smem(bool ang) {
   return kPairsThreads / 32 * (ang ? sizeof(PairsWarp<R, true>) : sizeof(PairsWarp<R, false>));
 }
 
-template <class R> const void *pairs_kernel(bool wall, bool ang) {
-  if (wall) return ang ? (const void *)mdot_pairs_kernel<R, true, true>
-                       : (const void *)mdot_pairs_kernel<R, true, false>;
-  return ang ? (const void *)mdot_pairs_kernel<R, false, true>
-             : (const void *)mdot_pairs_kernel<R, false, false>;
+template <class R, bool FULL> const void *pairs_kernel_of(bool wall, bool ang) {
+  if (wall) return ang ? (const void *)mdot_pairs_kernel<R, true, true, FULL>
+                       : (const void *)mdot_pairs_kernel<R, true, false, FULL>;
+  return ang ? (const void *)mdot_pairs_kernel<R, false, true, FULL>
+             : (const void *)mdot_pairs_kernel<R, false, false, FULL>;
+}
+template <class R> const void *pairs_kernel(bool wall, bool ang, bool full) {
+  return full ? pairs_kernel_of<R, true>(wall, ang) : pairs_kernel_of<R, false>(wall, ang);
 }
 
 }  // namespace
@@ -596,16 +612,27 @@ void mdot_pairs_plan_tables(int N, int nper, bool ang, long long resident, int f
   constexpr int TS = kPairsTile<R>;
   const int EL = (ang ? 6 : 3) * TS;
   const int tpb = (nper + TS - 1) / TS, nb = N / nper;
+  constexpr int NS = kPairsSlot<R>;
   const long long rows = (long long)nb * tpb;
   // 32-bit tile pair numbers; beyond a million particles a batch (FP32) the
   // passes' tables would grow past what they save
   if (tpb > 16384 || rows * (tpb + 1) / 2 >= (1LL << 30)) return;
+  // The slots of a tile in use: where there is work for every warp, as few as
+  // hold the batch in as many tiles, so that no tile is mostly padding (333
+  // particles: 6 tiles of 28 slots of two).  64 batches of 333 17.7 -> 16.9 us,
+  // above a wall with torques 48.0 -> 44.0; 64 of 100 in FP64 61 -> 52.  Where
+  // there is not, ranges of four steps fit 32 better (30 batches of 100 8.0 us,
+  // 8.8 with 25 slots).
+  const long long wpb = kPairsThreads / 32;
+  const int S = 16 * rows * (tpb + 1) > kPairsMinSteps * wpb * resident
+                    ? ((nper + tpb - 1) / tpb + NS - 1) / NS
+                    : 32;
   p.N = N;
   p.nper = nper;
   p.tpb = tpb;
+  p.slots = S;
   p.ang = ang;
   const size_t cap = max_part > 0 ? max_part : kPairsMaxPart;
-  const long long wpb = kPairsThreads / 32;
   // tile pairs of a pass: at least one row's, at most what the scratch holds
   // (the rows' and warps' slots come on top) and the steps' 31-bit count allows
   const long long max_pairs =
@@ -627,7 +654,7 @@ void mdot_pairs_plan_tables(int N, int nper, bool ang, long long resident, int f
     q.row0 = r;
     q.row1 = r1;
     const long long pairs = pairs_before(tpb, r1) - pairs_before(tpb, r);
-    const long long W = 32 * pairs;
+    const long long W = S * pairs;
     q.steps = (unsigned)W;
     long long nw = std::min(wpb * resident, (W + kPairsMinSteps - 1) / kPairsMinSteps);
     if (force_warps > 0) nw = std::min<long long>(nw, force_warps);
@@ -641,13 +668,13 @@ void mdot_pairs_plan_tables(int N, int nper, bool ang, long long resident, int f
     int row = r;
     long long start = 0;  // first tile pair of `row` in this pass
     for (int w = 1; w < q.warps; w++) {
-      const long long x = (long long)w * q.per_warp, pr = x >> 5;
+      const long long x = (long long)w * q.per_warp, pr = x / S;
       while (start + (tpb - row % tpb) <= pr) {
         start += tpb - row % tpb;
         row++;
       }
       const int J = row + (int)(pr - start);
-      if ((x & 31) != 0 && J != row) {
+      if (x % S != 0 && J != row) {
         col[w] = J;
         count[J + 1]++;
       }
@@ -672,14 +699,17 @@ void mdot_pairs_plan_tables(int N, int nper, bool ang, long long resident, int f
 template <class R>
 cudaError_t mdot_pairs_plan(int N, int nper, bool wall, bool ang, int num_sms, int force_warps,
                             size_t max_part, PairsPlan &p) {
-  int per_sm = 0;
-  cudaError_t e = cudaFuncSetAttribute(pairs_kernel<R>(wall, ang),
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)pairs_smem<R>(ang));
-  if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pairs_kernel<R>(wall, ang),
-                                                    kPairsThreads, pairs_smem<R>(ang));
-  if (e != cudaSuccess) return e;
+  int per_sm = 1 << 30;
+  for (const bool full : {true, false}) {
+    const void *k = pairs_kernel<R>(wall, ang, full);
+    int n = 0;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)pairs_smem<R>(ang));
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kPairsThreads, pairs_smem<R>(ang));
+    if (e != cudaSuccess) return e;
+    per_sm = std::min(per_sm, n);
+  }
   const long long tpb = (nper + kPairsTile<R> - 1) / kPairsTile<R>;
   const long long steps = 16 * tpb * (tpb + 1) * (N / nper);
   if (steps < pairs_few_steps(ang, tpb) * per_sm * num_sms * (kPairsThreads / 32)) per_sm = std::min(per_sm, 2);
@@ -704,6 +734,7 @@ cudaError_t mdot_pairs_launch(const PairsPlan &p, const int *cuts, const R *pos,
     a.N = p.N;
     a.nper = p.nper;
     a.tpb = p.tpb;
+    a.slots = p.slots;
     a.row0 = s.row0;
     a.row1 = s.row1;
     a.tiles = p.N / p.nper * p.tpb;
@@ -742,7 +773,7 @@ cudaError_t mdot_pairs_launch(const PairsPlan &p, const int *cuts, const R *pos,
     void *params[] = {(void *)&a};
     count_launch();
     const cudaError_t e =
-        cudaLaunchCooperativeKernel(pairs_kernel<R>(p.wall, p.ang), dim3(s.grid),
+        cudaLaunchCooperativeKernel(pairs_kernel<R>(p.wall, p.ang, p.slots == 32), dim3(s.grid),
                                     dim3(kPairsThreads), params, pairs_smem<R>(p.ang), stream);
     if (e != cudaSuccess) return e;
   }

@@ -10,12 +10,13 @@
 //
 // Work (per batch of nper particles, tiles of 32 slots; a slot is two
 // particles in FP32, one in FP64):
-//   * tile pairs (I, J), I <= J, are numbered row by row; each is 32 rotation
-//     steps: at step k lane l pairs the particles of its slot of tile I (in
-//     registers) with those of slot (l + k) mod 32 of tile J, staged in the
+//   * tile pairs (I, J), I <= J, are numbered row by row; each is S rotation
+//     steps, S the slots of a tile in use (32, or as few as hold a batch in as
+//     many tiles): at step k lane l < S pairs the particles of its slot of tile I
+//     (in registers) with those of slot (l + k) mod S of tile J, staged in the
 //     warp's shared memory beside that slot's sums.  No two lanes meet a slot
 //     in a step, so the J side needs neither atomics nor reductions.  On a
-//     diagonal tile (I, I) the 32 steps cover every ordered pair, and only the
+//     diagonal tile (I, I) the S steps cover every ordered pair, and only the
 //     I side is kept;
 //   * the steps of all tile pairs are cut into equal contiguous ranges, one
 //     per resident warp; the next tile is copied in while one is worked on.  A
@@ -49,7 +50,7 @@
 // open forces N = 4096 560 us (1019), wall with torques N = 3001 1264 us
 // (4974).  A few hundred particles cost 8 to 12 us (16 to 63), FP64 17 to 44
 // (298 to 3167): launch, one tile's latency, barrier and fold; 64 batches of 333,
-// open forces, 17.6 us, of which the steps take 8.
+// open forces, 16.9 us, of which the steps take 7.
 #pragma once
 #include <cstddef>
 #include <vector>
@@ -79,6 +80,7 @@ struct PairsPass {
 struct PairsPlan {
   bool ok = false;      // false: use mdot_kernel
   int N = 0, nper = 0, tpb = 0;
+  int slots = 32;       // of a tile in use (the same for all)
   bool wall = false, ang = false;
   std::vector<PairsPass> passes;
   size_t part_elems = 0;  // scratch (of R) of the largest pass

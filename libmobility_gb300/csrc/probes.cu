@@ -198,6 +198,7 @@ int lmg_internal_pairs_plan(int N, int nper, int ang, int precision, long long r
   info[2] = (long long)p.part_elems;
   info[3] = (long long)p.acc_elems;
   info[4] = p.tpb;
+  info[5] = p.slots;
   for (size_t q = 0; passes && q < p.passes.size(); q++) {
     const lmg::PairsPass &s = p.passes[q];
     const long long v[7] = {s.row0, s.row1, s.steps, s.per_warp, s.warps, s.grid,

@@ -26,7 +26,9 @@ SHAPES = [(1, 1, 0, 0), (2, 1, 0, 0), (33, 11, 0, 0), (63, 63, 0, 0), (65, 65, 1
           (129, 43, 3, 0), (640, 128, 0, 0), (1537, 1537, 0, 0), (1537, 1537, 37, 0),
           (1537, 1537, 40, 100000), (1998, 333, 16, 60000),
           # many tiles with few partials each: one warp folds a component of a tile
-          (9990, 333, 0, 0), (6000, 60, 0, 0), (9990, 333, 300, 300000)]
+          (9990, 333, 0, 0), (6000, 60, 0, 0), (9990, 333, 300, 300000),
+          # tiles with fewer slots in use (17 to 31, and ranges that cut them anywhere)
+          (9750, 65, 0, 0), (10000, 100, 0, 0), (8800, 200, 501, 0), (12000, 30, 0, 0)]
 
 
 @pytest.mark.parametrize("precision", ["float", "double"])

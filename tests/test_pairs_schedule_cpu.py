@@ -20,14 +20,14 @@ def lib():
 
 
 def plan(lib, N, nper, ang, double, resident, warps, max_part):
-    info = np.zeros(5, np.int64)
+    info = np.zeros(6, np.int64)
     ptr = lambda a: a.ctypes.data_as(ctypes.c_void_p)  # noqa: E731
     args = (N, nper, ang, double, resident, warps, max_part, ptr(info))
     assert lib.lmg_internal_pairs_plan(*args, None, None) == 0
     passes = np.zeros((int(info[0]), 7), np.int64)
     cuts = np.zeros(int(info[1]), np.int32)
     assert lib.lmg_internal_pairs_plan(*args, ptr(passes), ptr(cuts)) == 0
-    return passes, cuts, int(info[2]), int(info[3]), int(info[4])
+    return passes, cuts, int(info[2]), int(info[3]), int(info[4]), int(info[5])
 
 
 def before(tpb, r):
@@ -46,10 +46,18 @@ def test_every_step_and_partial_once(lib, N, nper, warps, max_part, double, ang)
     el = (6 if ang else 3) * tile
     # under a scratch limit only a few blocks are resident: two slots a warp
     resident = 3 if max_part else 152 * 3
-    passes, cuts, part, acc, tpb = plan(lib, N, nper, ang, double, resident, warps, max_part)
+    passes, cuts, part, acc, tpb, S = plan(lib, N, nper, ang, double, resident, warps, max_part)
     nb = N // nper
     rows = nb * tpb
     assert tpb == -(-nper // tile)
+    # equal tiles of S slots hold a batch; with work for every warp no slot more
+    # than needed, otherwise whole tiles
+    ns = 1 if double else 2
+    assert 1 <= S <= 32 and tpb * S * ns >= nper and (tpb - 1) * S * ns < nper
+    if 32 * nb * tpb * (tpb + 1) // 2 > 4 * 4 * resident:
+        assert tpb * (S - 1) * ns < nper
+    else:
+        assert S == 32
     assert passes[0, 0] == 0 and passes[-1, 1] == rows
     assert np.array_equal(passes[1:, 0], passes[:-1, 1])
     assert (acc > 0) == (len(passes) > 1)
@@ -63,7 +71,7 @@ def test_every_step_and_partial_once(lib, N, nper, warps, max_part, double, ang)
         assert row1 % tpb == 0 or row1 - row0 < tpb
         P0 = before(tpb, row0)
         npairs = before(tpb, row1) - P0
-        assert steps == 32 * npairs and nwarps <= 4 * grid and grid <= resident
+        assert steps == S * npairs and nwarps <= 4 * grid and grid <= resident
         assert (nwarps - 1) * per_warp < steps <= nwarps * per_warp
         slot_row, slot_irow = npairs, npairs + row1 - row0
         slot_cut = slot_irow + nwarps
@@ -74,12 +82,12 @@ def test_every_step_and_partial_once(lib, N, nper, warps, max_part, double, ang)
         assert len(pairs) == npairs
         for w in range(nwarps):
             x, left = w * per_warp, min(per_warp, steps - w * per_warp)
-            new_pair = x % 32 == 0
-            new_row = new_pair and pairs[x // 32][0] == pairs[x // 32][1]
+            new_pair = x % S == 0
+            new_row = new_pair and pairs[x // S][0] == pairs[x // S][1]
             while left > 0:
-                p, k = x // 32, x % 32
+                p, k = x // S, x % S
                 r, J = pairs[p]
-                n = min(32 - k, left)
+                n = min(S - k, left)
                 taken[x:x + n] += 1
                 if r != J:
                     slot = p if new_pair else slot_cut + w
@@ -103,7 +111,7 @@ def test_every_step_and_partial_once(lib, N, nper, warps, max_part, double, ang)
                 slot = before(tpb, b0) - P0 + I * tpb - I * (I - 1) // 2 + t - r
                 read[slot] = t
             if row0 <= t < row1:
-                xs, xe = 32 * (before(tpb, t) - P0), 32 * (before(tpb, t + 1) - P0)
+                xs, xe = S * (before(tpb, t) - P0), S * (before(tpb, t + 1) - P0)
                 read[slot_row + t - row0] = t
                 for g in range(xs // per_warp + 1, (xe - 1) // per_warp + 1):
                     read[slot_irow + g] = t
@@ -112,13 +120,19 @@ def test_every_step_and_partial_once(lib, N, nper, warps, max_part, double, ang)
         assert read == written
 
 
-def test_rotation_steps_cover_a_tile_pair():
-    """Lane l's slot meets slot (l + k) mod 32 at step k: every pair of slots
-    once over the 32 steps, and no slot twice in a step."""
+@pytest.mark.parametrize("S", [1, 2, 17, 31, 32])
+def test_rotation_steps_cover_a_tile_pair(S):
+    """Lane l's slot meets slot (l + k) mod S at step k: every pair of slots
+    once over the S steps, and no slot twice in a step; the lanes past S keep to
+    their own.  The slots of a lane's flagged steps, as a mask: bit k moves to
+    (k + l) mod S."""
     lane = np.arange(32)
-    seen = np.zeros((32, 32), int)
-    for k in range(32):
-        s = (lane + k) % 32
+    seen = np.zeros((S, S), int)
+    for k in range(S):
+        s = np.where(lane >= S, lane, np.where(lane + k >= S, lane + k - S, lane + k))
         assert len(set(s)) == 32
-        seen[lane, s] += 1
+        seen[lane[:S], s[:S]] += 1
+        for l in range(S):
+            at = (1 << k) << l
+            assert ((at | (at >> S)) & ((1 << S) - 1)) == 1 << s[l]
     assert (seen == 1).all()
