@@ -600,8 +600,8 @@ __global__ void __launch_bounds__(kSymThreads, MINB) mdot_sym_kernel(const SymAr
 // Register budget of the kernel: 2 resident blocks per SM (up to 255
 // registers a thread; the default: no spills, the rotation loop keeps the
 // broadcast slot values and two steps' sums in registers), 3 (168) or 4
-// (128, spills).  Measured at N = 4096 / 16384 / 65536: 22.1 / 192 / 2973 us
-// with 2, 25.1 / 193 / 2922 us with 3, 27.1 / 200 / 3008 us with 4.
+// (128, spills).  Measured at N = 4096 / 16384 / 65536: 19.3 / 174 / 2607 us
+// with 2, 22.7 / 181 / 2708 us with 3, 24.7 / 188 / 2757 us with 4.
 const void *sym_kernel(int variant) {
   if (variant == 3) return (const void *)mdot_sym_kernel<3>;
   if (variant == 4) return (const void *)mdot_sym_kernel<4>;
