@@ -473,6 +473,17 @@ mdot_kernel(const MdotArgs<R> a) {
                 wall_uf_far_x2(a.k, a.kw, bc(xi[t]), bc(yi[t]), bc(zi[t]), v[0], v[1], v[2],
                                v[3], v[4], v[5], u2[t]);
             };
+            // forces alone take four at a time where they can (N = 1000 24.5 -> 24.0
+            // us, 2048 25.9 -> 25.3, 4096 63.9 -> 63.1); with torques two are as many
+            // as the pipe takes (2048 41.3, 42.4 with four)
+            if (!PACK && pp < 13 && ((any[t] >> pp) & 15u) == 0u) {
+              far(pp);
+              far(pp + 1);
+              far(pp + 2);
+              far(pp + 3);
+              pp += 2;
+              continue;
+            }
             if (((any[t] >> pp) & 3u) == 0u) {
               far(pp);
               far(pp + 1);
