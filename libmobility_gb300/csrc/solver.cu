@@ -177,7 +177,7 @@ template <class R> class Solver final : public SolverBase {
   int step_per_sm_ = 0;  // resident krylov_step_kernel blocks per SM
   int step_ctas_ = -1;   // CTAs of the cluster of krylov_step_cluster_kernel (0: none fits)
   bool tickets_zeroed_ = false;
-  std::map<long, MdotPlan> plans_;
+  std::map<std::tuple<int, int, int, int, int>, MdotPlan> plans_;
   // symmetric open-space product (FP32): plans with their device tables,
   // partial sums and barrier counts, and the flag a barrier that timed out
   // raises
@@ -371,8 +371,10 @@ void Solver<R>::mdot_device(const R *pos, const R *F, const R *T, R *U, R *W, bo
   if (!few && s.geom == kOpen && s.has_f && !s.has_t && !s.ang && mdot_sym(pos, F, U)) return;
   if (!solve && mdot_pairs(pos, F, s.has_t ? T : nullptr, U, ang_ ? W : nullptr)) return;
   const int ftpt = g_force_tpt.load(), fsplit = g_force_split.load();
-  const long key = ((long)N << 30) | ((long)fsplit << 10) | (ftpt << 8) | (s.geom << 3) |
-                   (s.has_f << 2) | (s.has_t << 1) | s.ang;
+  // the batch size is part of a plan (its splits cover a tile's batches), and
+  // setParameters may change it at the same N
+  const int shape = (s.geom << 3) | (s.has_f << 2) | (s.has_t << 1) | (int)s.ang;
+  const auto key = std::make_tuple(N, nper, ftpt, fsplit, shape);
   auto it = plans_.find(key);
   if (it == plans_.end() || it->second.tiles == 0) {
     MdotPlan plan;
