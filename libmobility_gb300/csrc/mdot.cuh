@@ -393,7 +393,6 @@ mdot_kernel(const MdotArgs<R> a) {
           }
         }
       }
-#pragma unroll 1
       for (; jj < n_here; jj++) one(jj, std::true_type());
     } else if constexpr (EVENTS) {
       // Two sources per instruction, 32 sources at a time.  Packed pairs with a

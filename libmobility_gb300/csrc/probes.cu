@@ -17,6 +17,7 @@
 #include "common.hpp"
 #include "launch_count.hpp"
 #include "mdot_pairs.cuh"
+#include "mdot_route.hpp"
 #include "mdot_sym.cuh"
 
 namespace lmg {
@@ -167,6 +168,14 @@ int lmg_internal_sym_plan(int N, int nper, long long resident, int force_warps, 
   if (warps) std::memcpy(warps, p.warps.data(), p.warps.size() * sizeof(int4));
   if (tused) std::memcpy(tused, p.tused.data(), p.tused.size() * sizeof(int));
   return 0;
+}
+
+// The kernel that a product outside a solve takes on a GPU of num_sms SMs: 0
+// mdot_kernel, 1 mdot_sym_kernel, 2 mdot_pairs_kernel.  one: forces or torques
+// alone, with angular velocities.
+int lmg_internal_mdot_route(int precision, int wall, int ang, int one, int N, int nper,
+                            int num_sms) {
+  return (int)lmg::mdot_route(precision != 0, wall != 0, ang != 0, one != 0, N, nper, num_sms);
 }
 
 // Largest scratch (elements) of a pass of the unordered-pair product planned

@@ -21,6 +21,7 @@
 #include "launch_count.hpp"
 #include "mdot_launch.cuh"
 #include "mdot_pairs.cuh"
+#include "mdot_route.hpp"
 #include "mdot_sym.cuh"
 #include "precond.cuh"
 #include "solver.hpp"
@@ -360,16 +361,19 @@ void Solver<R>::mdot_device(const R *pos, const R *F, const R *T, R *U, R *W, bo
     if (W) LMG_CUDA(cudaMemsetAsync(W, 0, 3 * (size_t)N * sizeof(R), stream()));
     return;
   }
-  // Outside a solve the unordered-pair product takes every shape: against
-  // mdot_kernel 12 to 62 us at N = 500 (wall, torques, FP32), 680 to 1399 at
-  // 16384, 69 to 3004 at 500 and 1265 to 4974 at 3000 in FP64, and 6.6 to 5.6
-  // only at N = 50 (open, forces).  The symmetric open-space kernel keeps FP32
-  // forces from batches of 384 on (7.3 to 8.6 us at 200, 8.0 to 8.6 at 333,
-  // 8.4 to 8.3 at 500, 23.7 to 20.2 at 4096): four particles a slot and no
-  // staging of torques, but tiles of 128.
-  const bool few = !solve && nper < 384;
-  if (!few && s.geom == kOpen && s.has_f && !s.has_t && !s.ang && mdot_sym(pos, F, U)) return;
-  if (!solve && mdot_pairs(pos, F, s.has_t ? T : nullptr, U, ang_ ? W : nullptr)) return;
+  // (the products of a solve keep the kernels they had, see mdot_device's
+  // declaration; a test that caps the warps or the scratch means the pairs)
+  MdotRoute route = solve ? MdotRoute::symmetric
+                          : mdot_route(sizeof(R) == 8, wall_, ang_, ang_ && s.has_f != s.has_t, N,
+                                       nper, sms());
+  if (route == MdotRoute::tiled && (g_sym_warps.load() || g_pairs_max_part.load()))
+    route = MdotRoute::pairs;
+  if (route == MdotRoute::symmetric && s.geom == kOpen && s.has_f && !s.ang &&
+      mdot_sym(pos, F, U))
+    return;
+  if (!solve && route != MdotRoute::tiled &&
+      mdot_pairs(pos, F, s.has_t ? T : nullptr, U, ang_ ? W : nullptr))
+    return;
   const int ftpt = g_force_tpt.load(), fsplit = g_force_split.load();
   // the batch size is part of a plan (its splits cover a tile's batches), and
   // setParameters may change it at the same N
