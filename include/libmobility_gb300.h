@@ -96,7 +96,11 @@ lmg_status lmg_destroy(lmg_solver *h);
  * first use), which is also what a handle uses before this is ever called.
  * The solver may use one more internal stream for work that overlaps the
  * matrix-vector products of Lanczos; it is joined back before a call
- * returns. */
+ * returns.  The stream may change between calls: the calls of a handle share
+ * its buffers, and the first on another stream waits on the GPU for the work of
+ * the last one (whose stream may have been destroyed since).  Calls captured
+ * into a CUDA graph are outside this order: a graph's launches must not overlap
+ * each other or other calls of the handle. */
 #define LMG_OWN_STREAM ((void *)(intptr_t)-1)
 lmg_status lmg_set_stream(lmg_solver *h, void *cuda_stream);
 

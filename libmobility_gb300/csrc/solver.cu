@@ -271,6 +271,7 @@ template <class R> void Solver<R>::ensure_reduction(int blocks) {
 
 template <class R> void Solver<R>::set_positions(const void *pos, size_t n) {
   NvtxRange nvtx_range_("lmg setPositions");
+  const Call call_(*this);
   if (n % 3 != 0)
     throw Error(LMG_ERR_INVALID_ARGUMENT,
                 "[libMobility] The input arrays for positions, forces, and torques must each "
@@ -473,6 +474,7 @@ template <class R>
 void Solver<R>::mdot_rows(int64_t row_begin, int64_t row_end, const void *F, size_t nF,
                           const void *T, size_t nT, void *U, size_t nU, void *W, size_t nW) {
   NvtxRange nvtx_range_("lmg Mdot rows");
+  const Call call_(*this);
   if (!F) nF = 0;
   if (!T) nT = 0;
   if (!U) nU = 0;
@@ -640,6 +642,7 @@ template <class R>
 void Solver<R>::mdot(const void *F, size_t nF, const void *T, size_t nT, void *U, size_t nU,
                      void *W, size_t nW) {
   NvtxRange nvtx_range_("lmg Mdot");
+  const Call call_(*this);
   if (!F) nF = 0;
   if (!T) nT = 0;
   if (!U) nU = 0;
@@ -1069,6 +1072,7 @@ template <class R>
 void Solver<R>::sqrt_mdot_w(void *U, size_t nU, void *W, size_t nW, double prefactor,
                             const void *dW, size_t ndW, int *iterations, double *residual) {
   NvtxRange nvtx_range_("lmg sqrtMdotW");
+  const Call call_(*this);
   if (prefactor == 0) return;
   if (!initialized_)
     throw Error(LMG_ERR_NOT_INITIALIZED,
@@ -1187,6 +1191,7 @@ void Solver<R>::sqrt_mdot_w(void *U, size_t nU, void *W, size_t nW, double prefa
 template <class R>
 void Solver<R>::div_m(void *U, size_t nU, void *W, size_t nW, double prefactor) {
   NvtxRange nvtx_range_("lmg divM");
+  const Call call_(*this);
   if (prefactor == 0) return;
   if (!wall_) return;  // no wall, no thermal drift (mobility.h:189-190)
   if (!U) nU = 0;

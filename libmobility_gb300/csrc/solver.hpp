@@ -90,6 +90,8 @@ class SolverBase {
   bool include_angular() const { return ang_; }
   void set_stream(cudaStream_t s);   // s is used as given (0 = default stream)
   void use_own_stream();
+  // The stream of the call.  Calls share the handle's buffers, so the first use
+  // of another stream than the last call's makes it wait for that call's work.
   cudaStream_t stream();
   void set_iteration_limit(int limit);  // lanczos::Solver::setIterationHardLimit
   void synchronize();
@@ -129,6 +131,28 @@ class SolverBase {
   bool have_stream_ = false;
   bool own_stream_ = false;
   cudaStream_t own_ = nullptr;
+  // the last call's work: its stream, and the event recorded after it (a stream
+  // the caller has destroyed since cannot be asked)
+  cudaStream_t work_stream_ = nullptr;
+  cudaEvent_t work_done_ = nullptr;
+  bool has_work_ = false, work_recorded_ = false;
+  bool capturing();
+  void ensure_work_event();
+  void follow_last_call();
+  void record_work();
+  // Around a call that may leave work running on the stream.
+  struct Call {
+    SolverBase &s;
+    explicit Call(SolverBase &s_) : s(s_) {}
+    ~Call() {
+      try {
+        s.record_work();
+      } catch (const Error &) {  // (a failed launch before it is what the caller hears of)
+      }
+    }
+    Call(const Call &) = delete;
+    Call &operator=(const Call &) = delete;
+  };
 
   // shared argument checks (messages of pythonify.h / mobility.h)
   void check_positions_set(const char *who) const;

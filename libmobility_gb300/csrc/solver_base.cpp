@@ -30,6 +30,7 @@ SolverBase::SolverBase(Periodicity x, Periodicity y, Periodicity z) {
 }
 
 SolverBase::~SolverBase() {
+  if (work_done_) cudaEventDestroy(work_done_);
   if (own_) cudaStreamDestroy(own_);
 }
 
@@ -161,7 +162,52 @@ cudaStream_t SolverBase::stream() {
     have_stream_ = true;
     own_stream_ = true;
   }
+  // (cudaStreamPerThread names another stream in every thread)
+  if (has_work_ && (stream_ != work_stream_ || stream_ == cudaStreamPerThread)) follow_last_call();
   return stream_;
+}
+
+// Whether the call is being captured into a graph: nothing runs then, and an
+// event recorded in a capture or before it is no use on the other side.
+bool SolverBase::capturing() {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream_, &st) != cudaSuccess) {
+    (void)cudaGetLastError();  // the default stream while another is captured
+    return true;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
+void SolverBase::ensure_work_event() {
+  if (!work_done_) LMG_CUDA(cudaEventCreateWithFlags(&work_done_, cudaEventDisableTiming));
+}
+
+void SolverBase::follow_last_call() {
+  if (capturing()) return;
+  if (!work_recorded_) {
+    ensure_work_event();
+    LMG_CUDA(cudaEventRecord(work_done_, work_stream_));
+    work_recorded_ = true;
+  }
+  LMG_CUDA(cudaStreamWaitEvent(stream_, work_done_, 0));
+  work_stream_ = stream_;
+}
+
+// The default stream and the handle's own are there whenever the event is
+// wanted, so it is recorded when the stream changes; after work on a stream of
+// the caller's it is recorded at once (1 us a call; none on those two).
+void SolverBase::record_work() {
+  if (!have_stream_) return;
+  const bool lasting =
+      stream_ == nullptr || stream_ == cudaStreamLegacy || (own_ && stream_ == own_);
+  if (!lasting) {
+    if (capturing()) return;
+    ensure_work_event();
+    LMG_CUDA(cudaEventRecord(work_done_, stream_));
+  }
+  work_recorded_ = !lasting;
+  work_stream_ = stream_;
+  has_work_ = true;
 }
 
 // LanczosAlgorithm.h:272-274 (the reference default is 200)

@@ -151,7 +151,8 @@ class NBody:
         """Issue the work on the caller's current torch stream when CUDA
         tensors (inputs as _Arr, or output tensors) are involved, so it is
         ordered with the caller's own work (the default stream included);
-        otherwise on the handle's private stream."""
+        otherwise on the handle's private stream.  The library orders a call
+        after the calls before it, whichever streams they are on."""
         for x in objs:
             if x is None:
                 continue
