@@ -199,6 +199,9 @@ template <class R> class Solver final : public SolverBase {
   // of their own (a captured product names it: a solve must not move it)
   struct PairsState {
     PairsPlan plan;
+    // what is copied to the device buffer: the copy may still read it after the
+    // call (freeing the buffer, which comes first, waits for it)
+    std::vector<unsigned long long> upload;
     DeviceBuffer<unsigned long long> bars_and_cuts;
   };
   std::map<std::tuple<int, int, int, int>, std::unique_ptr<PairsState>> pairs_plans_;
@@ -611,8 +614,10 @@ bool Solver<R>::mdot_pairs(const R *pos, const R *F, const R *T, R *U, R *W) {
                                 g_pairs_max_part.load(), st->plan));
     const PairsPlan &p = st->plan;
     if (p.ok) {
-      std::vector<unsigned long long> up(p.passes.size() + (p.cuts.size() + 1) / 2, 0ull);
+      auto &up = st->upload;
+      up.assign(p.passes.size() + (p.cuts.size() + 1) / 2, 0ull);
       std::memcpy(up.data() + p.passes.size(), p.cuts.data(), p.cuts.size() * sizeof(int));
+      st->plan.cuts = {};
       LMG_CUDA(cudaMemcpyAsync(st->bars_and_cuts.ensure(up.size()), up.data(),
                                up.size() * sizeof(up[0]), cudaMemcpyHostToDevice, stream()));
     }

@@ -89,3 +89,28 @@ def test_captured(lib, precision, N, warm):
     assert rel_err(got[0], U.cpu().numpy()) <= TOL[precision]
     assert rel_err(got[1], W.cpu().numpy()) <= TOL[precision]
     F.copy_(F2)
+
+
+def test_first_call_with_large_tables(lib, oracle):
+    """The first product of a plan, whose tables (0.2 MB here) go to the device from
+    host memory that has to last until they are there; host memory of that size is
+    taken and overwritten at once."""
+    nper, nb = 30, 50000
+    rng = np.random.default_rng(3)
+    p = rng.uniform(0, 12, (nper * nb, 3)).astype(np.float32)
+    F, T = rng.normal(size=(2, nper * nb, 3)).astype(np.float32)
+    assert lib.lmg_internal_sym_override(0, 1300) == 0
+    s = make_solver(1, 1, 1.1, 0.9, "float", nper * nb, nper)
+    import torch
+    dp, dF, dT = (torch.tensor(x, device="cuda") for x in (p, F, T))
+    s.setPositions(dp)
+    torch.cuda.synchronize()
+    U, W = s.Mdot(dF, dT)
+    junk = [np.full(150000 + 1000 * k, -1, np.int64) for k in range(20)]
+    U, W = U.cpu().numpy(), W.cpu().numpy()
+    assert len(junk) == 20
+    some = slice(0, 200 * nper), slice((nb - 200) * nper, nb * nper)
+    for sl in some:
+        Uo, Wo = oracle.mdot(p[sl], F[sl], T[sl], a=1.1, viscosity=0.9, wall=1, include_angular=1,
+                             nper_batch=nper)
+        assert rel_err(U[sl], Uo) <= TOL["float"] and rel_err(W[sl], Wo) <= TOL["float"]
