@@ -47,10 +47,11 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar) {
 // multiple of gridDim.x.  Launches that share a count must all have the same
 // number of blocks and must not overlap (launches on one stream never do),
 // so their arrivals never mix.  One atomic per block, no reset; the wait is
-// bounded like grid_barrier's.
+// bounded like grid_barrier's, to `spins` polls (0: every block reports that its
+// wait ran out, after its arrival).
 constexpr long kMonoSpins = 1L << 26;
 
-__device__ __forceinline__ bool grid_barrier_mono(unsigned long long *count) {
+__device__ __forceinline__ bool grid_barrier_mono(unsigned long long *count, long spins) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -63,7 +64,7 @@ __device__ __forceinline__ bool grid_barrier_mono(unsigned long long *count) {
     asm volatile("atom.release.gpu.add.u64 %0, [%1], 1;" : "=l"(old) : "l"(count) : "memory");
     const unsigned long long target = (old / g + 1) * g;
     int ok = 0;
-    for (long it = 0; it < kMonoSpins; it++) {
+    for (long it = 0; it < spins; it++) {
       unsigned long long v;
       asm volatile("ld.acquire.gpu.u64 %0, [%1];" : "=l"(v) : "l"(count) : "memory");
       if (v >= target) {

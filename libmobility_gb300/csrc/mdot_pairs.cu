@@ -1,6 +1,7 @@
 // All-pairs product over unordered pairs: kernel, plan and launch.  The scheme
 // is described in mdot_pairs.cuh.  Compiled once per precision (LMG_REAL).
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <type_traits>
 
@@ -77,6 +78,7 @@ template <class R> struct PairsArgs {
   R *acc;
   const int *cuts;
   unsigned long long *bar;
+  long spins;  // of the barrier
   int *err;
 };
 
@@ -471,10 +473,10 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
     cur = nxt;
   }
 
-  if (!grid_barrier_mono(a.bar)) {
-    if (threadIdx.x == 0) *a.err = 1;
-    return;
-  }
+  // after a wait that ran out the partials may be incomplete: the sums that this
+  // block folds are NaN, and the host raises an error when it sees the flag
+  const bool complete = grid_barrier_mono(a.bar, a.spins);
+  if (!complete && threadIdx.x == 0) *a.err = 1;
 
   // ---- fold the partials: one component of a tile at a time, by a warp or by
   // the block's four warps, each taking every fourth partial, sixteen loads ahead ----
@@ -550,6 +552,7 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
             c += red[q][1][p];
           }
         }
+        if (!complete) s = R(NAN);
         if (!a.last) {
           a.acc[2 * o] = s;
           a.acc[2 * o + 1] = c;
@@ -754,6 +757,7 @@ cudaError_t mdot_pairs_launch(const PairsPlan &p, const int *cuts, const R *pos,
              ((reinterpret_cast<uintptr_t>(pos) | reinterpret_cast<uintptr_t>(F) |
                reinterpret_cast<uintptr_t>(T)) & 7) == 0;
     a.bar = bar + q;
+    a.spins = g_barrier_spins.load() < 0 ? kMonoSpins : g_barrier_spins.load();
     a.err = err;
     // Folding: rounds of loads one after the other (16 partials a warp, about
     // as much again to start and finish a component of a tile) with four warps

@@ -25,6 +25,7 @@ std::atomic<unsigned long long> g_launches{0};
 std::atomic<int> g_force_tpt{0}, g_force_split{0};
 std::atomic<int> g_sym_mode{0}, g_sym_warps{0}, g_sym_variant{0};
 std::atomic<size_t> g_pairs_max_part{0};
+std::atomic<long> g_barrier_spins{-1};
 std::atomic<unsigned long long *> g_sym_trace{nullptr};
 std::atomic<int> g_lanczos_device_sqrt{2};
 std::atomic<int> g_lanczos_lookahead{0};
@@ -183,6 +184,14 @@ int lmg_internal_mdot_route(int precision, int wall, int ang, int one, int N, in
 int lmg_internal_pairs_max_part(long long elems) {
   if (elems < 0) return 1;
   lmg::g_pairs_max_part.store((size_t)elems);
+  return 0;
+}
+
+// Polls of the grid barriers of the symmetric and unordered-pair products
+// launched after the call: 0 makes every wait run out, -1 restores the default.
+int lmg_internal_barrier_spins(long long spins) {
+  if (spins < -1) return 1;
+  lmg::g_barrier_spins.store((long)spins);
   return 0;
 }
 

@@ -117,6 +117,10 @@ template <class R> class Solver final : public SolverBase {
   void sqrt_mdot_w(void *U, size_t nU, void *W, size_t nW, double prefactor, const void *dW,
                    size_t ndW, int *iterations, double *residual) override;
   void div_m(void *U, size_t nU, void *W, size_t nW, double prefactor) override;
+  void synchronize() override {
+    SolverBase::synchronize();
+    check_barriers();
+  }
   void clean() override;
   void set_preconditioner(const std::string &kind, const float *params, size_t n) override;
 
@@ -515,12 +519,14 @@ void Solver<R>::mdot_rows(int64_t row_begin, int64_t row_end, const void *F, siz
 }
 
 // The flag the grid barriers of the symmetric and unordered-pair kernels raise
-// when a wait ran out in an earlier launch: the arrival counts are then
-// inconsistent, so they start afresh and the caller gets an error.
+// when a wait ran out: results of that launch are NaN and the arrival counts may
+// be inconsistent, so they start afresh and the caller gets an error: of the
+// call itself where it waits for its result, else of the next product or
+// synchronize.
 template <class R> void Solver<R>::check_barriers() {
-  if (!sym_err_.ptr) sym_err_.ensure(1);
-  if (!*(volatile int *)sym_err_.ptr) return;
+  if (!sym_err_.ptr || !*(volatile int *)sym_err_.ptr) return;
   LMG_CUDA(cudaStreamSynchronize(stream()));
+  if (side_) LMG_CUDA(cudaStreamSynchronize(side_));
   for (auto &kv : sym_plans_)
     if (kv.second->count.ptr)
       LMG_CUDA(cudaMemsetAsync(kv.second->count.ptr, 0, sizeof(unsigned long long), stream()));
@@ -531,7 +537,8 @@ template <class R> void Solver<R>::check_barriers() {
                                stream()));
   *(volatile int *)sym_err_.ptr = 0;
   throw Error(LMG_ERR_TIMEOUT,
-              "[libmobility_gb300] Mdot: grid barrier of the symmetric kernel timed out");
+              "[libmobility_gb300] Mdot: a grid barrier timed out (the products since the last "
+              "check are NaN)");
 }
 
 // U = M F with the symmetric open-space kernel (FP32, forces only, no
@@ -574,6 +581,7 @@ template <class R> bool Solver<R>::mdot_sym(const R *pos, const R *F, R *U) {
     const SymState &st = *it->second;
     const SymPlan &p = st.plan;
     if (p.grid <= 0) return false;
+    sym_err_.ensure(1);
     check_barriers();
     const PairConst<float> k = make_pair_const<float>(t0_, r0_, rt0_);
     SymTables tab;
@@ -625,6 +633,7 @@ bool Solver<R>::mdot_pairs(const R *pos, const R *F, const R *T, R *U, R *W) {
   }
   const PairsState &st = *it->second;
   if (!st.plan.ok) return false;
+  sym_err_.ensure(1);
   check_barriers();
   try {
     pairs_part_.ensure(st.plan.part_elems);
@@ -676,6 +685,7 @@ void Solver<R>::mdot(const void *F, size_t nF, const void *T, size_t nT, void *U
     LMG_CUDA(cudaStreamSynchronize(stream()));
     if (nU && !u_dev) std::memcpy(U, h, n3 * sizeof(R));
     if (nW && !w_dev) std::memcpy(W, h + n3, n3 * sizeof(R));
+    check_barriers();
   }
 }
 
@@ -940,6 +950,7 @@ int Solver<R>::lanczos(const R *z, R *y_out, size_t n, double tol, double *resid
     LMG_CUDA(cudaEventSynchronize(ev_check_[pi & 1]));
     if (mir[516] != 0.0)
       fail(LMG_ERR_TIMEOUT, "[libmobility_gb300] Lanczos step: grid barrier timed out");
+    check_barriers();  // of the symmetric product
     err = tested ? mir[512 + (pi & 1)] : HUGE_VAL;
     if (tested) {  // the reference never tests the first estimate (i > 0 there)
       if (residual) *residual = err;
@@ -1188,6 +1199,7 @@ void Solver<R>::sqrt_mdot_w(void *U, size_t nU, void *W, size_t nW, double prefa
   } else {
     LMG_CUDA(cudaStreamSynchronize(stream()));
   }
+  check_barriers();
 }
 
 // Thermal drift by random finite differences.  Positions are displaced in the
@@ -1259,6 +1271,7 @@ void Solver<R>::div_m(void *U, size_t nU, void *W, size_t nW, double prefactor) 
     LMG_CUDA(cudaStreamSynchronize(st));
     if (!u_dev) std::memcpy(U, h, n3 * sizeof(R));
     if (nW && !w_dev) std::memcpy(W, h + n3, n3 * sizeof(R));
+    check_barriers();
   }
 }
 

@@ -94,7 +94,7 @@ class SolverBase {
   // of another stream than the last call's makes it wait for that call's work.
   cudaStream_t stream();
   void set_iteration_limit(int limit);  // lanczos::Solver::setIterationHardLimit
-  void synchronize();
+  virtual void synchronize();
 
   std::string last_error;
 
