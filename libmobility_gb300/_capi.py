@@ -112,6 +112,7 @@ def load():
         "lmg_internal_mdot_route": [_I, _I, _I, _I, _I, _I, _I],
         "lmg_internal_pairs_max_part": [_L],
         "lmg_internal_barrier_spins": [_L],
+        "lmg_internal_pairs_refuse": [_I],
         "lmg_internal_pairs_plan": [_I, _I, _I, _I, _L, _I, _L, _VP, _VP, _VP],
         "lmg_internal_gemm": [_I, _I, _I, _I, _I, _VP, _I, _VP, _I, _VP, _I, _VP, _I, _F, _VP],
         "lmg_internal_tanh_backward": [_SZ, _VP, _VP, _VP],

@@ -17,6 +17,8 @@ extern std::atomic<int> g_sym_mode, g_sym_warps, g_sym_variant;
 // largest scratch of a pass of the unordered-pair product (0 = default);
 // g_sym_mode and g_sym_warps apply to that product too
 extern std::atomic<size_t> g_pairs_max_part;
+// tests: the unordered-pair product is refused 1 its scratch, 2 its launch
+extern std::atomic<int> g_pairs_refuse;
 // polls of the grid barriers of both (-1 = default; tests: 0, every wait runs out)
 extern std::atomic<long> g_barrier_spins;
 // T^{1/2} e1 of the single-system Lanczos checks: 0 the exact host QL; 1 on

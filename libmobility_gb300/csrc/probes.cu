@@ -26,6 +26,7 @@ std::atomic<int> g_force_tpt{0}, g_force_split{0};
 std::atomic<int> g_sym_mode{0}, g_sym_warps{0}, g_sym_variant{0};
 std::atomic<size_t> g_pairs_max_part{0};
 std::atomic<long> g_barrier_spins{-1};
+std::atomic<int> g_pairs_refuse{0};
 std::atomic<unsigned long long *> g_sym_trace{nullptr};
 std::atomic<int> g_lanczos_device_sqrt{2};
 std::atomic<int> g_lanczos_lookahead{0};
@@ -184,6 +185,14 @@ int lmg_internal_mdot_route(int precision, int wall, int ang, int one, int N, in
 int lmg_internal_pairs_max_part(long long elems) {
   if (elems < 0) return 1;
   lmg::g_pairs_max_part.store((size_t)elems);
+  return 0;
+}
+
+// The unordered-pair products after the call behave as if 1 the memory for their
+// partial sums, 2 their cooperative launch were refused; 0 restores the default.
+int lmg_internal_pairs_refuse(int what) {
+  if (what < 0 || what > 2) return 1;
+  lmg::g_pairs_refuse.store(what);
   return 0;
 }
 

@@ -635,20 +635,31 @@ bool Solver<R>::mdot_pairs(const R *pos, const R *F, const R *T, R *U, R *W) {
   if (!st.plan.ok) return false;
   sym_err_.ensure(1);
   check_barriers();
+  const int refuse = g_pairs_refuse.load();
   try {
+    if (refuse == 1) throw_cuda(cudaErrorMemoryAllocation, "lmg_internal_pairs_refuse");
     pairs_part_.ensure(st.plan.part_elems);
     if (st.plan.acc_elems) pairs_acc_.ensure(st.plan.acc_elems);
-  } catch (const Error &) {  // no memory left for the partial sums (at most 1 GiB)
+  } catch (const Error &) {  // no memory left for the partial sums (2^28 elements and more)
     (void)cudaGetLastError();
     pairs_part_.release();
     return false;
   }
   unsigned long long *bars = st.bars_and_cuts.ptr;
-  LMG_CUDA(mdot_pairs_launch<R>(st.plan,
-                                reinterpret_cast<const int *>(bars + st.plan.passes.size()), pos,
-                                F, T, U, W, (R)(1.0 / a_), make_pair_scale<R>(t0_, rt0_),
-                                pairs_part_.ptr, pairs_acc_.ptr, bars, sym_err_.device_ptr(),
-                                stream()));
+  const cudaError_t e =
+      refuse == 2 ? cudaErrorCooperativeLaunchTooLarge
+                  : mdot_pairs_launch<R>(
+                        st.plan, reinterpret_cast<const int *>(bars + st.plan.passes.size()), pos,
+                        F, T, U, W, (R)(1.0 / a_), make_pair_scale<R>(t0_, rt0_), pairs_part_.ptr,
+                        pairs_acc_.ptr, bars, sym_err_.device_ptr(), stream());
+  // fewer SMs for this context than the device reports: the blocks cannot all be
+  // resident, and the kernel that waits on nothing does the product
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    (void)cudaGetLastError();
+    it->second->plan.ok = false;
+    return false;
+  }
+  LMG_CUDA(e);
   return true;
 }
 

@@ -114,3 +114,39 @@ def test_first_call_with_large_tables(lib, oracle):
         Uo, Wo = oracle.mdot(p[sl], F[sl], T[sl], a=1.1, viscosity=0.9, wall=1, include_angular=1,
                              nper_batch=nper)
         assert rel_err(U[sl], Uo) <= TOL["float"] and rel_err(W[sl], Wo) <= TOL["float"]
+
+
+@pytest.mark.parametrize("refused", [1, 2])  # its scratch, its cooperative launch
+@pytest.mark.parametrize("precision,wall,ang,N", [("float", 0, 1, 900), ("float", 1, 1, 300),
+                                                  ("float", 1, 0, 3000), ("double", 1, 1, 500),
+                                                  ("double", 0, 0, 700)])
+def test_refused(lib, refused, precision, wall, ang, N):
+    """Without memory for the partial sums, or where the grid cannot be resident at
+    once, the product is mdot_kernel's, bit for bit."""
+    rng = np.random.default_rng(N)
+    dt = np.float32 if precision == "float" else np.float64
+    p = rng.uniform(0.5, 0.5 + (N * 4 * np.pi / 3 / 0.1) ** (1 / 3), (N, 3)).astype(dt)
+    F, T = rng.normal(size=(2, N, 3)).astype(dt)
+    T = T if ang else None
+
+    def product(s):
+        return [x for x in s.Mdot(F, T) if x is not None]
+
+    fresh = lambda: make_solver(wall, ang, 1.0, 1.0, precision)  # noqa: E731
+    s, t = fresh(), fresh()
+    s.setPositions(p), t.setPositions(p)
+    pairs = product(t)
+    assert lib.lmg_internal_sym_override(1, 0) == 0
+    want = product(s)
+    assert lib.lmg_internal_sym_override(0, 0) == 0
+    try:
+        assert lib.lmg_internal_pairs_refuse(refused) == 0
+        for _ in range(2):
+            got = product(s)
+            assert all(np.array_equal(x, y) for x, y in zip(got, want))
+    finally:
+        lib.lmg_internal_pairs_refuse(0)
+    # memory may be there the next time
+    got = product(s)
+    assert all(np.array_equal(x, y) for x, y in zip(got, pairs if refused == 1 else want))
+    assert not all(np.array_equal(x, y) for x, y in zip(pairs, want))
