@@ -18,7 +18,6 @@
 #pragma once
 #include <cmath>
 #include <cstdint>
-#include <type_traits>
 #include <cuda_runtime.h>
 
 #include "grid_sync.cuh"
@@ -96,9 +95,12 @@ __global__ void gauss_fill_kernel(R *out, size_t n, uint32_t s1, uint32_t s2) {
 // ---------------------------------------------------------------------------
 constexpr int kRedThreads = 256;
 
-__device__ __forceinline__ double warp_sum(double v) {
+// Sum over the warp (in every lane; with other arguments in lane 0).  Levels of the xor tree that would add zeros only
+// are left out: with STEP > 1 the lanes that are no multiple of it hold zero, with
+// LANES < 32 those from LANES on (an SM issues an FP64 addition every 16 cycles).
+template <int STEP = 1, int LANES = 32> __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = LANES / 2; o >= STEP; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
@@ -110,11 +112,11 @@ __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.launch_dependents;");
 }
 
-template <int NV>
+template <int NV, int STEP = 1>
 __device__ __forceinline__ void block_sum(double (&v)[NV]) {
   __shared__ double red[NV][kRedThreads / 32];
 #pragma unroll
-  for (int q = 0; q < NV; q++) v[q] = warp_sum(v[q]);
+  for (int q = 0; q < NV; q++) v[q] = warp_sum<STEP>(v[q]);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (lane == 0) {
 #pragma unroll
@@ -125,19 +127,20 @@ __device__ __forceinline__ void block_sum(double (&v)[NV]) {
 #pragma unroll
     for (int q = 0; q < NV; q++) {
       double x = lane < kRedThreads / 32 ? red[q][lane] : 0.0;
-      v[q] = warp_sum(x);
+      v[q] = warp_sum<1, kRedThreads / 32>(x);
     }
   }
 }
 
 // Publishes this block's NV partial sums; returns true in thread 0 of the
 // last block to arrive, whose `tot` then holds the grid totals (summed in
-// block order, so the result does not depend on arrival order).
-template <int NV>
+// block order, so the result does not depend on arrival order).  STEP: threads
+// that are no multiple of it bring zeros.
+template <int NV, int STEP = 1>
 __device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials,
                                          unsigned *ticket, double (&tot)[NV]) {
   __shared__ bool s_last;
-  block_sum<NV>(v);
+  block_sum<NV, STEP>(v);
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int q = 0; q < NV; q++) __stcg(partials + (size_t)q * gridDim.x + blockIdx.x, v[q]);
@@ -320,11 +323,6 @@ __device__ __forceinline__ float2 ld_dsmem(const float2 *local, unsigned rank) {
 template <class R> struct DotAcc {
   double v = 0.0;
   __device__ __forceinline__ void add_prod(R x, R y) { v += (double)x * (double)y; }
-  __device__ __forceinline__ void add_diff2(R x, R y) {  // (x - y)^2
-    const double d = (double)x - (double)y;
-    v += d * d;
-  }
-  __device__ __forceinline__ void merge(const DotAcc &o) { v += o.v; }
   __device__ __forceinline__ void warp_merge() { v = warp_sum(v); }
   __device__ __forceinline__ double value() const { return v; }
 };
@@ -342,16 +340,6 @@ template <> struct DotAcc<float> {
     const float p = __fmul_rn(x, y);
     add(p, __fmaf_rn(x, y, -p));
   }
-  // (x - y)^2: the difference as d + e exactly (two-sum), squared to first order
-  // in e
-  __device__ __forceinline__ void add_diff2(float x, float y) {
-    const float d = __fsub_rn(x, y);
-    const float bp = __fsub_rn(d, x);
-    const float e = __fsub_rn(__fsub_rn(x, __fsub_rn(d, bp)), __fadd_rn(y, bp));
-    const float p = __fmul_rn(d, d);
-    add(p, __fmaf_rn(__fadd_rn(d, d), e, __fmaf_rn(d, d, -p)));
-  }
-  __device__ __forceinline__ void merge(const DotAcc &o) { merge(o.s, o.c); }
   // (s, c) += (s2, c2); the same result for either order of the operands
   __device__ __forceinline__ void merge(float s2, float c2) {
     const float t = __fadd_rn(s, s2);
@@ -932,62 +920,6 @@ tridiag_sqrt_quad_kernel(const KrylovScalars *sc, int m, double *out, double *G,
   if (t == 0) *flag = 0.0;
 }
 
-// Grid totals of two accumulators, as grid_sum (same trees): FP32 vectors keep
-// them as pairs of floats throughout (two floats in the place of a double), so
-// that the whole grid does no FP64 arithmetic.  True in thread 0 of the last
-// block.
-template <class R>
-__device__ __forceinline__ bool grid_sum_dot(DotAcc<R> (&v)[2], double *partials,
-                                             unsigned *ticket, double (&tot)[2]) {
-  static_assert(sizeof(DotAcc<R>) == sizeof(double), "one partial each");
-  __shared__ DotAcc<R> red[2][kRedThreads / 32];
-  __shared__ bool s_last;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  auto block_merge = [&](DotAcc<R> (&x)[2]) {
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-      x[q].warp_merge();
-      if (lane == 0) red[q][wid] = x[q];
-    }
-    __syncthreads();
-    if (wid == 0) {
-#pragma unroll
-      for (int q = 0; q < 2; q++) {
-        x[q] = lane < kRedThreads / 32 ? red[q][lane] : DotAcc<R>();
-        x[q].warp_merge();
-      }
-    }
-  };
-  DotAcc<R> *part = reinterpret_cast<DotAcc<R> *>(partials);
-  block_merge(v);
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int q = 0; q < 2; q++) part[(size_t)q * gridDim.x + blockIdx.x] = v[q];
-    __threadfence();
-    s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!s_last) return false;
-  __threadfence();
-  DotAcc<R> acc[2];
-  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-      const double raw = __ldcg(partials + (size_t)q * gridDim.x + b);
-      DotAcc<R> p;
-      memcpy(&p, &raw, sizeof(p));
-      acc[q].merge(p);
-    }
-  }
-  block_merge(acc);
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int q = 0; q < 2; q++) tot[q] = acc[q].value();
-    *ticket = 0u;
-  }
-  return threadIdx.x == 0;
-}
-
 // y = |z| V c over m basis vectors and, when yprev is given, err = |y -
 // yprev| / |yprev| (FP64) -> sc->err and the mapped host copy: the estimate
 // and the error of one convergence check in one launch (each thread's
@@ -1010,14 +942,7 @@ __global__ void krylov_check_kernel(const R *V, size_t ldv, int m, const double 
   const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const int part = (int)(tid % TPE);
   const size_t per_pass = (size_t)gridDim.x * blockDim.x / TPE;
-  // The sums are taken over y / 2^k, 2^k about |z| c_0 <= |y|: the scale is
-  // exact, and FP32 squares neither overflow nor vanish for any size of z.
-  R scale = R(1);
-  if constexpr (std::is_same<R, float>::value) {
-    const double top = fabs(nz * c[0]);
-    if (top > 0.0 && top < 3e38) scale = ldexpf(1.0f, -max(-126, min(126, ilogb(top))));
-  }
-  DotAcc<R> v[2];  // |yprev|^2, |y - yprev|^2
+  double v[2] = {0.0, 0.0};  // |yprev|^2, |y - yprev|^2
   for (size_t e0 = 0; e0 < n; e0 += per_pass) {
     const size_t e = e0 + tid / TPE;
     const bool ok = e < n;
@@ -1041,15 +966,15 @@ __global__ void krylov_check_kernel(const R *V, size_t ldv, int m, const double 
     if (ok && part == 0) {
       y[e] = acc;
       if (yprev) {
-        const R a = scale * yprev[e];
-        v[0].add_prod(a, a);
-        v[1].add_diff2(scale * acc, a);
+        const double a = (double)yprev[e], dlt = (double)acc - a;
+        v[0] += a * a;
+        v[1] += dlt * dlt;
       }
     }
   }
   if (!yprev) return;
   double tot[2];
-  if (grid_sum_dot<R>(v, partials, ticket, tot)) {
+  if (grid_sum<2, TPE>(v, partials, ticket, tot)) {
     const double err = fabs(sqrt(tot[1]) / sqrt(tot[0]));
     sc->err = err;
     *host_err = err;
