@@ -29,6 +29,7 @@ constexpr long long kPairsMinSteps = 4;
 // line far from the origin (and one radius above a wall); their own sums are
 // never read.
 constexpr double kPadX = 1.0e6;
+constexpr double kTooHigh = 1.152921504606846976e18;  // 2^60 radii
 
 template <class R> struct LaneTypes;
 template <> struct LaneTypes<float> { using V = F2; using L = float2; };
@@ -164,6 +165,13 @@ __device__ __forceinline__ void scale_slot(const PairsArgs<R> &a, int S, int t, 
       const R z = v[q][2];
       const R b = z < R(0) ? R(0) : (z > R(1) ? R(1) : z);
       v[q][2] = z > R(1) ? z : R(1);
+      // The product of two heights must not overflow (pairwise.cuh; it is
+      // multiplied by a fifth power that is 0 by then): a particle 1e18 radii up,
+      // which meets nobody to within rounding, goes no higher but further away.
+      if (sizeof(R) == 4 && z > R(kTooHigh)) {
+        v[q][2] = R(kTooHigh);
+        v[q][0] += z - R(kTooHigh);
+      }
       sF *= b;
       sT *= b;
     }

@@ -150,3 +150,30 @@ def test_refused(lib, refused, precision, wall, ang, N):
     got = product(s)
     assert all(np.array_equal(x, y) for x, y in zip(got, pairs if refused == 1 else want))
     assert not all(np.array_equal(x, y) for x, y in zip(pairs, want))
+
+
+@pytest.mark.parametrize("far", [1e17, 3e18, 1e19, 1e20, 1e30])
+@pytest.mark.parametrize("ang", [0, 1])
+def test_particles_far_above_a_wall(lib, oracle, ang, far):
+    """Particles put out of the way (padding of uneven batches), up to where the
+    product of two heights overflows in FP32: finite and right for all, two of them
+    above each other and two in one place included."""
+    N = 130
+    rng = np.random.default_rng(12)
+    p = rng.uniform(1, 12, (N, 3))
+    p[100:, 2] = far * rng.uniform(1, 3, 30)
+    p[100:110, :2] += far
+    p[121, :2] = p[120, :2]
+    p[123] = p[122]
+    F, T = rng.normal(size=(2, N, 3))
+    p, F, T = (x.astype(np.float32) for x in (p, F, T))
+    T = T if ang else None
+    s = make_solver(1, ang, 1.1, 0.9, "float")
+    s.setPositions(p)
+    U, W = s.Mdot(F, T)
+    # with 64-bit positions nothing overflows
+    Uo, Wo = oracle.mdot(p.astype(np.float64), F, T, a=1.1, viscosity=0.9, wall=1,
+                         include_angular=ang)
+    assert rel_err(U, Uo) <= TOL["float"]
+    if ang:
+        assert rel_err(W, Wo) <= TOL["float"]
