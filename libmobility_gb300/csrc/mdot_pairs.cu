@@ -18,7 +18,8 @@ namespace lmg {
 
 namespace {
 
-// Largest scratch for the tile pairs of a pass, in elements (1 GiB in FP32).
+// Largest scratch for the tile pairs of a pass, in elements (1 GiB in FP32, 2 in
+// FP64); the slots of the rows and warps come on top.  A handle keeps it.
 constexpr size_t kPairsMaxPart = size_t(1) << 28;
 // Tile pairs of a row whose I sums a lane adds up before the two-sum (in FP32
 // the lanes of a packed sum then hold 128 terms each at most).
@@ -700,6 +701,7 @@ void mdot_pairs_plan_tables(int N, int nper, bool ang, long long resident, int f
       if (col[w] >= 0) warps[fill[col[w]]++] = w;
     p.part_elems = std::max(p.part_elems, (size_t)EL * (size_t)(pairs + (r1 - r) + 2 * q.warps));
     p.passes.push_back(q);
+    p.carries = p.carries || r1 % tpb != 0;
     r = r1;
   }
   // bands of one batch carry their sums; passes of whole batches need not

@@ -85,6 +85,7 @@ struct PairsPlan {
   std::vector<PairsPass> passes;
   size_t part_elems = 0;  // scratch (of R) of the largest pass
   size_t acc_elems = 0;   // sums carried between passes
+  bool carries = false;   // a batch takes several passes (else nothing is carried)
   // per pass: for each tile, where its list of J-side partials of cut tile
   // pairs begins (tiles + 1 entries), then the warps that wrote them
   std::vector<int> cuts;

@@ -608,7 +608,8 @@ bool Solver<R>::mdot_pairs(const R *pos, const R *F, const R *T, R *U, R *W) {
   // takes mdot_kernel, which needs no scratch for the smallest systems
   if (it == pairs_plans_.end() || (it->second->plan.ok &&
                                    (pairs_part_.count < it->second->plan.part_elems ||
-                                    pairs_acc_.count < it->second->plan.acc_elems))) {
+                                    (it->second->plan.carries &&
+                                     pairs_acc_.count < it->second->plan.acc_elems)))) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream(), &capture) != cudaSuccess) {
       (void)cudaGetLastError();
@@ -639,8 +640,8 @@ bool Solver<R>::mdot_pairs(const R *pos, const R *F, const R *T, R *U, R *W) {
   try {
     if (refuse == 1) throw_cuda(cudaErrorMemoryAllocation, "lmg_internal_pairs_refuse");
     pairs_part_.ensure(st.plan.part_elems);
-    if (st.plan.acc_elems) pairs_acc_.ensure(st.plan.acc_elems);
-  } catch (const Error &) {  // no memory left for the partial sums (2^28 elements and more)
+    if (st.plan.carries) pairs_acc_.ensure(st.plan.acc_elems);
+  } catch (const Error &) {  // no memory left for the partial sums (kPairsMaxPart and more)
     (void)cudaGetLastError();
     pairs_part_.release();
     return false;

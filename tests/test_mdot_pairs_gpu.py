@@ -177,3 +177,24 @@ def test_particles_far_above_a_wall(lib, oracle, ang, far):
     assert rel_err(U, Uo) <= TOL["float"]
     if ang:
         assert rel_err(W, Wo) <= TOL["float"]
+
+
+def test_passes_of_whole_batches_carry_nothing(lib):
+    """Sums are carried from pass to pass (61 MB here) only where a batch takes
+    several passes; these passes hold whole batches, with 4 MB of partial sums."""
+    import torch
+    nper, nb = 30, 20000
+    rng = np.random.default_rng(3)
+    p, F, T = (torch.tensor(x, dtype=torch.float32, device="cuda")
+               for x in (rng.uniform(1, 12, (nper * nb, 3)), *rng.normal(size=(2, nper * nb, 3))))
+    assert lib.lmg_internal_pairs_max_part(1000000) == 0
+    s = make_solver(1, 1, 1.1, 0.9, "float", nper * nb, nper)
+    s.setPositions(p)
+    out = s.Mdot(F, T)
+    del out  # (in torch's pool)
+    s.clean()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    U, W = s.Mdot(F, T)
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] < 40 << 20
