@@ -100,7 +100,8 @@ lmg_status lmg_destroy(lmg_solver *h);
  * its buffers, and the first on another stream waits on the GPU for the work of
  * the last one (whose stream may have been destroyed since).  Calls captured
  * into a CUDA graph are outside this order: a graph's launches must not overlap
- * each other or other calls of the handle. */
+ * each other or other calls of the handle, and they name its buffers, which more
+ * particles than at the capture, lmg_initialize and lmg_clean move. */
 #define LMG_OWN_STREAM ((void *)(intptr_t)-1)
 lmg_status lmg_set_stream(lmg_solver *h, void *cuda_stream);
 

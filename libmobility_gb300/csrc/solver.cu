@@ -183,11 +183,36 @@ template <class R> class Solver final : public SolverBase {
   int step_ctas_ = -1;   // CTAs of the cluster of krylov_step_cluster_kernel (0: none fits)
   bool tickets_zeroed_ = false;
   std::map<std::tuple<int, int, int, int, int>, MdotPlan> plans_;
+  // Plans hold device memory of their own, so a handle keeps the last kMaxPlans
+  // of each kind (a program may change N at every step), and those that a
+  // captured call names.
+  static constexpr size_t kMaxPlans = 32;
+  struct PlanUse {
+    unsigned long last = 0;
+    bool captured = false;
+  };
+  unsigned long plan_clock_ = 0;
+  void use_plan(PlanUse &u) {
+    u.last = ++plan_clock_;
+    u.captured = u.captured || capturing();
+  }
+  template <class Map> static void make_room(Map &plans) {
+    while (plans.size() >= kMaxPlans) {
+      auto oldest = plans.end();
+      for (auto it = plans.begin(); it != plans.end(); ++it)
+        if (!it->second->use.captured &&
+            (oldest == plans.end() || it->second->use.last < oldest->second->use.last))
+          oldest = it;
+      if (oldest == plans.end()) return;
+      plans.erase(oldest);
+    }
+  }
   // symmetric open-space product (FP32): plans with their device tables,
   // partial sums and barrier counts, and the flag a barrier that timed out
   // raises
   struct SymState {
     SymPlan plan;
+    PlanUse use;
     DeviceBuffer<int4> pairs, warps;
     DeviceBuffer<int> pseg;
     // arrival count of the kernel's grid barrier: one per plan, so every
@@ -203,6 +228,7 @@ template <class R> class Solver final : public SolverBase {
   // of their own (a captured product names it: a solve must not move it)
   struct PairsState {
     PairsPlan plan;
+    PlanUse use;
     // what is copied to the device buffer: the copy may still read it after the
     // call (freeing the buffer, which comes first, waits for it)
     std::vector<unsigned long long> upload;
@@ -576,8 +602,10 @@ template <class R> bool Solver<R>::mdot_sym(const R *pos, const R *F, R *U) {
         // the host tables must outlive the copies
         LMG_CUDA(cudaStreamSynchronize(stream()));
       }
+      make_room(sym_plans_);
       it = sym_plans_.insert_or_assign(key, std::move(st)).first;
     }
+    use_plan(it->second->use);
     const SymState &st = *it->second;
     const SymPlan &p = st.plan;
     if (p.grid <= 0) return false;
@@ -630,8 +658,10 @@ bool Solver<R>::mdot_pairs(const R *pos, const R *F, const R *T, R *U, R *W) {
       LMG_CUDA(cudaMemcpyAsync(st->bars_and_cuts.ensure(up.size()), up.data(),
                                up.size() * sizeof(up[0]), cudaMemcpyHostToDevice, stream()));
     }
+    make_room(pairs_plans_);
     it = pairs_plans_.insert_or_assign(key, std::move(st)).first;
   }
+  use_plan(it->second->use);
   const PairsState &st = *it->second;
   if (!st.plan.ok) return false;
   sym_err_.ensure(1);

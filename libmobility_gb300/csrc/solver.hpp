@@ -136,6 +136,7 @@ class SolverBase {
   cudaStream_t work_stream_ = nullptr;
   cudaEvent_t work_done_ = nullptr;
   bool has_work_ = false, work_recorded_ = false;
+  bool lasting() const;  // the stream is the default one or the handle's own
   bool capturing();
   void ensure_work_event();
   void follow_last_call();

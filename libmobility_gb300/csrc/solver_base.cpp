@@ -167,9 +167,15 @@ cudaStream_t SolverBase::stream() {
   return stream_;
 }
 
-// Whether the call is being captured into a graph: nothing runs then, and an
-// event recorded in a capture or before it is no use on the other side.
+bool SolverBase::lasting() const {
+  return stream_ == nullptr || stream_ == cudaStreamLegacy || (own_ && stream_ == own_);
+}
+
+// Whether the call is being captured into a graph (the streams above never are):
+// nothing runs then, and an event recorded in a capture or before it is no use on
+// the other side.
 bool SolverBase::capturing() {
+  if (lasting()) return false;
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream_, &st) != cudaSuccess) {
     (void)cudaGetLastError();  // the default stream while another is captured
@@ -198,14 +204,12 @@ void SolverBase::follow_last_call() {
 // the caller's it is recorded at once (1 us a call; none on those two).
 void SolverBase::record_work() {
   if (!have_stream_) return;
-  const bool lasting =
-      stream_ == nullptr || stream_ == cudaStreamLegacy || (own_ && stream_ == own_);
-  if (!lasting) {
-    if (capturing()) return;
+  if (capturing()) return;
+  if (!lasting()) {
     ensure_work_event();
     LMG_CUDA(cudaEventRecord(work_done_, stream_));
   }
-  work_recorded_ = !lasting;
+  work_recorded_ = !lasting();
   work_stream_ = stream_;
   has_work_ = true;
 }

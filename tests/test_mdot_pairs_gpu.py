@@ -198,3 +198,46 @@ def test_passes_of_whole_batches_carry_nothing(lib):
     U, W = s.Mdot(F, T)
     torch.cuda.synchronize()
     assert free - torch.cuda.mem_get_info()[0] < 40 << 20
+
+
+@pytest.mark.parametrize("wall,ang", [(1, 1), (0, 0)])  # the pairs and the symmetric kernel
+def test_plans_are_bounded(lib, oracle, wall, ang):
+    """A handle whose particles change in number at every call keeps a bounded number
+    of plans with device memory, those of captured calls among them."""
+    import torch
+    rng = np.random.default_rng(8)
+    top = 3000
+    p, F = (torch.tensor(x, dtype=torch.float32, device="cuda")
+            for x in (rng.uniform(1, 60, (top, 3)), rng.normal(size=(top, 3))))
+    s = make_solver(wall, ang, 1.1, 0.9, "float")
+
+    def product(n):
+        s.setPositions(p[:n])
+        return s.Mdot(F[:n])
+
+    first = [x.clone() for x in product(1000) if x is not None]
+    for _ in range(2):  # both position buffers at their largest: the graph names one
+        product(top)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    s.setPositions(p[:1000])
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        out = [x for x in s.Mdot(F[:1000]) if x is not None]
+    used = []
+    for k in range(4):
+        for n in range(1500 + 100 * k, 1600 + 100 * k):
+            product(n)
+        torch.cuda.synchronize()
+        used.append(torch.cuda.mem_get_info()[0])
+    # 100 further plans take nothing (2 MB: how the driver hands out memory)
+    assert used[1] - used[3] <= 2 << 20, used
+    for _ in range(2):
+        s.setPositions(p[:1000])
+    torch.cuda.synchronize()
+    for x in out:
+        x.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    for x, y in zip(out, first):
+        assert torch.equal(x, y)
