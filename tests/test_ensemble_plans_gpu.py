@@ -63,3 +63,34 @@ def test_one_launch_step_is_the_three_kernel_step(cuda, sizes, precision):
     m = sum(sizes[:-1])
     assert (out[0][1] == out[1][1][:-1]).all()
     assert np.array_equal(out[0][0][:m], out[1][0][:m])
+
+
+@pytest.mark.parametrize("precision", ["float", "double"])
+@pytest.mark.parametrize("sizes,wide", [([300, 310, 290, 380], False), ([200, 256, 250, 140], True),
+                                        ([600, 700, 620, 760], False), ([400, 512, 390, 400], None),
+                                        ([500, 400, 510, 390], True), ([300], True),
+                                        ([800, 900, 1000, 990], False)])
+def test_tuner_tries_wide_tiles_only_within_systems(cuda, sizes, wide, precision):
+    """Whatever the timing says: tiles of two targets a thread are among the plans
+    tried only where none covers two systems, that is where every system but the
+    last of its group is padded to a multiple of 256."""
+    from libmobility_gb300.ensemble import Ensemble
+    rng = np.random.default_rng(0)
+    e = Ensemble(precision=precision)
+    e.setSystems(sizes, ["open"] * len(sizes), [0.0] * len(sizes))
+    e.initialize(1.0, 1.0, tolerance=1e-4, seed=1)
+    n = sum(sizes)
+    dtype = np.float32 if precision == "float" else np.float64
+    e.setPositions(rng.uniform(0, 40, (n, 3)).astype(dtype))
+    e.Mdot(rng.normal(size=(n, 3)).astype(dtype))
+    groups = e.describe()["groups"]
+    bucket = lambda s: s.bit_length() - 1  # noqa: E731
+    assert len(groups) == len({bucket(s) for s in sizes})
+    for g in groups:
+        lo, hi = g["size_range"]
+        padded = [-(-s // 128) * 128 for s in sizes if lo <= s <= hi]
+        tried = {t for t, _, _ in g["trials_ms"]}
+        within = all(p % 256 == 0 for p in padded[:-1])
+        assert tried == ({1, 2} if within else {1})
+        if wide is not None:
+            assert within == wide
