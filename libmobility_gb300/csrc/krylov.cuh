@@ -104,7 +104,6 @@ template <int STEP = 1, int LANES = 32> __device__ __forceinline__ double warp_s
   return v;
 }
 
-// Sums `v` over the block; result valid in thread 0.
 // In a kernel launched ahead of its predecessor's end: waits for that end, then
 // lets the next one be launched.
 __device__ __forceinline__ void pdl_wait() {
@@ -112,6 +111,7 @@ __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.launch_dependents;");
 }
 
+// Sums `v` over the block; result valid in thread 0.
 template <int NV, int STEP = 1>
 __device__ __forceinline__ void block_sum(double (&v)[NV]) {
   __shared__ double red[NV][kRedThreads / 32];

@@ -32,7 +32,6 @@ __device__ __forceinline__ void stf(__half *p, float v) { *p = __float2half_rn(v
 // closer than s h lies in a cell at Chebyshev distance <= s, so the list is
 // exact.  Cost O(N x particles in the searched cells) instead of O(N^2).
 // ---------------------------------------------------------------------------
-constexpr int kKnnThreads = 128;
 constexpr int kScanThreads = 1024;
 
 // order-preserving map of floats to unsigned (for atomic min / max)

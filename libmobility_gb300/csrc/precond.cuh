@@ -138,7 +138,8 @@ cudaError_t precond_rows_launch(int K, const PrecRows &rows, bool transpose, flo
                                 const float *x, float *out, const int *skip,
                                 cudaStream_t stream, bool early = false);
 
-// The same with FP32 blocks in the build's own layout (training and checks):
+// The same with FP32 blocks in the build's own layout (checks of a build against a
+// dense P; no solve takes them):
 // out_i = sum_n B[n][i] x_{nb[n][i]}   (P x)
 cudaError_t precond_apply_launch(int K, const float *blocks, const int *nb, int N,
                                  const float *x, float *out, cudaStream_t stream);

@@ -205,9 +205,9 @@ int lmg_internal_barrier_spins(long long spins) {
 }
 
 // Host plan of the unordered-pair product for `resident` resident blocks (no
-// device needed).  info[0..4] receives passes, ints of the cut tables, scratch
-// elements, elements carried between passes and tiles per batch; passes: 7
-// values each (first and end row, steps, steps per warp, warps, blocks, offset
+// device needed).  info[0..5] receives passes, ints of the cut tables, scratch
+// elements, elements carried between passes, tiles per batch and slots of a tile
+// in use; passes: 7 values each (first and end row, steps, steps per warp, warps, blocks, offset
 // of its cut table).  Returns 0, or 2 when the shape does not suit the kernel.
 int lmg_internal_pairs_plan(int N, int nper, int ang, int precision, long long resident,
                             int force_warps, long long max_part, long long *info,
