@@ -917,7 +917,10 @@ int Solver<R>::lanczos(const R *z, R *y_out, size_t n, double tol, double *resid
     // the end (N = 2048 wall with torques, 50 us an iteration: 3.15 ms a step
     // with one ahead, 3.22 with two, 3.27 with three).  FP32 forces in open
     // space up to 4096 particles take 20 to 30 us an iteration: two ahead
-    // (N = 2000 1.05 ms, 1.06 with one or three)
+    // (N = 2000 1.05 ms, 1.06 with one or three).  From 4097 to 8192 one is no
+    // slower than the three there were: N = 5000 2.26 -> 1.90 ms, 8192 to 1e-6
+    // 6.85 -> 6.21, wall forces 5000 7.52 -> 6.84, with torques 8000 30.4 -> 27.2
+    // (all that changed since counted in)
     return sizeof(R) == 4 && !wall_ && !ang_ && !prec_active() && batch_size() <= 4096 ? 2 : 1;
   };
   auto issue = [&](int j) {
