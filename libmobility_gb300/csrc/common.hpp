@@ -6,6 +6,7 @@
 #include <cstring>
 #include <stdexcept>
 #include <string>
+#include <vector>
 
 #include "libmobility_gb300.h"
 
@@ -93,6 +94,35 @@ template <class T> struct DeviceBuffer {
     if (ptr) cudaFree(ptr);
     ptr = nullptr;
     count = 0;
+  }
+};
+
+// The same for scratch that captured calls may name: when it grows after one did,
+// the allocation that the graph uses stays until release.
+template <class T> struct ScratchBuffer : DeviceBuffer<T> {
+  using Base = DeviceBuffer<T>;
+  bool named = false;  // a captured call uses the present allocation
+  std::vector<T *> kept;
+  ~ScratchBuffer() { release(); }
+  T *ensure(size_t n) {
+    if (n > this->count) drop();
+    return Base::ensure(n);
+  }
+  // gives the present allocation up
+  void drop() {
+    if (named && this->ptr) {
+      kept.push_back(this->ptr);
+      this->ptr = nullptr;
+      this->count = 0;
+    }
+    named = false;
+    Base::release();
+  }
+  void release() {
+    for (T *p : kept) cudaFree(p);
+    kept.clear();
+    named = false;
+    Base::release();
   }
 };
 

@@ -129,8 +129,8 @@ template <class R> class Solver final : public SolverBase {
   DeviceBuffer<R> pos_, pos_tmp_;
   DeviceBuffer<R> in_stage_, out_stage_;  // host<->device staging of user arrays
   PinnedBuffer<R> pin_;                   // pinned bounce buffer
-  DeviceBuffer<R> part_;                  // Mdot split partials
-  DeviceBuffer<unsigned> tickets_;        // Mdot split tickets (self-resetting)
+  ScratchBuffer<R> part_;                 // Mdot split partials
+  ScratchBuffer<unsigned> tickets_;       // Mdot split tickets (self-resetting)
   DeviceBuffer<double> red_part_;         // reduction partials
   DeviceBuffer<unsigned> red_ticket_;     // reduction ticket (self-resetting)
   DeviceBuffer<double> dmin_;
@@ -192,9 +192,11 @@ template <class R> class Solver final : public SolverBase {
     bool captured = false;
   };
   unsigned long plan_clock_ = 0;
-  void use_plan(PlanUse &u) {
+  bool use_plan(PlanUse &u) {  // whether the call is being captured
+    const bool c = capturing();
     u.last = ++plan_clock_;
-    u.captured = u.captured || capturing();
+    u.captured = u.captured || c;
+    return c;
   }
   template <class Map> static void make_room(Map &plans) {
     while (plans.size() >= kMaxPlans) {
@@ -235,7 +237,7 @@ template <class R> class Solver final : public SolverBase {
     DeviceBuffer<unsigned long long> bars_and_cuts;
   };
   std::map<std::tuple<int, int, int, int>, std::unique_ptr<PairsState>> pairs_plans_;
-  DeviceBuffer<R> pairs_part_, pairs_acc_;
+  ScratchBuffer<R> pairs_part_, pairs_acc_;
   bool mdot_pairs(const R *pos, const R *F, const R *T, R *U, R *W);
   void check_barriers();
 
@@ -430,6 +432,7 @@ void Solver<R>::mdot_device(const R *pos, const R *F, const R *T, R *U, R *W, bo
       LMG_CUDA(cudaMemsetAsync(tickets_.ptr, 0, tickets_.count * sizeof(unsigned), stream()));
       tickets_zeroed_ = true;
     }
+    if (capturing()) part_.named = tickets_.named = true;
   }
   MdotArgs<R> a{};
   a.pos = pos;
@@ -484,6 +487,7 @@ void Solver<R>::mdot_rows_device(const R *pos, const R *F, const R *T, R *U, R *
       LMG_CUDA(cudaMemsetAsync(tickets_.ptr, 0, tickets_.count * sizeof(unsigned), stream()));
       tickets_zeroed_ = true;
     }
+    if (capturing()) part_.named = tickets_.named = true;
   }
   MdotArgs<R> a{};
   a.pos = pos;
@@ -661,7 +665,7 @@ bool Solver<R>::mdot_pairs(const R *pos, const R *F, const R *T, R *U, R *W) {
     make_room(pairs_plans_);
     it = pairs_plans_.insert_or_assign(key, std::move(st)).first;
   }
-  use_plan(it->second->use);
+  const bool captured = use_plan(it->second->use);
   const PairsState &st = *it->second;
   if (!st.plan.ok) return false;
   sym_err_.ensure(1);
@@ -673,9 +677,10 @@ bool Solver<R>::mdot_pairs(const R *pos, const R *F, const R *T, R *U, R *W) {
     if (st.plan.carries) pairs_acc_.ensure(st.plan.acc_elems);
   } catch (const Error &) {  // no memory left for the partial sums (kPairsMaxPart and more)
     (void)cudaGetLastError();
-    pairs_part_.release();
+    pairs_part_.drop();
     return false;
   }
+  if (captured) pairs_part_.named = pairs_acc_.named = true;
   unsigned long long *bars = st.bars_and_cuts.ptr;
   const cudaError_t e =
       refuse == 2 ? cudaErrorCooperativeLaunchTooLarge
