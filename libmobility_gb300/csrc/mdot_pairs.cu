@@ -482,10 +482,26 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
     cur = nxt;
   }
 
-  // after a wait that ran out the partials may be incomplete: the sums that this
-  // block folds are NaN, and the host raises an error when it sees the flag
-  const bool complete = grid_barrier_mono(a.bar, a.spins);
-  if (!complete && threadIdx.x == 0) *a.err = 1;
+  // After a wait that ran out the partials may be incomplete: what this block
+  // would fold is NaN (for certain that part; it marks all of the pass), and the
+  // host raises an error when it sees the flag.
+  if (!grid_barrier_mono(a.bar, a.spins)) {
+    if (threadIdx.x == 0) *a.err = 1;
+    const int b_lo = a.row0 / a.tpb, b_hi = (a.row1 - 1) / a.tpb + 1;  // batches
+    if (a.last) {
+      for (size_t e = 3 * (size_t)b_lo * a.nper + threadIdx.x; e < 3 * (size_t)b_hi * a.nper;
+           e += kPairsThreads) {
+        if (!LMG_IN_BOUNDS(e < 3 * (size_t)a.N, 25, e)) continue;
+        if (a.U) a.U[e] = R(NAN);
+        if (ANG && a.W) a.W[e] = R(NAN);
+      }
+    } else {
+      for (size_t e = 2 * (size_t)b_lo * a.tpb * EL + threadIdx.x;
+           e < 2 * (size_t)b_hi * a.tpb * EL; e += kPairsThreads)
+        a.acc[e] = R(NAN);
+    }
+    return;
+  }
 
   // ---- fold the partials: one component of a tile at a time, by a warp or by
   // the block's four warps, each taking every fourth partial, sixteen loads ahead ----
@@ -561,7 +577,6 @@ mdot_pairs_kernel(const PairsArgs<R> a) {
             c += red[q][1][p];
           }
         }
-        if (!complete) s = R(NAN);
         if (!a.last) {
           a.acc[2 * o] = s;
           a.acc[2 * o + 1] = c;
