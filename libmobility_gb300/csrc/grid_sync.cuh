@@ -49,9 +49,9 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar) {
 // so their arrivals never mix.  One atomic per block, no reset; the wait is
 // bounded like grid_barrier's, to `spins` polls (0: every block reports that its
 // wait ran out, after its arrival).
-constexpr long kMonoSpins = 1L << 26;
+constexpr int kMonoSpins = 1 << 26;
 
-__device__ __forceinline__ bool grid_barrier_mono(unsigned long long *count, long spins) {
+__device__ __forceinline__ bool grid_barrier_mono(unsigned long long *count, int spins) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -64,7 +64,7 @@ __device__ __forceinline__ bool grid_barrier_mono(unsigned long long *count, lon
     asm volatile("atom.release.gpu.add.u64 %0, [%1], 1;" : "=l"(old) : "l"(count) : "memory");
     const unsigned long long target = (old / g + 1) * g;
     int ok = 0;
-    for (long it = 0; it < spins; it++) {
+    for (int it = 0; it < spins; it++) {
       unsigned long long v;
       asm volatile("ld.acquire.gpu.u64 %0, [%1];" : "=l"(v) : "l"(count) : "memory");
       if (v >= target) {

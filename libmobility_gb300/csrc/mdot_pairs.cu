@@ -80,7 +80,7 @@ template <class R> struct PairsArgs {
   R *acc;
   const int *cuts;
   unsigned long long *bar;
-  long spins;  // of the barrier
+  int spins;  // of the barrier
   int *err;
 };
 
@@ -782,7 +782,7 @@ cudaError_t mdot_pairs_launch(const PairsPlan &p, const int *cuts, const R *pos,
              ((reinterpret_cast<uintptr_t>(pos) | reinterpret_cast<uintptr_t>(F) |
                reinterpret_cast<uintptr_t>(T)) & 7) == 0;
     a.bar = bar + q;
-    a.spins = g_barrier_spins.load() < 0 ? kMonoSpins : g_barrier_spins.load();
+    a.spins = g_barrier_spins.load() < 0 ? kMonoSpins : (int)g_barrier_spins.load();
     a.err = err;
     // Folding: rounds of loads one after the other (16 partials a warp, about
     // as much again to start and finish a component of a tile) with four warps

@@ -39,7 +39,7 @@ struct SymArgs {
   SymTables tab;
   float *part;
   unsigned long long *bar;
-  long spins;  // of the barrier
+  int spins;  // of the barrier
   int *err;
   // optional timeline (nanoseconds, %globaltimer): per warp [start, end of
   // its steps], then per block [after the barrier, end of the fold], then
@@ -479,8 +479,11 @@ __global__ void __launch_bounds__(kSymThreads, MINB) mdot_sym_kernel(const SymAr
   asm volatile("griddepcontrol.launch_dependents;");
   // ---- every partial is written: fold them into U ----
   // (a wait that ran out: as in mdot_pairs_kernel)
-  const bool complete = grid_barrier_mono(a.bar, a.spins);
-  if (!complete && threadIdx.x == 0) *a.err = 1;
+  if (!grid_barrier_mono(a.bar, a.spins)) {
+    if (threadIdx.x == 0) *a.err = 1;
+    for (size_t e = threadIdx.x; e < 3 * (size_t)a.N; e += kSymThreads) a.U[e] = NAN;
+    return;
+  }
   const size_t tb = 2 * (size_t)gridDim.x * (kSymThreads / 32) + 2 * blockIdx.x;
   if (a.trace && threadIdx.x == 0) {
     a.trace[tb] = global_ns();
@@ -584,7 +587,7 @@ __global__ void __launch_bounds__(kSymThreads, MINB) mdot_sym_kernel(const SymAr
           for (int c = 0; c < 2; c++)
             if (e[h] + c < 3 * td.y &&
                 LMG_IN_BOUNDS(3 * (size_t)td.x + e[h] + c < 3 * (size_t)a.N, 14, td.x))
-              a.U[3 * (size_t)td.x + e[h] + c] = complete ? S[h][c] + C[h][c] : NAN;
+              a.U[3 * (size_t)td.x + e[h] + c] = S[h][c] + C[h][c];
         }
       }
     }
@@ -755,7 +758,7 @@ cudaError_t mdot_sym_launch(const SymPlan &p, const SymTables &tab, const float 
   a.tab = tab;
   a.part = part;
   a.bar = bar;
-  a.spins = g_barrier_spins.load() < 0 ? kMonoSpins : g_barrier_spins.load();
+  a.spins = g_barrier_spins.load() < 0 ? kMonoSpins : (int)g_barrier_spins.load();
   a.err = err;
   a.trace = g_sym_trace.load();
   void *params[] = {(void *)&a};

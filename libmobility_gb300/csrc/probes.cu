@@ -199,7 +199,7 @@ int lmg_internal_pairs_refuse(int what) {
 // Polls of the grid barriers of the symmetric and unordered-pair products
 // launched after the call: 0 makes every wait run out, -1 restores the default.
 int lmg_internal_barrier_spins(long long spins) {
-  if (spins < -1) return 1;
+  if (spins < -1 || spins > (1 << 30)) return 1;
   lmg::g_barrier_spins.store((long)spins);
   return 0;
 }
