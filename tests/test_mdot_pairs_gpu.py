@@ -230,7 +230,7 @@ def test_plans_are_bounded(lib, oracle, wall, ang):
             product(n)
         torch.cuda.synchronize()
         used.append(torch.cuda.mem_get_info()[0])
-    # 100 further plans take nothing (2 MB: how the driver hands out memory)
+    # 100 further plans take nothing (2 MB: the unit in which memory is given out)
     assert used[1] - used[3] <= 2 << 20, used
     for _ in range(2):
         s.setPositions(p[:1000])
