@@ -35,6 +35,18 @@ CASES = [
     (0, 0, 1, 1, 1, 16384, TILED), (0, 0, 1, 1, 1, 3000, PAIRS), (0, 0, 1, 1, 2000, 100, TILED),
     (0, 0, 1, 1, 400, 200, PAIRS), (0, 0, 1, 1, 100, 256, TILED), (0, 0, 1, 1, 100, 500, PAIRS),
     (0, 0, 1, 1, 2000, 20, PAIRS), (0, 1, 1, 1, 1, 16384, PAIRS),
+    (0, 0, 1, 1, 4, 2500, PAIRS), (0, 0, 1, 1, 2, 4000, PAIRS), (0, 0, 1, 1, 2, 9001, PAIRS),
+    (0, 0, 1, 1, 2, 16384, TILED), (0, 0, 1, 1, 10, 512, TILED), (0, 0, 1, 1, 2000, 72, TILED),
+    (0, 0, 1, 1, 267, 160, PAIRS), (0, 0, 1, 1, 1000, 160, TILED),
+    (0, 0, 1, 1, 160, 600, PAIRS), (0, 0, 1, 1, 153, 400, PAIRS), (0, 0, 1, 1, 400, 96, TILED),
+    (0, 1, 1, 0, 84, 1, TILED), (0, 0, 0, 0, 49, 1, TILED), (1, 1, 0, 0, 6, 1, TILED),
+    (0, 0, 1, 0, 117, 1, PAIRS), (0, 1, 0, 0, 95, 1, PAIRS), (0, 0, 1, 0, 30, 1, TILED),
+    (0, 0, 1, 1, 1, 28, TILED), (0, 1, 1, 1, 1, 19, TILED), (0, 1, 1, 1, 988, 6, TILED),
+    (1, 0, 1, 1, 1427, 8, TILED), (1, 0, 1, 1, 619, 1, TILED), (1, 0, 1, 1, 1, 9, TILED),
+    (1, 1, 0, 0, 300, 1, PAIRS), (0, 0, 0, 0, 2, 17, TILED), (0, 1, 1, 0, 655, 12, PAIRS),
+    (0, 1, 1, 0, 322, 7, PAIRS), (0, 0, 1, 0, 375, 8, TILED), (0, 1, 1, 0, 2500, 12, TILED),
+    (1, 0, 1, 1, 369, 64, TILED), (1, 0, 1, 1, 2591, 3, TILED), (1, 1, 1, 1, 1, 5, TILED),
+    (1, 0, 1, 1, 160, 65, PAIRS), (1, 0, 1, 1, 200, 48, PAIRS), (1, 0, 1, 1, 400, 33, TILED),
     (1, 0, 1, 1, 400, 64, TILED), (1, 0, 1, 1, 100, 200, PAIRS), (1, 0, 1, 1, 1, 4096, PAIRS),
     (1, 1, 1, 1, 400, 64, PAIRS),
     # both: everything larger
