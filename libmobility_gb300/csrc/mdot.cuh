@@ -219,8 +219,11 @@ template <class R, int GEOM, bool HAS_F, bool HAS_T, bool ANG> struct PairKernel
   }
 };
 
+// Forms of the kernel (the reasons for them: mdot_launch.cu).
+constexpr int kPlainForm = 0, kDenseForm = 1, kTinyForm = 2;
+
 template <class R, int GEOM, bool HAS_F, bool HAS_T, bool ANG, int TPT, int TILE, int SUB,
-          bool DENSE>
+          int FORM>
 __global__ void __launch_bounds__(TILE / SUB)
 mdot_kernel(const MdotArgs<R> a) {
   using PK = PairKernel<R, GEOM, HAS_F, HAS_T, ANG>;
@@ -245,7 +248,7 @@ mdot_kernel(const MdotArgs<R> a) {
   __shared__ Q4<R> st[USE_T && !SOA ? TILE : 1];
   __shared__ __align__(16) float sv[NSV][SOA ? TILE : 4];
   // packed wall pairs: events (lane, packed pair) closer than 2a and their values
-  constexpr bool EVENTS = DENSE && GEOM == kWall && (PACK || PACK_UF);
+  constexpr bool EVENTS = FORM == kDenseForm && GEOM == kWall && (PACK || PACK_UF);
   constexpr int kCloseCap = 64;
   __shared__ unsigned short s_event[EVENTS ? THREADS / 32 : 1][EVENTS ? kCloseCap : 1];
   __shared__ float2 s_close[EVENTS ? THREADS / 32 : 1][EVENTS ? NC : 1][EVENTS ? kCloseCap : 1];
@@ -341,7 +344,33 @@ mdot_kernel(const MdotArgs<R> a) {
     }
     __syncthreads();
     const int n_here = min(TILE, c_end - ts);
-    if (!(uniform && n_here == TILE)) {
+    if (FORM == kTinyForm) {
+      // batches smaller than a tile: most sources are in the batch of no target of
+      // the warp, so a source is read only where one is
+      for (int jj = 0; jj < n_here; jj++) {
+        const int j = ts + jj;
+#pragma unroll
+        for (int t = 0; t < TPT; t++) {
+          if (j >= lo[t] && j < hi[t]) {
+            Q4<R> p, fv = {0, 0, 0, 0}, tv = {0, 0, 0, 0};
+            if constexpr (SOA) {
+              p = {sv[0][jj], sv[1][jj], sv[2][jj], 0};
+              fv = {sv[3][jj], sv[4][jj], sv[5][jj], 0};
+              if constexpr (PACK) tv = {sv[6][jj], sv[7][jj], sv[8][jj], 0};
+            } else {
+              p = sp[jj];
+              if (HAS_F) fv = sf[jj];
+              if (USE_T) tv = st[jj];
+            }
+            if constexpr (PACK)
+              wall_pair_fused(a.k, a.kw, xi[t], yi[t], zi[t], p.x, p.y, p.z, fv.x, fv.y, fv.z,
+                              tv.x, tv.y, tv.z, u[t], w[t]);
+            else
+              PK::eval(a.k, a.kw, xi[t], yi[t], zi[t], p, fv, tv, u[t], w[t]);
+          }
+        }
+      }
+    } else if (!(uniform && n_here == TILE)) {
       // a ragged tile or one over a batch boundary: one source after another;
       // two without branches where no target of the warp is close to either (not
       // the block-by-block wall form, whose sums the compiler would contract

@@ -20,27 +20,36 @@ constexpr int kThreads = 128;
 template <class R> constexpr int kSub = sizeof(R) == 8 ? 4 : 1;
 
 // Packed wall pairs (FP32): up to this many sources a batch, close pairs are
-// dealt out over the warp before the sums (DENSE); beyond, they are rare and
+// dealt out over the warp before the sums (kDenseForm); beyond, they are rare and
 // are evaluated where they are met, with fewer registers.  Above a wall at one
 // particle per unit area, dealt out and in place: N = 300 with torques 52 and
 // 64 us, 2048 41 and 45 us, 16384 1475 and 1397 us.
 constexpr int kDenseSpan = 4096;
 
+// Outside a solve FP32 batches smaller than a tile take a form of their own (the
+// sums of a solve keep their bits, and the compiler contracts other products in
+// it): 1 000 000 batches of one above a wall with torques 206 us, 279 in the plain
+// form, 125 000 of 8 379 and 474 (forces 243 and 301).
 template <class R, int GEOM, bool HF, bool HT, bool ANG, int TPT>
-void *kernel_ptr(bool dense) {
+void *kernel_ptr(int form) {
   constexpr int S = TPT == 1 ? kSub<R> : 1;
-  if constexpr (sizeof(R) == 4 && GEOM == kWall && HF && HT == ANG && TPT == 1) {
-    if (dense) return (void *)mdot_kernel<R, GEOM, HF, HT, ANG, TPT, kThreads, S, true>;
+  if constexpr (sizeof(R) == 4 && HF && HT == ANG) {
+    if constexpr (GEOM == kWall && TPT == 1) {
+      if (form == kDenseForm)
+        return (void *)mdot_kernel<R, GEOM, HF, HT, ANG, TPT, kThreads, S, kDenseForm>;
+    }
+    if (form == kTinyForm)
+      return (void *)mdot_kernel<R, GEOM, HF, HT, ANG, TPT, kThreads, S, kTinyForm>;
   }
-  return (void *)mdot_kernel<R, GEOM, HF, HT, ANG, TPT, kThreads, S, false>;
+  return (void *)mdot_kernel<R, GEOM, HF, HT, ANG, TPT, kThreads, S, kPlainForm>;
 }
 
 // kernel pointer for a shape; TPT in {1, 2}
 template <class R>
-void *select_kernel(const MdotShape &s, int tpt, bool dense) {
+void *select_kernel(const MdotShape &s, int tpt, int form) {
 #define LMG_SEL(G, HF, HT, A)                                              \
   if (s.geom == G && s.has_f == HF && s.has_t == HT && s.ang == A)         \
-    return tpt == 2 ? kernel_ptr<R, G, HF, HT, A, 2>(dense) : kernel_ptr<R, G, HF, HT, A, 1>(dense);
+    return tpt == 2 ? kernel_ptr<R, G, HF, HT, A, 2>(form) : kernel_ptr<R, G, HF, HT, A, 1>(form);
   LMG_SEL(kOpen, true, false, false)
   LMG_SEL(kOpen, true, false, true)
   LMG_SEL(kOpen, false, true, true)
@@ -69,7 +78,7 @@ cudaError_t mdot_plan(const MdotShape &s, int N, int max_src_span, int num_sms, 
   const int bt = kThreads * tpt;
   plan.tiles = (N + bt - 1) / bt;
   // (the splits are planned for the kernel without it, whichever runs)
-  void *k = select_kernel<R>(s, tpt, false);
+  void *k = select_kernel<R>(s, tpt, kPlainForm);
   if (!k) return cudaErrorInvalidValue;
   int per_sm = 0;
   cudaError_t e =
@@ -113,8 +122,9 @@ cudaError_t mdot_plan(const MdotShape &s, int N, int max_src_span, int num_sms, 
 
 template <class R>
 cudaError_t mdot_launch(const MdotShape &s, const MdotArgs<R> &args, const MdotPlan &plan,
-                        cudaStream_t stream, bool early) {
-  void *k = select_kernel<R>(s, plan.tpt, plan.dense);
+                        cudaStream_t stream, bool early, bool tiny) {
+  const int form = tiny ? kTinyForm : plan.dense ? kDenseForm : kPlainForm;
+  void *k = select_kernel<R>(s, plan.tpt, form);
   if (!k) return cudaErrorInvalidValue;
   MdotArgs<R> a = args;
   a.chunk = plan.chunk;
@@ -143,6 +153,6 @@ unsigned long long LMG_STATUS_NAME(LMG_REAL)(bool reset) { return bounds_status_
 
 template cudaError_t mdot_plan<LMG_REAL>(const MdotShape &, int, int, int, int, int, MdotPlan &);
 template cudaError_t mdot_launch<LMG_REAL>(const MdotShape &, const MdotArgs<LMG_REAL> &,
-                                           const MdotPlan &, cudaStream_t, bool);
+                                           const MdotPlan &, cudaStream_t, bool, bool);
 
 }  // namespace lmg

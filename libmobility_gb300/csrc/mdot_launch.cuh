@@ -23,10 +23,11 @@ cudaError_t mdot_plan(const MdotShape &s, int N, int max_src_span, int num_sms, 
                       int force_split, MdotPlan &plan);
 
 // early: the launch may begin while the kernel before it on the stream ends
-// (the kernel waits for it before it reads anything)
+// (the kernel waits for it before it reads anything); tiny: batches of fewer
+// particles than a tile has, not in a solve
 template <class R>
 cudaError_t mdot_launch(const MdotShape &s, const MdotArgs<R> &args, const MdotPlan &plan,
-                        cudaStream_t stream, bool early = false);
+                        cudaStream_t stream, bool early = false, bool tiny = false);
 
 // Longest source range needed by a tile of `bt` consecutive targets (batches
 // of nper, or the explicit batch table `sys_begin` of nsys batches), tiles

@@ -86,10 +86,12 @@ inline MdotRoute mdot_route(bool fp64, bool wall, bool ang, bool one, int N, int
   if (one && !wall) {
     if (fp64) {
       // 369 x 64 139 and 230, 400 x 33 115 and 156, 2000 x 100 2048 and 2658, but
-      // 160 x 65 188 and 148, 200 x 48 142 and 113, 500 x 30 114 and 101; 619 x 1 53
-      // and 69, 1427 x 8 55 and 105; one batch of 4096 1390 and 1275
-      if (nb >= 2 * num_sms && N >= 80 * num_sms) return MdotRoute::tiled;
-      if (nper <= 8 && nb >= 4 * num_sms) return MdotRoute::tiled;
+      // 160 x 65 188 and 148, 200 x 48 142 and 113, 500 x 30 114 and 101; 320 x 1 53
+      // and 69, 1427 x 8 55 and 105, 2591 x 3 66 and 101 (721 x 3 67 and 41); one batch
+      // of 4096 1390 and 1275
+      if (nb >= 2 * num_sms && (N >= 80 * num_sms || nper % 32 == 0 || nper == 1))
+        return MdotRoute::tiled;
+      if (nper <= 8 && nb >= 8 * num_sms) return MdotRoute::tiled;
     } else {
       // one batch: N = 16384 354 and 433, 6000 67 and 70, 4096 37.1 and 37.5 (but
       // 4 x 2500 76 and 55, 2 x 9001 293 and 269)

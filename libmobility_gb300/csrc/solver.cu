@@ -449,7 +449,8 @@ void Solver<R>::mdot_device(const R *pos, const R *F, const R *T, R *U, R *W, bo
   a.kw = make_wall_const(t0_, r0_, rt0_);
   a.part = part_.ptr;
   a.ticket = tickets_.ptr;
-  LMG_CUDA(mdot_launch<R>(s, a, plan, stream(), solve));
+  const bool tiny = !solve && nper < plan.threads && nper < N;
+  LMG_CUDA(mdot_launch<R>(s, a, plan, stream(), solve, tiny));
 }
 
 // Targets [row_begin, row_end) only, with the tiled kernel: every source of

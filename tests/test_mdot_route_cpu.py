@@ -42,7 +42,7 @@ CASES = [
     (0, 1, 1, 0, 84, 1, TILED), (0, 0, 0, 0, 49, 1, TILED), (1, 1, 0, 0, 6, 1, TILED),
     (0, 0, 1, 0, 117, 1, PAIRS), (0, 1, 0, 0, 95, 1, PAIRS), (0, 0, 1, 0, 30, 1, TILED),
     (0, 0, 1, 1, 1, 28, TILED), (0, 1, 1, 1, 1, 19, TILED), (0, 1, 1, 1, 988, 6, TILED),
-    (1, 0, 1, 1, 1427, 8, TILED), (1, 0, 1, 1, 619, 1, TILED), (1, 0, 1, 1, 1, 9, TILED),
+    (1, 0, 1, 1, 721, 3, PAIRS), (1, 0, 1, 1, 334, 32, TILED), (1, 0, 1, 1, 1427, 8, TILED), (1, 0, 1, 1, 619, 1, TILED), (1, 0, 1, 1, 1, 9, TILED),
     (1, 1, 0, 0, 300, 1, PAIRS), (0, 0, 0, 0, 2, 17, TILED), (0, 1, 1, 0, 655, 12, PAIRS),
     (0, 1, 1, 0, 322, 7, PAIRS), (0, 0, 1, 0, 375, 8, TILED), (0, 1, 1, 0, 2500, 12, TILED),
     (1, 0, 1, 1, 369, 64, TILED), (1, 0, 1, 1, 2591, 3, TILED), (1, 1, 1, 1, 1, 5, TILED),
